@@ -192,7 +192,7 @@ __device__ __forceinline__ bool box_far(float xh, float xl, float yh, float yl, 
 // limit means every point of the warp is far by the per-point test, and the
 // 32 point tests are skipped.
 __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, const float4* __restrict__ rows,
-                                                            const ElemRec* __restrict__ elems,
+                                                            const ElemRec* __restrict__ elems, int nn,
                                                             int* pair_count, int2* pairs, int pair_cap) {
   __shared__ ElemRec s_e[256];
   const int i = blockIdx.x * 256 + threadIdx.x;
@@ -216,7 +216,8 @@ __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, cons
     const float dx = fmaxf(fmaxf(__fsub_rn(E.lox, bx1), __fsub_rn(bx0, E.hix)), 0.f);
     const float dy = fmaxf(fmaxf(__fsub_rn(E.loy, by1), __fsub_rn(by0, E.hiy)), 0.f);
     if (__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) > E.lim2) continue;  // warp-uniform
-    const bool need = valid && !box_far(r.x, r.y, r.z, r.w, E);
+    // (a point on the element itself belongs to the on-element kernel)
+    const bool need = valid && (i < (e0 + el) * nn || i >= (e0 + el + 1) * nn) && !box_far(r.x, r.y, r.z, r.w, E);
     const unsigned m = __ballot_sync(0xffffffffu, need);
     if (m) {
       const int leader = __ffs(m) - 1;
@@ -744,7 +745,7 @@ static void launch_variant(const AsmRequest& q, cudaStream_t st) {
   {
     KScope ks(st, KC_NEAR);
     dim3 cg((g.nt + 255) / 256, (g.ne + 255) / 256);
-    near_classify_kernel<<<cg, 256, 0, st>>>(g.nt, g.ne, q.rows, q.elems, q.counters, q.pairs, q.pair_cap);
+    near_classify_kernel<<<cg, 256, 0, st>>>(g.nt, g.ne, q.rows, q.elems, g.nn, q.counters, q.pairs, q.pair_cap);
   }
   const bool side = q.aux != nullptr && g.n > 0;
   const bool side2 = side && q.aux2 != nullptr;

@@ -94,6 +94,24 @@ void build_rules(const bem_geom2d* g, int npg, const double* ew_host, Rules& R) 
   };
   product_weights(R.leg_x, nn, R.leg_pw);
   if (g->ngeo > 0) product_weights(R.geo_x, g->ngeo, R.geo_pw);
+  // basis k = pw_k prod_{j != k} (xi - x_j), multiplied out
+  auto monomials = [](const double* xs, int n, double* M) {
+    for (int k = 0; k < n; ++k) {
+      long double c[BEM_MAXGEO] = {1.0L}, den = 1.0L;
+      int deg = 0;
+      for (int j = 0; j < n; ++j) {
+        if (j == k) continue;
+        den *= (long double)xs[k] - (long double)xs[j];
+        ++deg;
+        for (int d = deg; d >= 0; --d) c[d] = (d > 0 ? c[d - 1] : 0.0L) - (d < deg ? c[d] * xs[j] : 0.0L);
+      }
+      for (int d = 0; d < n; ++d) M[k * BEM_MAXGEO + d] = (double)(c[d] / den);
+    }
+  };
+  monomials(R.leg_x, nn, R.leg_mono);
+  if (g->ngeo > 0) monomials(R.geo_x, g->ngeo, R.geo_mono);
+  R.p3c_e = bem::nm::p3c_width(1e-14).v;
+  R.p3c_cb = bem::crm::cr_cbrt(1e-14);
 }
 
 }  // namespace

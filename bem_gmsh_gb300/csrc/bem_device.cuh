@@ -46,6 +46,11 @@ struct Rules {
   // product-form weights 1 / prod_{j != i} (x_i - x_j) of the field and CAD
   // nodes (the barycentric weights above carry an arbitrary scale)
   double leg_pw[BEM_MAXNN], geo_pw[BEM_MAXGEO];
+  // the Lagrange bases as polynomials: coefficient of xi^d of basis k at
+  // [k * BEM_MAXGEO + d]
+  double leg_mono[BEM_MAXNN * BEM_MAXGEO], geo_mono[BEM_MAXGEO * BEM_MAXGEO];
+  // the p3c pole's width and cube root for the tangent maps' e0 = 1e-14
+  double p3c_e, p3c_cb;
 };
 
 // Physics of one assembly.

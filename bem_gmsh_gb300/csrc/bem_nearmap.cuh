@@ -171,21 +171,9 @@ BEM_HD int tangenttrans(const RuleT& R, ieee z0, ieee e0, double* x, double* wx)
 
 BEM_HD ieee jsign(ieee v) { return v > ieee(0.0) ? ieee(1.0) : (v < ieee(0.0) ? ieee(-1.0) : ieee(0.0)); }
 
-// _p3c_inv_pole: the p3c pole (zt, et) of (z0, e0), Newton on eq. (65)
-BEM_HD void p3c_inv_pole(ieee z0, ieee e0, ieee& zt, ieee& et) {
-  if (abs(e0) < ieee(1e-14)) {
-    ieee x = z0;
-    for (int it = 0; it < 25; ++it) {
-      ieee g = x * x * x - ieee(3.0) * z0 * (x * x) + ieee(3.0) * x - z0;
-      ieee gp = ieee(3.0) * (x * x) - ieee(6.0) * z0 * x + ieee(3.0);
-      if (abs(gp) < ieee(1e-30)) break;
-      x -= g / gp;
-      if (abs(g) < ieee(1e-14)) break;
-    }
-    zt = x;
-    et = 0.0;
-    return;
-  }
+// first stage of the p3c pole: the width e of a pole at z0 = 0 (20 Newton
+// steps of 2 e^3 - 3 e0 e^2 - e0; it depends on e0 alone)
+BEM_HD ieee p3c_width(ieee e0) {
   ieee e = ieee(crm::cr_cbrt(abs(e0).v)) * jsign(e0);
   for (int it = 0; it < 20; ++it) {
     ieee g = ieee(2.0) * (e * e * e) - ieee(3.0) * e0 * (e * e) - e0;
@@ -193,7 +181,12 @@ BEM_HD void p3c_inv_pole(ieee z0, ieee e0, ieee& zt, ieee& et) {
     if (abs(gp) < ieee(1e-30)) break;
     e -= g / gp;
   }
-  e += ieee(crm::cr_cbrt(e0.v)) * sqrt(z0 * z0 + e0 * e0);
+  return e;
+}
+
+// second stage: Newton on eq. (65) from that width and cb = cbrt(e0)
+BEM_HD void p3c_inv_pole_refine(ieee z0, ieee e0, ieee e, ieee cb, ieee& zt, ieee& et) {
+  e += cb * sqrt(z0 * z0 + e0 * e0);
   ieee z = z0;
   for (int it = 0; it < 30; ++it) {
     ieee den = ieee(1.0) + ieee(3.0) * (z * z) + ieee(3.0) * (e * e);
@@ -218,6 +211,25 @@ BEM_HD void p3c_inv_pole(ieee z0, ieee e0, ieee& zt, ieee& et) {
   }
   zt = z;
   et = e;
+}
+
+// _p3c_inv_pole: the p3c pole (zt, et) of (z0, e0), Newton on eq. (65)
+BEM_HD void p3c_inv_pole(ieee z0, ieee e0, ieee& zt, ieee& et) {
+  if (abs(e0) < ieee(1e-14)) {
+    ieee x = z0;
+    for (int it = 0; it < 25; ++it) {
+      ieee g = x * x * x - ieee(3.0) * z0 * (x * x) + ieee(3.0) * x - z0;
+      ieee gp = ieee(3.0) * (x * x) - ieee(6.0) * z0 * x + ieee(3.0);
+      if (abs(gp) < ieee(1e-30)) break;
+      x -= g / gp;
+      if (abs(g) < ieee(1e-14)) break;
+    }
+    zt = x;
+    et = 0.0;
+    return;
+  }
+  const ieee cb = crm::cr_cbrt(e0.v);
+  p3c_inv_pole_refine(z0, e0, p3c_width(e0), cb, zt, et);
 }
 
 // _p3ctrans

@@ -1,0 +1,27 @@
+"""Near and on-element integrals at the edges of their split over warps and
+lanes, against the oracle: one pair a warp up to 16 (few and many elements),
+1 to 32 rule nodes (a lane with none, or several), 2 to 6 field nodes."""
+import numpy as np
+import pytest
+
+from bem_gmsh_gb300 import star_domain, Elasticity
+from bem_gmsh_gb300.api import H_G_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kelvin", [False, True])
+@pytest.mark.parametrize("ne, p, npg", [(5, 1, 20), (8, 2, 1), (9, 2, 7), (40, 3, 32), (33, 4, 9), (40, 5, 17),
+                                        (300, 1, 8), (700, 2, 16)])
+def test_near_and_own_entries(orc, ne, p, npg, kelvin):
+    if kelvin and ne > 300:
+        ne = 300
+    props = Elasticity(1.0, 0.3) if kelvin else None
+    dad = star_domain(ne, p=p, seed=ne, props=props, pontointerno=True)
+    H, G = H_G_gpu(dad, T=np.float64, npg=npg, store=False)
+    Hr, Gr = orc.assemble(dad, npg=npg, store=False)
+    # the same rule nodes to the bit; up to 64 samples of about 20 rounded
+    # operations each: 64 * 20 * 2^-53 of the largest entry, and a factor 7 for
+    # the cancellation of the basis values
+    assert np.max(np.abs(H - Hr)) <= 1e-12 * np.max(np.abs(Hr))
+    assert np.max(np.abs(G - Gr)) <= 1e-12 * np.max(np.abs(Gr))
