@@ -34,7 +34,7 @@
 #include "bem_lu.h"
 
 int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const double* b, double tol,
-                        int max_iter, int x3, double* x, bem_solve_stats* stats);
+                        int max_iter, int x3, double* x, bem_solve_stats* stats, double* hx = nullptr);
 
 namespace bem {
 namespace {

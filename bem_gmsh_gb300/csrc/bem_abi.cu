@@ -181,6 +181,14 @@ char* bem_ctx::pinned(size_t bytes) {
   return pin;
 }
 
+char* bem_ctx::solver_words() {
+  if (!swords && cudaHostAlloc((void**)&swords, 1024, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    swords = nullptr;
+  }
+  return swords;
+}
+
 cudaEvent_t bem_ctx::timing_event(int i) {
   if (!tev[i] && cudaEventCreate(&tev[i]) != cudaSuccess) {
     cudaGetLastError();
@@ -252,6 +260,7 @@ extern "C" int bem_ctx_destroy(bem_ctx* c) {
   for (auto& b : c->slots)
     if (b.p) cudaFree(b.p);
   if (c->pin) cudaFreeHost(c->pin);
+  if (c->swords) cudaFreeHost(c->swords);
   if (c->pin_ev) cudaEventDestroy(c->pin_ev);
   for (auto e : c->tev)
     if (e) cudaEventDestroy(e);

@@ -75,6 +75,11 @@ struct bem_ctx {
   // marks the end of the last copy issued from the pinned buffer; pinned()
   // waits for it before handing the buffer out again
   void pin_issued();
+  // 1 KB of page-locked words that kernels of a solve write their scalars to
+  // (apart from the staging buffer, whose next use waits for its last copy);
+  // NULL on allocation failure
+  char* solver_words();
+  char* swords = nullptr;
   char* pin = nullptr;
   size_t pin_bytes = 0;
   cudaEvent_t pin_ev = nullptr;

@@ -31,30 +31,34 @@ void lu_couplings(const float* A, int64_t ld, int Npad, const float* Dinv, float
 // and the helpers' partial sums (at most LU_TRSV_PMAX CTAs per block row)
 constexpr int LU_TRSV_PMAX = 4;
 inline size_t lu_tag_words(int Npad) { return (size_t)(2 + 2 * LU_TRSV_PMAX) * (size_t)Npad; }
-// out <- U^{-1} L^{-1} r on padded FP32 vectors.  tmp: Npad floats (the
-// forward result); tags: lu_tag_words(Npad) words of (epoch, value) scratch,
-// zeroed before the first call; epoch: > 0 and different in every call on
-// the same tags; err: timeout flag, set when a wait polled wait_limit times
-// in vain.  wepoch_shift (failure injection, normally 0): results are
+// z <- cs .* U^{-1} L^{-1} v (v, z FP64 of length N, the sweeps FP32) and
+// w <- 0, in one launch.  tags: lu_tag_words(Npad) words of (epoch, value)
+// scratch, zeroed before the first call; epoch: > 0 and different in every
+// call on the same tags; err: timeout flag, set when a wait polled wait_limit
+// times in vain.  rf: 2 Npad floats, used when the block rows do not all stay
+// resident.  wepoch_shift (failure injection, normally 0): results are
 // published under epoch + wepoch_shift, so that a nonzero shift makes every
 // dependent wait run out.  pmax: at most this many CTAs per block row (the
-// count also stays within what the GPU keeps resident).  r may be clobbered.
-// Returns 0 or a CUDA error.
-int lu_solve_vec(const float* A, int64_t ld, int Npad, const float* Dinv, const float* Mc, float* r, float* tmp,
-                 float* out, unsigned long long* tags, int epoch, int* err, cudaStream_t st,
-                 int wait_limit = 1 << 20, int wepoch_shift = 0, int pmax = LU_TRSV_PMAX);
+// count also stays within what the GPU keeps resident).  Returns 0 or a CUDA
+// error.
+int lu_solve_vec(const float* A, int64_t ld, int N, int Npad, const float* Dinv, const float* Mc, const double* v,
+                 const double* cs, double* z, double* w, float* rf, unsigned long long* tags, int epoch, int* err,
+                 cudaStream_t st, int wait_limit = 1 << 20, int wepoch_shift = 0, int pmax = LU_TRSV_PMAX);
 
-void residual64(const double* A, int64_t lda, int N, const double* x, const double* b, double* r,
-                cudaStream_t st);
-void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, cudaStream_t st);
-void dots64(const double* V, int64_t ldv, int N, int m, const double* w, double* h, cudaStream_t st);
-void sub_vh64(const double* V, int64_t ldv, int N, int m, const double* h, double* w, cudaStream_t st);
-void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, cudaStream_t st);
-void scale_copy64(const double* w, double s, double* v, int N, cudaStream_t st);
-// v = w / sqrt(*n2), n2 on the device
-void scale_by_norm64(const double* w, const double* n2, double* v, int N, cudaStream_t st);
-void to_f32(const double* v, int N, int Npad, float* o, cudaStream_t st);
-void from_f32_scale(const float* y, const double* cs, int N, double* z, cudaStream_t st);
+// y += alpha A x
+void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, double alpha, cudaStream_t st);
+// Two passes of classical Gram-Schmidt of w against V[:, 0:m] (m <= 30) and
+// the normalization vn = w / |w|.  host (page-locked, 64 doubles): the
+// coefficients of the passes at [0] and [32], |w|^2 at [62]; hinfo: the two
+// ints at info.
+void gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
+                    int* hinfo, cudaStream_t st);
+// v = r / |r| (zeros for r = 0), x = 0 when given; *host = |r|^2
+void normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
+                 cudaStream_t st);
+// x += Z[:, 0:m] y (y on the host, m <= 32), w = b
+void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
+              cudaStream_t st);
 
 // C (M x N) = beta C + alpha A (M x 128) B (128 x N); M, N multiples of 128.
 void gemm_tile128(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,

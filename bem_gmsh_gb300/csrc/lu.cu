@@ -13,6 +13,7 @@
 // final solution has FP64 accuracy.
 #include <cstdint>
 #include <mutex>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "bem_lu.h"
@@ -546,16 +547,24 @@ __global__ void __launch_bounds__(256) k_lu_couplings(const float* __restrict__ 
 
 // Words per CTA of the partial sums (ptags): 128 (epoch, value) words, P at
 // most TRSV_PMAX CTAs per block row.
+struct TrsvShared {
+  float ys[LU_NB];
+  float part[2][LU_NB];
+  int bad;
+};
+
+// One sweep of k_trsv for this CTA's block row.  Forward (UPPER = false): the
+// right-hand side is v (FP64, N values, zero beyond); backward: the forward
+// sweep's words `rtags`.  The owner publishes y_b in `tags`; backward, it also
+// writes z = cs .* y (FP64) and zeroes w for the product that follows.  false:
+// a wait ran out.
 template <bool UPPER>
-__global__ void __launch_bounds__(256) k_trsv_wave(const float* __restrict__ A, int64_t ld, int K,
-                                                   const float* __restrict__ Dinv, const float* __restrict__ Mc,
-                                                   const float* r, float* y, unsigned long long* tags,
-                                                   unsigned long long* ptags, int P, int epoch, int wepoch,
-                                                   int wait_limit, int* err) {
-  extern __shared__ float Ds[];  // the block's inverse, [col][row], LU_NB * (LU_NB + 1)
-  __shared__ float ys[LU_NB];
-  __shared__ float part[2][LU_NB];
-  __shared__ int bad;
+__device__ __forceinline__ bool trsv_sweep(TrsvShared& sh, float* Ds, const float* __restrict__ A, int64_t ld, int K,
+                                           const float* __restrict__ Dinv, const float* __restrict__ Mc,
+                                           const double* __restrict__ v, int N, const unsigned long long* rtags,
+                                           unsigned long long* tags, unsigned long long* ptags, int P, int epoch,
+                                           int wepoch, int wait_limit, const double* __restrict__ cs,
+                                           double* __restrict__ z, double* __restrict__ w) {
   const int t = threadIdx.x, row = t & (LU_NB - 1), half = t >> 7;
   const int bi = (int)blockIdx.x / P, pp = (int)blockIdx.x % P;
   const bool owner = pp == P - 1;
@@ -565,7 +574,7 @@ __global__ void __launch_bounds__(256) k_trsv_wave(const float* __restrict__ A, 
   const int noff = nj > 1 ? nj - 1 : 0;    // ... but the adjacent one
   // this CTA's share of the non-adjacent blocks, in solve order
   const int s0 = (int)((long long)noff * pp / P), s1 = (int)((long long)noff * (pp + 1) / P);
-  if (t == 0) bad = 0;
+  if (t == 0) sh.bad = 0;
   float mreg[LU_NB / 2];
   if (owner) {
     const float* Db = Dinv + (size_t)b * 2 * LU_NB * LU_NB + (UPPER ? LU_NB * LU_NB : 0);
@@ -580,7 +589,8 @@ __global__ void __launch_bounds__(256) k_trsv_wave(const float* __restrict__ A, 
       for (int q = 0; q < LU_NB / 2; ++q) mreg[q] = Mb[(size_t)(half * (LU_NB / 2) + q) * LU_NB + row];
     }
   }
-  float acc = (owner && half == 0) ? r[rb + row] : 0.f;
+  float acc = 0.f;
+  if (!UPPER && owner && half == 0 && (int)rb + row < N) acc = (float)v[rb + row];
   __syncthreads();
   // waits for the 128 (epoch, value) words at w: each of the first 128
   // threads polls its own word; false when the wait ran out
@@ -591,16 +601,16 @@ __global__ void __launch_bounds__(256) k_trsv_wave(const float* __restrict__ A, 
       int it = 0;
       while ((int)(v >> 32) != epoch) {
         if (++it > wait_limit) {
-          bad = 1;
+          sh.bad = 1;
           break;
         }
         if (it > 8) __nanosleep(32);
         v = ld_acquire_u64(w);
       }
-      ys[t] = __uint_as_float((uint32_t)v);
+      sh.ys[t] = __uint_as_float((uint32_t)v);
     }
     __syncthreads();
-    return bad == 0;
+    return sh.bad == 0;
   };
   // the same, starting from a word loaded earlier (no round trip when its
   // block was already published then)
@@ -612,18 +622,23 @@ __global__ void __launch_bounds__(256) k_trsv_wave(const float* __restrict__ A, 
         int it = 0;
         while ((int)(v >> 32) != epoch) {
           if (++it > wait_limit) {
-            bad = 1;
+            sh.bad = 1;
             break;
           }
           if (it > 8) __nanosleep(32);
           v = ld_acquire_u64(w);
         }
       }
-      ys[t] = __uint_as_float((uint32_t)v);
+      sh.ys[t] = __uint_as_float((uint32_t)v);
     }
     __syncthreads();
-    return bad == 0;
+    return sh.bad == 0;
   };
+  if (UPPER && owner) {
+    if (!fetch(rtags + rb)) return false;
+    if (half == 0) acc = sh.ys[row];
+    __syncthreads();
+  }
   auto blk = [&](int s) { return UPPER ? (K - 1 - s) : s; };
   // this thread's 64 coefficients of block (b, j): row `row`, columns
   // half * 64 .. + 63 (coalesced across the warp)
@@ -667,12 +682,9 @@ __global__ void __launch_bounds__(256) k_trsv_wave(const float* __restrict__ A, 
         for (int q = 0; q < LU_NB / 2; ++q) pb[q] = P1[(size_t)q * ld];
         tb = word(s + 1);
       }
-      if (!fetch_pre(tags + (size_t)blk(s) * LU_NB, ta)) {
-        if (t == 0) atomicExch(err, 1);
-        return;
-      }
+      if (!fetch_pre(tags + (size_t)blk(s) * LU_NB, ta)) return false;
 #pragma unroll
-      for (int q = 0; q < LU_NB / 2; ++q) acc -= pa[q] * ys[half * (LU_NB / 2) + q];
+      for (int q = 0; q < LU_NB / 2; ++q) acc -= pa[q] * sh.ys[half * (LU_NB / 2) + q];
       __syncthreads();
       if (++s >= s1) break;
       if (s + 1 < s1) {
@@ -681,155 +693,271 @@ __global__ void __launch_bounds__(256) k_trsv_wave(const float* __restrict__ A, 
         for (int q = 0; q < LU_NB / 2; ++q) pa[q] = P1[(size_t)q * ld];
         ta = word(s + 1);
       }
-      if (!fetch_pre(tags + (size_t)blk(s) * LU_NB, tb)) {
-        if (t == 0) atomicExch(err, 1);
-        return;
-      }
+      if (!fetch_pre(tags + (size_t)blk(s) * LU_NB, tb)) return false;
 #pragma unroll
-      for (int q = 0; q < LU_NB / 2; ++q) acc -= pb[q] * ys[half * (LU_NB / 2) + q];
+      for (int q = 0; q < LU_NB / 2; ++q) acc -= pb[q] * sh.ys[half * (LU_NB / 2) + q];
       __syncthreads();
       ++s;
     }
   }
-  part[half][row] = acc;
+  sh.part[half][row] = acc;
   __syncthreads();
   unsigned long long* pw = ptags + (size_t)(b * P + pp) * LU_NB;
   if (!owner) {
     // a helper publishes its partial sum (0 for an empty share)
     if (t < LU_NB)
-      st_relaxed_u64(pw + t, ((unsigned long long)(unsigned)wepoch << 32) | __float_as_uint(part[0][t] + part[1][t]));
-    return;
+      st_relaxed_u64(pw + t, ((unsigned long long)(unsigned)wepoch << 32) | __float_as_uint(sh.part[0][t] + sh.part[1][t]));
+    return true;
   }
-  float sum = (t < LU_NB) ? part[0][t] + part[1][t] : 0.f;
+  float sum = (t < LU_NB) ? sh.part[0][t] + sh.part[1][t] : 0.f;
 #pragma unroll
   for (int q = 0; q < LU_TRSV_PMAX - 1; ++q) {
     if (q + 1 >= P) break;
-    if (!fetch_pre(ptags + (size_t)(b * P + q) * LU_NB, pwv[q])) {
-      if (t == 0) atomicExch(err, 1);
-      return;
-    }
-    if (t < LU_NB) sum += ys[t];
+    if (!fetch_pre(ptags + (size_t)(b * P + q) * LU_NB, pwv[q])) return false;
+    if (t < LU_NB) sum += sh.ys[t];
     __syncthreads();
   }
   // z_b = D_b (r_b - ...)
-  if (t < LU_NB) ys[t] = sum;
+  if (t < LU_NB) sh.ys[t] = sum;
   __syncthreads();
   float o0 = 0.f, o1 = 0.f;
 #pragma unroll 16
   for (int q = half * (LU_NB / 2); q < (half + 1) * (LU_NB / 2); q += 2) {
-    o0 += Ds[q * (LU_NB + 1) + row] * ys[q];
-    o1 += Ds[(q + 1) * (LU_NB + 1) + row] * ys[q + 1];
+    o0 += Ds[q * (LU_NB + 1) + row] * sh.ys[q];
+    o1 += Ds[(q + 1) * (LU_NB + 1) + row] * sh.ys[q + 1];
   }
-  part[half][row] = o0 + o1;
+  sh.part[half][row] = o0 + o1;
   __syncthreads();
-  float yb = (t < LU_NB) ? part[0][t] + part[1][t] : 0.f;
+  float yb = (t < LU_NB) ? sh.part[0][t] + sh.part[1][t] : 0.f;
   if (nj > 0) {
     // y_b = z_b - M_b y_adjacent
     __syncthreads();  // part and ys are reused
-    if (!fetch(tags + (size_t)(UPPER ? b + 1 : b - 1) * LU_NB)) {
-      if (t == 0) atomicExch(err, 1);
-      return;
-    }
+    if (!fetch(tags + (size_t)(UPPER ? b + 1 : b - 1) * LU_NB)) return false;
     float m0 = 0.f, m1 = 0.f;
 #pragma unroll
     for (int q = 0; q < LU_NB / 2; q += 2) {
-      m0 = fmaf(mreg[q], ys[half * (LU_NB / 2) + q], m0);
-      m1 = fmaf(mreg[q + 1], ys[half * (LU_NB / 2) + q + 1], m1);
+      m0 = fmaf(mreg[q], sh.ys[half * (LU_NB / 2) + q], m0);
+      m1 = fmaf(mreg[q + 1], sh.ys[half * (LU_NB / 2) + q + 1], m1);
     }
-    part[half][row] = m0 + m1;
+    sh.part[half][row] = m0 + m1;
     __syncthreads();
-    if (t < LU_NB) yb -= part[0][t] + part[1][t];
+    if (t < LU_NB) yb -= sh.part[0][t] + sh.part[1][t];
   }
   if (t < LU_NB) {
-    y[rb + t] = yb;
     st_relaxed_u64(tags + rb + t, ((unsigned long long)(unsigned)wepoch << 32) | __float_as_uint(yb));
+    const int i = (int)rb + t;
+    if (UPPER && i < N) {
+      z[i] = (double)yb * cs[i];
+      w[i] = 0.0;
+    }
   }
+  return true;
+}
+
+// z = cs .* (L U)^{-1} v in one launch: a CTA takes its block row of the
+// forward sweep, then its block row of the backward one (whose inverse and
+// coupling loads so overlap the forward sweep's waits, and the block solved
+// last forward is solved first backward by another CTA without a launch
+// between).
+__global__ void __launch_bounds__(256) k_trsv(const float* __restrict__ A, int64_t ld, int K,
+                                              const float* __restrict__ Dinv, const float* __restrict__ Mc,
+                                              const double* __restrict__ v, int N, const double* __restrict__ cs,
+                                              double* __restrict__ z, double* __restrict__ w,
+                                              unsigned long long* t0, unsigned long long* t1, unsigned long long* p0,
+                                              unsigned long long* p1, int P, int epoch, int wepoch, int wait_limit,
+                                              int* err) {
+  extern __shared__ float Ds[];  // the block's inverse, [col][row], LU_NB * (LU_NB + 1)
+  __shared__ TrsvShared sh;
+  bool ok = trsv_sweep<false>(sh, Ds, A, ld, K, Dinv, Mc, v, N, nullptr, t0, p0, P, epoch, wepoch, wait_limit, cs, z, w);
+  __syncthreads();
+  if (ok) ok = trsv_sweep<true>(sh, Ds, A, ld, K, Dinv, Mc, v, N, t0, t1, p1, P, epoch, wepoch, wait_limit, cs, z, w);
+  if (!ok && threadIdx.x == 0) atomicExch(err, 1);
 }
 
 // ---------------------------------------------------------------------------
 // FP64 vector kernels of the refinement loop
 // ---------------------------------------------------------------------------
-// y = b - A x (FP64), one warp per 4 rows... simple row-parallel version:
-// each thread owns rows; A column-major so threads read consecutive rows.
-__global__ void k_residual64(const double* __restrict__ A, int64_t lda, int N,
-                             const double* __restrict__ x, const double* __restrict__ b,
-                             double* __restrict__ r, int col_chunk) {
-  // 2-D split: blockIdx.y picks a column chunk, partial sums added atomically
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c0 = blockIdx.y * col_chunk;
-  const int c1 = min(N, c0 + col_chunk);
-  if (i >= N) return;
-  double acc = 0.0;
-  for (int c = c0; c < c1; ++c) acc = fma(A[i + (size_t)c * lda], x[c], acc);
-  if (blockIdx.y == 0) acc = b[i] - acc;
-  else acc = -acc;
-  atomicAdd(r + i, acc);
-}
-
-__global__ void k_gemv64(const double* __restrict__ A, int64_t lda, int N,
-                         const double* __restrict__ x, double* __restrict__ y, int col_chunk) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c0 = blockIdx.y * col_chunk;
-  const int c1 = min(N, c0 + col_chunk);
-  if (i >= N) return;
-  double acc = 0.0;
-  for (int c = c0; c < c1; ++c) acc = fma(A[i + (size_t)c * lda], x[c], acc);
-  atomicAdd(y + i, acc);
-}
-
-// h[j] = sum_i V[i, j] w[i] for j < m  (V column-major, ld = N)
-// h[j] += V[:, j] . w over this CTA's slice of the rows (h zeroed before):
-// blockIdx.x = j, blockIdx.y = slice, so each vector is spread over
-// gridDim.y SMs (one SM's FP64 rate is a small fraction of the GPU's)
-__global__ void k_dots(const double* __restrict__ V, int64_t ldv, int N, int m,
-                       const double* __restrict__ w, double* __restrict__ h) {
-  const int j = blockIdx.x;
-  if (j >= m) return;
-  double acc = 0.0;
-  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < N; i += gridDim.y * blockDim.x)
-    acc = fma(V[i + (size_t)j * ldv], w[i], acc);
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  __shared__ double s[32];
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
+// y += alpha A x (FP64), A column-major.  A CTA takes 32 rows (a warp's load
+// is 256 contiguous bytes of a column) and `cols` columns, an eighth of them
+// per warp; its eight partial sums meet in shared memory and one atomic per
+// row adds them to y.  The column split keeps at least 8 columns per warp and
+// spreads a small matrix over all SMs (the loop over 512 columns that every
+// thread ran took 90 us at N = 1023 whatever the GPU had idle: now 5 us);
+// at N = 8193 the bound is FP64 issue, 2 multiply-adds per clock and SM
+// (110 us; measured 136 before, 118 now).
+constexpr int GV_WARPS = 8;
+__global__ void __launch_bounds__(32 * GV_WARPS) k_gemv64(const double* __restrict__ A, int64_t lda, int N,
+                                                          const double* __restrict__ x, double* __restrict__ y,
+                                                          double alpha, int cols) {
+  __shared__ double part[GV_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  const int cw = cols / GV_WARPS;
+  const int c0 = blockIdx.y * cols + warp * cw, c1 = min(N, c0 + cw);
+  const double* a = A + min(i, N - 1) + (size_t)c0 * lda;
+  double s0 = 0.0, s1 = 0.0;
+  int c = c0;
+  for (; c + 8 <= c1; c += 8, a += 8 * lda) {
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = a[(size_t)q * lda];
+#pragma unroll
+    for (int q = 0; q < 8; q += 2) {
+      s0 = fma(v[q], x[c + q], s0);
+      s1 = fma(v[q + 1], x[c + q + 1], s1);
+    }
+  }
+  for (; c < c1; ++c, a += lda) s0 = fma(*a, x[c], s0);
+  part[warp][lane] = s0 + s1;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) r += s[q];
-    atomicAdd(h + j, r);
+  if (warp == 0 && i < N) {
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < GV_WARPS; ++q) s += part[q][lane];
+    atomicAdd(y + i, alpha * s);
   }
 }
 
-// w -= V[:, 0:m] h ; out[i] = w (FP64)
-__global__ void k_sub_vh(const double* __restrict__ V, int64_t ldv, int N, int m,
-                         const double* __restrict__ h, double* __restrict__ w) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    double acc = w[i];
-    for (int j = 0; j < m; ++j) acc = fma(-V[i + (size_t)j * ldv], h[j], acc);
-    w[i] = acc;
+// ---------------------------------------------------------------------------
+// Gram-Schmidt step of the refinement in one cluster of eight CTAs.
+// The vectors are short (N <= 10^4 doubles, all in L2) and the arithmetic is
+// small; what cost was the launches: three dot products, two updates, a
+// normalization, three memsets and a copy to the host, about 30 us of stream
+// time per iteration.  Eight SMs hold an eighth of the rows each; the partial
+// sums meet through distributed shared memory, one cluster barrier per
+// reduction, and the coefficients go straight to the host's page-locked
+// words.  8 us at N = 8193 with five vectors (FP64 issue of eight SMs), 5 us
+// at N = 160.
+// ---------------------------------------------------------------------------
+constexpr int GS_CTAS = 8, GS_THREADS = 512, GS_MAXV = 32;
+
+struct GsShared {
+  double warp[GS_THREADS / 32][GS_MAXV];
+  double part[2][GS_CTAS][GS_MAXV];  // written by the cluster's CTAs
+  double h[GS_MAXV];
+};
+
+// sum over the warp of eight values per lane: lane 4 q holds value q's sum
+// (recursive halving: 9 adds instead of 40)
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int k = 4, o = 16; k >= 1; k >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < k; ++q) {
+      const double send = up ? v[q] : v[q + k], keep = up ? v[q + k] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  double s = v[0];
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+// s.h[0..m) = the cluster's sums of the per-warp sums in s.warp
+__device__ __forceinline__ void gs_reduce(GsShared& s, int m, int buf) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int t = threadIdx.x;
+  __syncthreads();
+  if (t < m * GS_CTAS) {
+    const int q = t % m, to = t / m;
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < GS_THREADS / 32; ++w) v += s.warp[w][q];
+    *cl.map_shared_rank(&s.part[buf][cl.block_rank()][q], to) = v;
+  }
+  cl.sync();
+  if (t < m) {
+    double v = 0.0;
+#pragma unroll
+    for (int r = 0; r < GS_CTAS; ++r) v += s.part[buf][r][t];
+    s.h[t] = v;
+  }
+  __syncthreads();
+}
+
+// w -= V (V^T w) twice (classical Gram-Schmidt with reorthogonalization),
+// vn = w / |w|.  host: [0..31] and [32..61] the two passes' coefficients,
+// [62] |w|^2; hinfo: the two LU status words.
+__global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
+    k_gram_schmidt(const double* __restrict__ V, int64_t ldv, int N, int m, double* w, double* __restrict__ vn,
+                   double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo) {
+  __shared__ GsShared s;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int chunk = (N + GS_CTAS - 1) / GS_CTAS, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int q0 = 0; q0 < m; q0 += 8) {
+      double acc[8] = {};
+      for (int i = i0 + t; i < i1; i += GS_THREADS) {
+        const double wi = w[i];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (q0 + q < m) acc[q] = fma(V[i + (size_t)(q0 + q) * ldv], wi, acc[q]);
+      }
+      const double v = warp_sum8(acc, lane);
+      if ((lane & 3) == 0) s.warp[warp][q0 + (lane >> 2)] = v;
+    }
+    gs_reduce(s, m, pass);
+    if (blockIdx.x == 0 && t < m) host[32 * pass + t] = s.h[t];
+    for (int i = i0 + t; i < i1; i += GS_THREADS) {
+      double a = w[i];
+      for (int q = 0; q < m; ++q) a = fma(-V[i + (size_t)q * ldv], s.h[q], a);
+      w[i] = a;
+    }
+    __syncthreads();
+  }
+  double acc = 0.0;
+  for (int i = i0 + t; i < i1; i += GS_THREADS) acc = fma(w[i], w[i], acc);
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) s.warp[warp][0] = acc;
+  gs_reduce(s, 1, 0);
+  const double n2 = s.h[0], sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+  for (int i = i0 + t; i < i1; i += GS_THREADS) vn[i] = w[i] * sc;
+  if (blockIdx.x == 0 && t == 0) {
+    host[62] = n2;
+    hinfo[0] = info[0];
+    hinfo[1] = info[1];
   }
 }
 
-// x += Z[:, 0:m] y
-__global__ void k_add_zy(const double* __restrict__ Z, int64_t ldz, int N, int m,
-                         const double* __restrict__ y, double* __restrict__ x) {
+// v = r / |r|, |r|^2 to the host; x (when given) zeroed
+__global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
+    k_normalize(const double* __restrict__ r, int N, double* __restrict__ v, double* __restrict__ x,
+                double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo) {
+  __shared__ GsShared s;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int chunk = (N + GS_CTAS - 1) / GS_CTAS, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
+  double acc = 0.0;
+  for (int i = i0 + t; i < i1; i += GS_THREADS) acc = fma(r[i], r[i], acc);
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) s.warp[warp][0] = acc;
+  gs_reduce(s, 1, 0);
+  const double n2 = s.h[0], sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+  for (int i = i0 + t; i < i1; i += GS_THREADS) {
+    v[i] = r[i] * sc;
+    if (x) x[i] = 0.0;
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    *host = n2;
+    hinfo[0] = info[0];
+    hinfo[1] = info[1];
+  }
+}
+
+// x += Z[:, 0:m] y, w = b (the next residual's start)
+struct SmallVec {
+  double v[GS_MAXV];
+};
+__global__ void k_add_zy(const double* __restrict__ Z, int64_t ldz, int N, int m, const __grid_constant__ SmallVec y,
+                         double* __restrict__ x, const double* __restrict__ b, double* __restrict__ w) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
     double acc = x[i];
-    for (int j = 0; j < m; ++j) acc = fma(Z[i + (size_t)j * ldz], y[j], acc);
+    for (int j = 0; j < m; ++j) acc = fma(Z[i + (size_t)j * ldz], y.v[j], acc);
     x[i] = acc;
+    w[i] = b[i];
   }
-}
-
-// v = w / sqrt(*n2) (zeros when *n2 is not positive): normalization by a
-// norm that stays on the device
-__global__ void k_scale_by_norm(const double* __restrict__ w, const double* __restrict__ n2,
-                                double* __restrict__ v, int N) {
-  const double q = *n2;
-  const double s = q > 0.0 ? 1.0 / sqrt(q) : 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) v[i] = w[i] * s;
-}
-
-__global__ void k_scale_copy(const double* __restrict__ w, double s, double* __restrict__ v, int N) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) v[i] = w[i] * s;
 }
 
 // FP64 -> FP32 padded vector
@@ -1756,8 +1884,6 @@ static void lu_solve_vec_steps(const float* A, int64_t ld, int Npad, const float
   }
 }
 
-// y = (L U)^{-1} r on a padded FP32 vector.  r is overwritten with the
-// forward result; the solution lands in `out`.  flags: 2K ints of scratch.
 void lu_couplings(const float* A, int64_t ld, int Npad, const float* Dinv, float* Mc, cudaStream_t st) {
   static std::once_flag once;
   std::call_once(once, [] {
@@ -1770,9 +1896,9 @@ void lu_couplings(const float* A, int64_t ld, int Npad, const float* Dinv, float
   k_lu_couplings<<<dim3(K, 2, 4), 256, CPL_SMEM, st>>>(A, ld, K, Dinv, Mc);
 }
 
-int lu_solve_vec(const float* A, int64_t ld, int Npad, const float* Dinv, const float* Mc, float* r, float* tmp,
-                 float* out, unsigned long long* tags, int epoch, int* err, cudaStream_t st, int wait_limit,
-                 int wepoch_shift, int pmax) {
+int lu_solve_vec(const float* A, int64_t ld, int N, int Npad, const float* Dinv, const float* Mc, const double* v,
+                 const double* cs, double* z, double* w, float* rf, unsigned long long* tags, int epoch, int* err,
+                 cudaStream_t st, int wait_limit, int wepoch_shift, int pmax) {
   const int wepoch = epoch + wepoch_shift;
   const int K = Npad / LU_NB;
   static int max_coresident = 0;
@@ -1782,94 +1908,62 @@ int lu_solve_vec(const float* A, int64_t ld, int Npad, const float* Dinv, const 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int dsm = (int)(sizeof(float) * LU_NB * (LU_NB + 1));
-    cudaFuncSetAttribute(k_trsv_wave<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm);
-    cudaFuncSetAttribute(k_trsv_wave<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trsv_wave<false>, 256, dsm);
+    cudaFuncSetAttribute(k_trsv, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trsv, 256, dsm);
     max_coresident = nsm * per;
   });
   const size_t dsm = sizeof(float) * LU_NB * (LU_NB + 1);
   if (K > max_coresident) {  // too many block rows to keep resident: step-wise launches
-    lu_solve_vec_steps(A, ld, Npad, Dinv, r, tmp, st);
-    cudaMemcpyAsync(out, r, sizeof(float) * Npad, cudaMemcpyDeviceToDevice, st);
-    return 0;
+    k_to_f32<<<(Npad + 255) / 256, 256, 0, st>>>(v, N, Npad, rf);
+    lu_solve_vec_steps(A, ld, Npad, Dinv, rf, rf + Npad, st);
+    k_from_f32_scale<<<(N + 255) / 256, 256, 0, st>>>(rf, cs, N, z);
+    cudaMemsetAsync(w, 0, sizeof(double) * N, st);
+    count_launches(2);
+    return (int)cudaGetLastError();
   }
   // CTAs per block row: as many as stay resident, at most pmax
   const int pcap = pmax < 1 ? 1 : (pmax > LU_TRSV_PMAX ? LU_TRSV_PMAX : pmax);
   int P = max_coresident / K;
   P = P < 1 ? 1 : (P > pcap ? pcap : P);
   KScope ks(st, KC_TRSV);
-  count_launches(2);
+  count_launches(1);
   unsigned long long* t0 = tags;
   unsigned long long* t1 = tags + Npad;
   unsigned long long* p0 = tags + 2 * (size_t)Npad;
   unsigned long long* p1 = p0 + (size_t)LU_TRSV_PMAX * Npad;
-  const dim3 grid(K * P);
-  {
-    void* args[] = {(void*)&A, (void*)&ld, (void*)&K, (void*)&Dinv, (void*)&Mc, (void*)&r, (void*)&tmp,
-                    (void*)&t0, (void*)&p0, (void*)&P, (void*)&epoch, (void*)&wepoch, (void*)&wait_limit,
-                    (void*)&err};
-    // forward: r -> tmp (separate output so that no CTA reads a block another rewrote)
-    cudaError_t e = cudaLaunchCooperativeKernel((void*)k_trsv_wave<false>, grid, dim3(256), args, dsm, st);
-    if (e != cudaSuccess) return (int)e;
-  }
-  {
-    void* args[] = {(void*)&A, (void*)&ld, (void*)&K, (void*)&Dinv, (void*)&Mc, (void*)&tmp, (void*)&out,
-                    (void*)&t1, (void*)&p1, (void*)&P, (void*)&epoch, (void*)&wepoch, (void*)&wait_limit,
-                    (void*)&err};
-    cudaError_t e = cudaLaunchCooperativeKernel((void*)k_trsv_wave<true>, grid, dim3(256), args, dsm, st);
-    if (e != cudaSuccess) return (int)e;
-  }
-  return 0;
+  void* args[] = {(void*)&A,  (void*)&ld, (void*)&K, (void*)&Dinv, (void*)&Mc,    (void*)&v,      (void*)&N,
+                  (void*)&cs, (void*)&z,  (void*)&w, (void*)&t0,   (void*)&t1,    (void*)&p0,     (void*)&p1,
+                  (void*)&P,  (void*)&epoch, (void*)&wepoch, (void*)&wait_limit, (void*)&err};
+  return (int)cudaLaunchCooperativeKernel((void*)k_trsv, dim3(K * P), dim3(256), args, dsm, st);
 }
 
-void residual64(const double* A, int64_t lda, int N, const double* x, const double* b, double* r,
-                cudaStream_t st) {
+void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, double alpha, cudaStream_t st) {
   KScope ks(st, KC_GEMV);
   count_launches(1);
-  cudaMemsetAsync(r, 0, sizeof(double) * N, st);
-  const int chunk = 512;
-  dim3 grid((N + 127) / 128, (N + chunk - 1) / chunk);
-  k_residual64<<<grid, 128, 0, st>>>(A, lda, N, x, b, r, chunk);
+  const int rb = (N + 31) / 32;
+  // column chunks: enough CTAs for 8 per SM, and at least 64 columns each
+  int nc = 152 * 8 / rb, most = (N + 63) / 64;
+  nc = nc < 1 ? 1 : (nc > most ? most : nc);
+  const int cols = ((N + nc - 1) / nc + GV_WARPS - 1) / GV_WARPS * GV_WARPS;
+  k_gemv64<<<dim3(rb, (N + cols - 1) / cols), 32 * GV_WARPS, 0, st>>>(A, lda, N, x, y, alpha, cols);
 }
 
-void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, cudaStream_t st) {
-  KScope ks(st, KC_GEMV);
+void gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
+                    int* hinfo, cudaStream_t st) {
   count_launches(1);
-  cudaMemsetAsync(y, 0, sizeof(double) * N, st);
-  const int chunk = 512;
-  dim3 grid((N + 127) / 128, (N + chunk - 1) / chunk);
-  k_gemv64<<<grid, 128, 0, st>>>(A, lda, N, x, y, chunk);
+  k_gram_schmidt<<<GS_CTAS, GS_THREADS, 0, st>>>(V, ldv, N, m, w, vn, host, info, hinfo);
 }
-
-void dots64(const double* V, int64_t ldv, int N, int m, const double* w, double* h, cudaStream_t st) {
+void normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
+                 cudaStream_t st) {
   count_launches(1);
-  cudaMemsetAsync(h, 0, sizeof(double) * m, st);
-  const int slices = (N + 2047) / 2048 < 16 ? (N + 2047) / 2048 : 16;
-  k_dots<<<dim3(m, slices > 0 ? slices : 1), 256, 0, st>>>(V, ldv, N, m, w, h);
+  k_normalize<<<GS_CTAS, GS_THREADS, 0, st>>>(r, N, v, x, host, info, hinfo);
 }
-void sub_vh64(const double* V, int64_t ldv, int N, int m, const double* h, double* w, cudaStream_t st) {
+void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
+              cudaStream_t st) {
   count_launches(1);
-  k_sub_vh<<<(N + 255) / 256, 256, 0, st>>>(V, ldv, N, m, h, w);
-}
-void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, cudaStream_t st) {
-  count_launches(1);
-  k_add_zy<<<(N + 255) / 256, 256, 0, st>>>(Z, ldz, N, m, y, x);
-}
-void scale_by_norm64(const double* w, const double* n2, double* v, int N, cudaStream_t st) {
-  count_launches(1);
-  k_scale_by_norm<<<(N + 255) / 256, 256, 0, st>>>(w, n2, v, N);
-}
-void scale_copy64(const double* w, double s, double* v, int N, cudaStream_t st) {
-  count_launches(1);
-  k_scale_copy<<<(N + 255) / 256, 256, 0, st>>>(w, s, v, N);
-}
-void to_f32(const double* v, int N, int Npad, float* o, cudaStream_t st) {
-  count_launches(1);
-  k_to_f32<<<(Npad + 255) / 256, 256, 0, st>>>(v, N, Npad, o);
-}
-void from_f32_scale(const float* y, const double* cs, int N, double* z, cudaStream_t st) {
-  count_launches(1);
-  k_from_f32_scale<<<(N + 255) / 256, 256, 0, st>>>(y, cs, N, z);
+  SmallVec yv{};
+  for (int j = 0; j < m; ++j) yv.v[j] = y[j];
+  k_add_zy<<<(N + 127) / 128, 128, 0, st>>>(Z, ldz, N, m, yv, x, b, w);
 }
 
 }  // namespace bem

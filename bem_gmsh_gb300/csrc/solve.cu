@@ -95,30 +95,19 @@ struct Timer {
   }
 };
 
-// <v, w> on the device, read back through the pinned word `hpin`
-double dev_dot(bem_ctx* c, const double* v, const double* w, int N, double* hbuf, double* hpin) {
-  bem::dots64(v, N, N, 1, w, hbuf, c->stream);
-  cudaMemcpyAsync(hpin, hbuf, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-  cudaStreamSynchronize(c->stream);
-  return *hpin;
-}
-
-// Pinned host words of one solve: the Gram-Schmidt coefficients (64), the
-// least-squares solution (32), a dot product, the LU status words.
+// Page-locked host words of one solve, written by the kernels themselves:
+// the Gram-Schmidt coefficients (64), a squared norm, the status words.
 struct SolvePin {
   double* hh;
-  double* y;
   double* dot;
-  int* info;  // 4 ints
+  int* info;  // 4 ints: after the factorization, after the last iteration
 };
 bool solve_pin(bem_ctx* c, SolvePin& p) {
-  char* b = c->pinned(1024);
-  if (!b) return false;
-  double* d = (double*)b;
+  double* d = (double*)c->solver_words();
+  if (!d) return false;
   p.hh = d;
-  p.y = d + 64;
-  p.dot = d + 96;
-  p.info = (int*)(d + 100);
+  p.dot = d + 64;
+  p.info = (int*)(d + 66);
   return true;
 }
 
@@ -134,8 +123,9 @@ void bem_release_solver(bem_ctx* c) {
 // mixed precision: FP32 LU (3xTF32 updates) preconditioning FP64 FGMRES
 // ---------------------------------------------------------------------------
 // A64, b, x: device FP64 (x is output).  A64 is not modified.
+// hx (optional): page-locked host copy of x, made with the last residual.
 int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const double* b,
-                        double tol, int max_iter, int x3, double* x, bem_solve_stats* stats) {
+                        double tol, int max_iter, int x3, double* x, bem_solve_stats* stats, double* hx) {
   const int Npad = (N + LU_NB - 1) / LU_NB * LU_NB;
   const int K = Npad / LU_NB;
   const int m = 30;  // restart length
@@ -146,18 +136,15 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   float* Dinv = (float*)c->get(bem_ctx::SLOT_LU2, sizeof(float) * bem::lu_dinv_floats(K));
   double* V = (double*)c->get(bem_ctx::SLOT_LU3, sizeof(double) * (size_t)N * (m + 1));
   double* Z = (double*)c->get(bem_ctx::SLOT_LU4, sizeof(double) * (size_t)N * m);
-  double* w = (double*)c->get(bem_ctx::SLOT_LU5, sizeof(double) * ((size_t)N + 64));
-  float* rf = (float*)c->get(bem_ctx::SLOT_LU6, sizeof(float) * (3 * (size_t)Npad + 64) +
+  double* w = (double*)c->get(bem_ctx::SLOT_LU5, sizeof(double) * (size_t)N);
+  float* rf = (float*)c->get(bem_ctx::SLOT_LU6, sizeof(float) * (2 * (size_t)Npad + 64) +
                                                    sizeof(unsigned long long) * bem::lu_tag_words(Npad));
   int* info = (int*)c->get(bem_ctx::SLOT_LU7, 256);
   float* Mc = (float*)c->get(bem_ctx::SLOT_LU8, sizeof(float) * (size_t)K * 2 * LU_NB * LU_NB);
   if (!A32 || !cs || !Dinv || !V || !Z || !w || !rf || !info || !Mc) return BEM_ERR_NOMEM;
-  double* hbuf = w + N;  // 64 doubles of scratch
-  float* tmpf = rf + Npad;
-  float* outf = rf + 2 * (size_t)Npad;
   // (epoch, value) words of the triangular sweeps; zeroed once per solve,
   // every preconditioner application uses the next epoch
-  unsigned long long* tags = (unsigned long long*)(rf + 3 * (size_t)Npad + 64);
+  unsigned long long* tags = (unsigned long long*)(rf + 2 * (size_t)Npad + 64);
   cudaMemsetAsync(tags, 0, sizeof(unsigned long long) * bem::lu_tag_words(Npad), c->stream);
   int epoch = 0;
   int* werr = info + 1;
@@ -243,89 +230,68 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   }
   if (rc) return c->cuda_fail((cudaError_t)rc, "lu_factor");
   tf.stop(st);
-  int* hinfo2 = pin.info;
-  cudaMemcpyAsync(hinfo2, info, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaError_t e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return c->cuda_fail(e, "factor");
-  if (stats) stats->t_factor_ms = tf.ms();
-  const int hinfo = hinfo2[0];
-  if (hinfo2[1]) {
-    c->last_error = "tensor-core GEMM wait timed out in the LU";
-    return BEM_ERR_INTERNAL;
-  }
-  if (hinfo != 0) {
-    c->last_error = "vanishing pivot in block " + std::to_string(hinfo - 1) + " of the LU";
-    c->mixed_fail = bem_ctx::MIXED_PIVOT;
-    if (stats) stats->status = BEM_ERR_NOT_CONVERGED;
-    return BEM_ERR_NOT_CONVERGED;
-  }
-  int prc = 0;
-  auto precond = [&](const double* v, double* z) {
-    bem::to_f32(v, N, Npad, rf, st);
-    int e2 = bem::lu_solve_vec(A32, Npad, Npad, Dinv, Mc, rf, tmpf, outf, tags, ++epoch, werr, st,
-                               c->opt_wait_limit, (c->opt_inject & 2) ? 1 : 0, c->opt_sweep_ctas);
-    if (e2) prc = e2;
-    bem::from_f32_scale(outf, cs, N, z, st);
-  };
   tr.start(st);
-  cudaMemsetAsync(x, 0, sizeof(double) * N, st);
-  const double bnorm = std::sqrt(dev_dot(c, b, b, N, hbuf, pin.dot));
-  if (!(bnorm > 0)) {
-    tr.stop(st);
-    if (stats) { stats->iterations = 0; stats->rel_residual = 0; stats->status = BEM_OK; stats->t_refine_ms = tr.ms(); }
-    return BEM_OK;
-  }
-  int iters = 0;
-  double relres = 1.0;
+  // Restarted FGMRES.  Each iteration is three launches (both sweeps of the
+  // preconditioner, the product, the Gram-Schmidt step) and one host
+  // synchronization, after which the page-locked words hold its results; the
+  // first iteration is queued behind the factorization before anything of
+  // either is known.  x = 0 at the start, so the first residual is b.
   std::vector<double> H((m + 1) * m), cg(m), sg(m), gvec(m + 1), y(m);
-  bool converged = false;
-  double prev_beta = INFINITY;
-  bool x_zero = true;  // x was just zeroed: the first residual is b itself
-  while (iters < max_iter && !converged) {
-    // r = b - A x (FP64)
-    if (x_zero)
-      cudaMemcpyAsync(w, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, st);
-    else
-      bem::residual64(A64, lda, N, x, b, w, st);
-    x_zero = false;
-    double beta = std::sqrt(dev_dot(c, w, w, N, hbuf, pin.dot));
-    relres = beta / bnorm;
-    if (relres <= tol) { converged = true; break; }
-    if (beta > 0.5 * prev_beta) {
-      // a restart cycle that no longer halves the true residual.  Below 1e-10
-      // this is the FP64 rounding floor of the matrix (about eps |A| |x| / |b|;
-      // a tol below it cannot be reached): x is then backward stable, as
-      // accurate as FP64 allows -- what the reference's LU returns -- and
-      // counts as converged (stats report the residual reached).
-      if (relres < 1e-10) { converged = true; break; }
-      // far above that floor the same stall means the unpivoted FP32 factors
-      // are no preconditioner for this matrix (pivot growth)
-      c->mixed_fail = bem_ctx::MIXED_STAGNATION;
-      break;
-    }
-    prev_beta = beta;
-    bem::scale_copy64(w, 1.0 / beta, V, N, st);
-    std::fill(gvec.begin(), gvec.end(), 0.0);
-    gvec[0] = beta;
+  bem::normalize64(b, N, V, x, pin.dot, info, pin.info, st);
+  int iters = 0, prc = 0;
+  bool converged = false, first = true;
+  double bnorm = 0.0, beta = 0.0, prev_beta = INFINITY, relres = 1.0;
+  while (!converged) {
     int j = 0;
     for (; j < m && iters < max_iter; ++j) {
-      ++iters;
       double* zj = Z + (size_t)j * N;
-      precond(V + (size_t)j * N, zj);
-      bem::gemv64(A64, lda, N, zj, w, st);
-      // classical Gram-Schmidt, two passes, and the normalization, all on
-      // the device (pass p's coefficients in hbuf[32 p ..], the squared
-      // norm in hbuf[62]); one copy brings them to the host
-      for (int pass = 0; pass < 2; ++pass) {
-        bem::dots64(V, N, N, j + 1, w, hbuf + 32 * pass, st);
-        bem::sub_vh64(V, N, N, j + 1, hbuf + 32 * pass, w, st);
+      int e2 = bem::lu_solve_vec(A32, Npad, N, Npad, Dinv, Mc, V + (size_t)j * N, cs, zj, w, rf, tags, ++epoch, werr,
+                                 st, c->opt_wait_limit, (c->opt_inject & 2) ? 1 : 0, c->opt_sweep_ctas);
+      if (e2) prc = e2;
+      bem::gemv64(A64, lda, N, zj, w, 1.0, st);
+      bem::gram_schmidt64(V, N, N, j + 1, w, V + (size_t)(j + 1) * N, pin.hh, info, pin.info + 2, st);
+      cudaError_t e = cudaStreamSynchronize(st);
+      if (e != cudaSuccess) return c->cuda_fail(e, first ? "factor" : "refinement");
+      if (first) {
+        first = false;
+        if (stats) stats->t_factor_ms = tf.ms();
+        if (pin.info[1]) {
+          c->last_error = "tensor-core GEMM wait timed out in the LU";
+          return BEM_ERR_INTERNAL;
+        }
+        if (pin.info[0] != 0) {
+          c->last_error = "vanishing pivot in block " + std::to_string(pin.info[0] - 1) + " of the LU";
+          c->mixed_fail = bem_ctx::MIXED_PIVOT;
+          if (hx) std::memset(hx, 0, sizeof(double) * N);
+          if (stats) stats->status = BEM_ERR_NOT_CONVERGED;
+          return BEM_ERR_NOT_CONVERGED;
+        }
+        bnorm = beta = prev_beta = std::sqrt(*pin.dot);
+        if (!(bnorm > 0) || tol >= 1.0) {
+          // x = 0 solves it, or is as close as asked for
+          tr.stop(st);
+          if (hx) std::memset(hx, 0, sizeof(double) * N);
+          if (stats) {
+            stats->iterations = 0;
+            stats->rel_residual = bnorm > 0 ? 1.0 : 0.0;
+            stats->status = BEM_OK;
+            stats->t_refine_ms = tr.ms();
+          }
+          return BEM_OK;
+        }
       }
-      bem::dots64(w, N, N, 1, w, hbuf + 62, st);
-      bem::scale_by_norm64(w, hbuf + 62, V + (size_t)(j + 1) * N, N, st);
+      if (prc) return c->cuda_fail((cudaError_t)prc, "triangular solve launch");
+      if (pin.info[3]) {
+        c->last_error = "triangular-solve wait timed out";
+        return BEM_ERR_INTERNAL;
+      }
+      ++iters;
+      if (j == 0) {
+        std::fill(gvec.begin(), gvec.end(), 0.0);
+        gvec[0] = beta;
+      }
       const double* hh = pin.hh;
-      cudaMemcpyAsync(pin.hh, hbuf, sizeof(double) * 64, cudaMemcpyDeviceToHost, st);
-      cudaStreamSynchronize(st);
-      std::vector<double> h(j + 2, 0.0);
+      double h[m + 2];
       for (int q = 0; q <= j; ++q) h[q] = hh[q] + hh[32 + q];
       const double hn = hh[62] > 0.0 ? std::sqrt(hh[62]) : 0.0;
       h[j + 1] = hn;
@@ -345,30 +311,36 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
       for (int q = 0; q <= j; ++q) H[q + (size_t)j * (m + 1)] = h[q];
       if (std::fabs(gvec[j + 1]) / bnorm <= 0.1 * tol || hn == 0.0) { ++j; break; }
     }
-    // y = R^{-1} g, x += Z y
+    // y = R^{-1} g, x += Z y, then the true residual r = b - A x and its norm
     for (int q = j - 1; q >= 0; --q) {
       double s = gvec[q];
       for (int p = q + 1; p < j; ++p) s -= H[q + (size_t)p * (m + 1)] * y[p];
       y[q] = s / H[q + (size_t)q * (m + 1)];
     }
-    std::memcpy(pin.y, y.data(), sizeof(double) * j);
-    cudaMemcpyAsync(hbuf, pin.y, sizeof(double) * j, cudaMemcpyHostToDevice, st);
-    bem::add_zy64(Z, N, N, j, hbuf, x, st);
-  }
-  if (!converged) {
-    bem::residual64(A64, lda, N, x, b, w, st);
-    relres = std::sqrt(dev_dot(c, w, w, N, hbuf, pin.dot)) / bnorm;
+    bem::add_zy64(Z, N, N, j, y.data(), x, b, w, st);
+    bem::gemv64(A64, lda, N, x, w, -1.0, st);
+    bem::normalize64(w, N, V, nullptr, pin.dot, info, pin.info + 2, st);
+    if (hx) cudaMemcpyAsync(hx, x, sizeof(double) * N, cudaMemcpyDeviceToHost, st);
+    tr.stop(st);
+    cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return c->cuda_fail(e, "refinement");
+    beta = std::sqrt(*pin.dot);
+    relres = beta / bnorm;
     converged = relres <= tol;
-  }
-  tr.stop(st);
-  cudaMemcpyAsync(pin.info + 2, werr, sizeof(int), cudaMemcpyDeviceToHost, st);
-  e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return c->cuda_fail(e, "refinement");
-  if (prc) return c->cuda_fail((cudaError_t)prc, "triangular solve launch");
-  const int herr = pin.info[2];
-  if (herr) {
-    c->last_error = "triangular-solve wait timed out";
-    return BEM_ERR_INTERNAL;
+    if (converged || iters >= max_iter) break;
+    if (beta > 0.5 * prev_beta) {
+      // a restart cycle that no longer halves the true residual.  Below 1e-10
+      // this is the FP64 rounding floor of the matrix (about eps |A| |x| / |b|;
+      // a tol below it cannot be reached): x is then backward stable, as
+      // accurate as FP64 allows -- what the reference's LU returns -- and
+      // counts as converged (stats report the residual reached).
+      if (relres < 1e-10) { converged = true; break; }
+      // far above that floor the same stall means the unpivoted FP32 factors
+      // are no preconditioner for this matrix (pivot growth)
+      c->mixed_fail = bem_ctx::MIXED_STAGNATION;
+      break;
+    }
+    prev_beta = beta;
   }
   if (stats) {
     stats->iterations = iters;
@@ -445,8 +417,8 @@ int bem_solve_fp64_dev(bem_ctx* c, int N, double* A64, int64_t lda, const double
 // solved again by LU with partial pivoting in FP64.  A64 is factored in
 // place when `a_scratch` (the caller's copy), otherwise a copy is.
 int bem_solve_mixed_safe(bem_ctx* c, int N, double* A64, int64_t lda, bool a_scratch, const double* b,
-                         double tol, int max_iter, double* x, bem_solve_stats* stats) {
-  int rc = bem_solve_mixed_dev(c, N, A64, lda, b, tol, max_iter, 1, x, stats);
+                         double tol, int max_iter, double* x, bem_solve_stats* stats, double* hx = nullptr) {
+  int rc = bem_solve_mixed_dev(c, N, A64, lda, b, tol, max_iter, 1, x, stats, hx);
   if (rc != BEM_ERR_NOT_CONVERGED || !c->opt_pivot_fallback) return rc;
   if (c->mixed_fail != bem_ctx::MIXED_PIVOT && c->mixed_fail != bem_ctx::MIXED_STAGNATION) return rc;
   double* Af = A64;
@@ -460,6 +432,10 @@ int bem_solve_mixed_safe(bem_ctx* c, int N, double* A64, int64_t lda, bool a_scr
   }
   bem_solve_stats st2{};
   int rc2 = bem_solve_fp64_dev(c, N, Af, ldf, b, x, &st2);
+  if (hx) {
+    cudaMemcpyAsync(hx, x, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream);
+    cudaStreamSynchronize(c->stream);
+  }
   if (stats) {
     stats->pivoted = 1;
     stats->status = st2.status;
@@ -554,18 +530,24 @@ extern "C" int bem_solve2d(bem_ctx* c, const bem_geom2d* g, int kind, double prm
   ta.stop(c->stream);
   if (rc) return rc;
   double t_asm = ta.ms();
-  rc = mode == BEM_SOLVE_MIXED ? bem_solve_mixed_safe(c, N, A, ld, true, b, tol, max_iter, dx, stats)
-                               : bem_solve_fp64_dev(c, N, A, ld, b, dx, stats);
+  double* hx = nullptr;
+  if (mem == BEM_MEM_HOST) {
+    hx = (double*)c->pinned(sizeof(double) * (size_t)N);
+    if (!hx) return BEM_ERR_NOMEM;
+  }
+  if (mode == BEM_SOLVE_MIXED) {
+    rc = bem_solve_mixed_safe(c, N, A, ld, true, b, tol, max_iter, dx, stats, hx);
+  } else {
+    rc = bem_solve_fp64_dev(c, N, A, ld, b, dx, stats);
+    if (hx && (rc == BEM_OK || rc == BEM_ERR_NOT_CONVERGED)) {
+      cudaMemcpyAsync(hx, dx, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream);
+      cudaError_t e = cudaStreamSynchronize(c->stream);
+      if (e != cudaSuccess) return c->cuda_fail(e, "copy x to host");
+    }
+  }
   if (stats) stats->t_assemble_ms = t_asm;
   if (rc != BEM_OK && rc != BEM_ERR_NOT_CONVERGED) return rc;
-  if (mem == BEM_MEM_HOST) {
-    double* hx = (double*)c->pinned(sizeof(double) * (size_t)N);
-    if (!hx) return BEM_ERR_NOMEM;
-    cudaMemcpyAsync(hx, dx, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream);
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return c->cuda_fail(e, "copy x to host");
-    std::memcpy(x, hx, sizeof(double) * N);
-  }
+  if (hx) std::memcpy(x, hx, sizeof(double) * N);
   return rc;
 }
 
