@@ -32,6 +32,7 @@
 
 #include "bem_abi_internal.h"
 #include "bem_lu.h"
+#include "near_coop.cuh"
 
 int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const double* b, double tol,
                         int max_iter, int x3, double* x, bem_solve_stats* stats, double* hx = nullptr);
@@ -49,9 +50,15 @@ struct AdjArgs {
   double* gX;      // 2n: dJ/dx, dJ/dy per node (node-major)
   double* gn;      // 2n: dJ/dn per node
   double* gJ;      // n : dJ/dJacobian per node
+  const float4* rows;    // records and candidate pairs of the assembly
+  const ElemRec* elems;
+  const int2* cand;
+  const int* ncand;
+  int ccap;
   int2* pairs;     // near pairs (i, e)
   int* count;      // [0] near pair count, [1] overflow flag
   int cap;
+  double* S;       // values of the near integrals, neval per pair
 };
 
 // derivative contributions of one far pair (source i, node j) -- nodal
@@ -82,59 +89,121 @@ __device__ __forceinline__ void far_pair_grad(const AdjArgs& a, int i, int j, do
   node5[4] += (aH * H + aG * G) / Jj;  // d/dJ
 }
 
-// Dense pass over (row block of 32) x (element block of 32): exact near test
-// per pair; far pairs get analytic derivatives, near pairs are listed for
-// the finite-difference kernel, on-element pairs are left to the singular
-// kernel.  Warp w takes elements w, w+8, ... of the block; lane = row.
-__global__ void __launch_bounds__(256) adj_far_kernel(AdjArgs a) {
-  __shared__ double s_row[8][32][2];
-  const GeomDev& g = a.g;
-  const int nn = g.nn;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + lane;
-  const bool valid = i < g.n;
-  const int ic = valid ? i : g.n - 1;
-  const V2 pf{g.px[ic], g.py[ic]};
-  double gxi = 0.0, gyi = 0.0;
-  const int e_end = min(g.ne, (int)(blockIdx.y + 1) * 32);
-  for (int e = blockIdx.y * 32 + warp; e < e_end; e += 8) {
-    V2 nodes[BEM_MAXNN];
-    for (int kk = 0; kk < nn; ++kk) nodes[kk] = V2{g.px[e * nn + kk], g.py[e * nn + kk]};
-    const bool on = ic >= e * nn && ic < (e + 1) * nn;
-    const bool near = valid && !on && near_element(pf, nodes, nn, g.elen[e], a.near_factor);
-    if (near) {
-      const int slot = atomicAdd(a.count, 1);
-      if (slot < a.cap) a.pairs[slot] = make_int2(i, e);
-      else a.count[1] = 1;
-    }
-    const bool far = valid && !on && !near;
-    for (int kk = 0; kk < nn; ++kk) {
-      double node5[5] = {0, 0, 0, 0, 0};
-      if (far) far_pair_grad(a, i, e * nn + kk, a.R.ew[kk], gxi, gyi, node5);
+// Analytic derivatives of the far pairs (those that the assembly's box test
+// calls far).  A lane takes one node and walks the CTA's rows, so the five
+// sums per node stay in registers; the two sums per row meet across the lanes
+// eight rows at a time (warp_sum8: 9 adds for 8 sums; with rows on the lanes
+// and five shuffle trees per node the sums were half of the kernel).  With
+//   m = lambda_i / R2,  d = -m (T_j - T_i),  g = -(q_j / k) m - 2 d (r.n) / R2
+// the pair adds J w / 2 pi times  r g + n d  to x_j (minus that to x_i),
+// r d to the normal, and to the Jacobian (d (r.n) - lambda_i q_j log R2 / 2 k)
+// / J: 40 FP64 operations and a box test in FP32.
+constexpr int AF_ROWS = 64;
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 #pragma unroll
-      for (int v = 0; v < 5; ++v)
-        for (int o = 16; o > 0; o >>= 1) node5[v] += __shfl_xor_sync(0xffffffffu, node5[v], o);
-      if (lane == 0) {
-        const int j = e * nn + kk;
-        atomicAdd(a.gX + 2 * j, node5[0]);
-        atomicAdd(a.gX + 2 * j + 1, node5[1]);
-        atomicAdd(a.gn + 2 * j, node5[2]);
-        atomicAdd(a.gn + 2 * j + 1, node5[3]);
-        atomicAdd(a.gJ + j, node5[4]);
-      }
+  for (int k = 4, o = 16; k >= 1; k >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < k; ++q) {
+      const double send = up ? v[q] : v[q + k], keep = up ? v[q + k] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  s_row[warp][lane][0] = gxi;
-  s_row[warp][lane][1] = gyi;
+  double s = v[0];
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+__global__ void __launch_bounds__(128) adj_far_kernel(const __grid_constant__ AdjArgs a) {
+  __shared__ float4 s_row[AF_ROWS];
+  __shared__ double s_x[AF_ROWS], s_y[AF_ROWS], s_l[AF_ROWS], s_T[AF_ROWS];
+  const GeomDev& g = a.g;
+  const int i0 = blockIdx.y * AF_ROWS, nr = min(AF_ROWS, g.n - i0);
+  for (int r = threadIdx.x; r < AF_ROWS; r += blockDim.x) {
+    const int i = min(i0 + r, g.n - 1);
+    s_row[r] = a.rows[i];
+    s_x[r] = g.px[i];
+    s_y[r] = g.py[i];
+    s_l[r] = a.lam[i];
+    s_T[r] = a.T[i];
+  }
   __syncthreads();
-  if (warp == 0 && valid) {
-    double sx = 0.0, sy = 0.0;
-    for (int w = 0; w < 8; ++w) {
-      sx += s_row[w][lane][0];
-      sy += s_row[w][lane][1];
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = j < g.n;
+  const int jc = valid ? j : g.n - 1, e = jc / g.nn;
+  const ElemRec E = a.elems[e];
+  const double xj = g.px[jc], yj = g.py[jc], nx = g.nx[jc], ny = g.ny[jc], J = g.jac[jc];
+  const double Tj = a.T[jc], qk = a.q[jc] / a.k;
+  const double c = J * a.R.ew[jc - e * g.nn] / kTwoPi;
+  double sx = 0.0, sy = 0.0, tx = 0.0, ty = 0.0, sd = 0.0, sl = 0.0;
+  for (int r0 = 0; r0 < nr; r0 += 8) {
+    double vx[8], vy[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int r = r0 + q;
+      vx[q] = vy[q] = 0.0;
+      const float4 rec = s_row[r];
+      if (r < nr && valid && box_far(rec.x, rec.y, rec.z, rec.w, E)) {
+        const double rx = xj - s_x[r], ry = yj - s_y[r], lam = s_l[r];
+        const double R2 = fma(rx, rx, ry * ry), rn = fma(rx, nx, ry * ny);
+        const double inv = f64::rcp(R2), m = lam * inv;
+        const double d = m * (s_T[r] - Tj);
+        const double gm = fma(-2.0 * d, rn * inv, -(qk * m));
+        const double gx = fma(rx, gm, nx * d), gy = fma(ry, gm, ny * d);
+        sx += gx;
+        sy += gy;
+        tx = fma(d, rx, tx);
+        ty = fma(d, ry, ty);
+        sd = fma(d, rn, sd);
+        sl = fma(lam, f64::log(R2), sl);
+        vx[q] = -c * gx;
+        vy[q] = -c * gy;
+      }
     }
-    atomicAdd(a.gX + 2 * i, sx);
-    atomicAdd(a.gX + 2 * i + 1, sy);
+    const double wx = warp_sum8(vx, lane), wy = warp_sum8(vy, lane);
+    const int r = r0 + (lane >> 2);
+    if ((lane & 3) < 2 && r < nr) atomicAdd(a.gX + 2 * (i0 + r) + (lane & 3), (lane & 3) ? wy : wx);
+  }
+  if (valid) {
+    atomicAdd(a.gX + 2 * j, c * sx);
+    atomicAdd(a.gX + 2 * j + 1, c * sy);
+    atomicAdd(a.gn + 2 * j, c * tx);
+    atomicAdd(a.gn + 2 * j + 1, c * ty);
+    atomicAdd(a.gJ + j, c / J * (sd - 0.5 * qk * sl));
+  }
+}
+
+// The assembly's candidate pairs by the exact near test: near pairs are
+// listed for the difference kernels, the others get their far derivatives.
+__global__ void __launch_bounds__(128) adj_pairs_kernel(const __grid_constant__ AdjArgs a) {
+  const GeomDev& g = a.g;
+  const int nn = g.nn, count = min(*a.ncand, a.ccap);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+    const int2 pr = a.cand[t];
+    const int i = pr.x, e = pr.y;
+    V2 nodes[BEM_MAXNN];
+    for (int kk = 0; kk < nn; ++kk) nodes[kk] = V2{g.px[e * nn + kk], g.py[e * nn + kk]};
+    if (near_element(V2{g.px[i], g.py[i]}, nodes, nn, g.elen[e], a.near_factor)) {
+      const int slot = atomicAdd(a.count, 1);
+      if (slot < a.cap) a.pairs[slot] = pr;
+      else a.count[1] = 1;
+      continue;
+    }
+    double gxi = 0.0, gyi = 0.0;
+    for (int kk = 0; kk < nn; ++kk) {
+      double node5[5] = {0, 0, 0, 0, 0};
+      const int j = e * nn + kk;
+      far_pair_grad(a, i, j, a.R.ew[kk], gxi, gyi, node5);
+      atomicAdd(a.gX + 2 * j, node5[0]);
+      atomicAdd(a.gX + 2 * j + 1, node5[1]);
+      atomicAdd(a.gn + 2 * j, node5[2]);
+      atomicAdd(a.gn + 2 * j + 1, node5[3]);
+      atomicAdd(a.gJ + j, node5[4]);
+    }
+    atomicAdd(a.gX + 2 * i, gxi);
+    atomicAdd(a.gX + 2 * i + 1, gyi);
   }
 }
 
@@ -169,87 +238,222 @@ __device__ double near_value(const AdjArgs& a, int i, int e, const V2* nodes, V2
   return s;
 }
 
-// one thread per near pair: central differences w.r.t. the source point and
-// the element's node coordinates
-__global__ void __launch_bounds__(64) adj_near_kernel(AdjArgs a) {
-  const int cnt = min(a.count[0], a.cap);
+// The near integrals of a pair are wanted at its nodes and source as they
+// are (value 0) and with each coordinate c moved by +h (value 2 c + 1) and -h
+// (2 c + 2), h = 1e-5 element lengths: c = 0, 1 the source, then the nodes.
+__device__ __forceinline__ int near_values(int nn) { return 1 + 2 * (2 + 2 * nn); }
+
+template <int NN>
+__device__ __forceinline__ void perturb(int ev, double h, V2& pf, V2* nodes) {
+  const int c = (ev - 1) >> 1;
+  const double d = ev == 0 ? 0.0 : ((ev & 1) ? h : -h);
+  if (ev > 0 && c == 0) pf.x += d;
+  if (ev > 0 && c == 1) pf.y += d;
+#pragma unroll
+  for (int k = 0; k < NN; ++k) {
+    if (ev > 0 && c == 2 + 2 * k) nodes[k].x += d;
+    if (ev > 0 && c == 3 + 2 * k) nodes[k].y += d;
+  }
+}
+
+// one value by one thread: the near-field maps other than tanp3c, and the
+// pairs that take none of its regular branches
+__device__ __noinline__ void near_value_general(const AdjArgs& a, int i, int e, int ev, double* out) {
   const GeomDev& g = a.g;
-  const int nn = g.nn;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-    const int2 pr = a.pairs[t];
-    const int i = pr.x, e = pr.y;
-    V2 nodes[BEM_MAXNN];
-    for (int kk = 0; kk < nn; ++kk) nodes[kk] = V2{g.px[e * nn + kk], g.py[e * nn + kk]};
-    V2 pf{g.px[i], g.py[i]};
-    const double h = 1e-5 * g.elen[e];
-    const double s0 = near_value(a, i, e, nodes, pf);
-    for (int d = 0; d < 2; ++d) {
-      double* c = d == 0 ? &pf.x : &pf.y;
-      const double c0 = *c;
-      *c = c0 + h;
-      const double sp = near_value(a, i, e, nodes, pf);
-      *c = c0 - h;
-      const double sm = near_value(a, i, e, nodes, pf);
-      *c = c0;
-      atomicAdd(a.gX + 2 * i + d, fd_slope(sm, s0, sp, h));
+  V2 nodes[BEM_MAXNN];
+  for (int k = 0; k < g.nn; ++k) nodes[k] = V2{g.px[e * g.nn + k], g.py[e * g.nn + k]};
+  V2 pf{g.px[i], g.py[i]};
+  if (ev > 0) {
+    const int c = (ev - 1) >> 1;
+    const double d = (ev & 1) ? 1e-5 * g.elen[e] : -1e-5 * g.elen[e];
+    if (c == 0) pf.x += d;
+    else if (c == 1) pf.y += d;
+    else if (c & 1) nodes[(c - 2) >> 1].y += d;
+    else nodes[(c - 2) >> 1].x += d;
+  }
+  *out = near_value(a, i, e, nodes, pf);
+}
+
+__global__ void __launch_bounds__(64) adj_near_general_kernel(const __grid_constant__ AdjArgs a) {
+  const int ne = near_values(a.g.nn), cnt = min(a.count[0], a.cap);
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)cnt * ne;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int2 pr = a.pairs[t / ne];
+    near_value_general(a, pr.x, pr.y, (int)(t % ne), a.S + t);
+  }
+}
+
+// The values by warps, 16 at a time (near_coop.cuh).  One thread per pair
+// went through its 17 integrals (quadratic elements) one after another: at
+// 1023 nodes 2730 threads, four per scheduler, 4.7 ms; now 46 000 values fill
+// the GPU and share their lanes.
+template <int NN>
+__global__ void __launch_bounds__(128) adj_near_kernel(const __grid_constant__ AdjArgs a) {
+  using namespace coop;
+  __shared__ Slot s_slots[4][PAIRS];
+  __shared__ double s_q[BEM_MAXNPG], s_w[BEM_MAXNPG];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const GeomDev& g = a.g;
+  const Rules& R = a.R;
+  const int nev = near_values(NN);
+  const int64_t count = (int64_t)min(a.count[0], a.cap) * nev;
+  const int nwarps = gridDim.x * 4, gw = warp * gridDim.x + blockIdx.x;
+  for (int q = threadIdx.x; q < R.npg; q += blockDim.x) {
+    s_q[q] = R.qsi[q];
+    s_w[q] = R.w[q];
+  }
+  __syncthreads();
+  Physics ph{};
+  ph.k = a.k;
+  const Consts kc = make_consts<1>(ph);
+  Slot* slots = s_slots[warp];
+  for (int64_t base = (int64_t)gw * PAIRS; base < count; base += (int64_t)nwarps * PAIRS) {
+    const int np = (int)min((int64_t)PAIRS, count - base);
+    if (lane < np) {
+      const int64_t t = base + lane;
+      const int2 pr = a.pairs[t / nev];
+      const int i = pr.x, e = pr.y;
+      Slot& s = slots[lane];
+      V2 nodes[NN];
+#pragma unroll
+      for (int k = 0; k < NN; ++k) nodes[k] = V2{g.px[e * NN + k], g.py[e * NN + k]};
+      V2 pf{g.px[i], g.py[i]};
+      perturb<NN>((int)(t % nev), 1e-5 * g.elen[e], pf, nodes);
+      s.kind = K_TANGENT;
+#pragma unroll
+      for (int k = 0; k < NN; ++k) {
+        s.cx[k] = nodes[k].x;
+        s.cy[k] = nodes[k].y;
+      }
+      s.sx = pf.x;
+      s.sy = pf.y;
+      s.nrx = g.nx[e * NN];
+      s.nry = g.ny[e * NN];
+      complex_pole_1d(R, nodes, NN, pf, s.z0, s.e0);
     }
-    for (int kk = 0; kk < nn; ++kk) {
-      for (int d = 0; d < 2; ++d) {
-        double* c = d == 0 ? &nodes[kk].x : &nodes[kk].y;
-        const double c0 = *c;
-        *c = c0 + h;
-        const double sp = near_value(a, i, e, nodes, pf);
-        *c = c0 - h;
-        const double sm = near_value(a, i, e, nodes, pf);
-        *c = c0;
-        atomicAdd(a.gX + 2 * (e * nn + kk) + d, fd_slope(sm, s0, sp, h));
+    __syncwarp();
+    map_constants(R, slots, np, lane);
+    constexpr int G = 8;
+    const int lg = lane & (G - 1);
+    for (int p0 = 0; p0 < np; p0 += 32 / G) {
+      const int p = p0 + lane / G;
+      const bool valid = p < np;
+      const Slot& s = slots[valid ? p : 0];
+      const int kind = valid ? s.kind : K_NONE;
+      double h[NN], gg[NN];
+      integrate_group<1, NN, true>(s, kind == K_TANGENT || kind == K_REALPOLE, R.npg, s_q, s_w, R, NN, kc, lg, G, h,
+                                   gg);
+      // S = sum_k a_k h_k + c_k g_k, this lane's nodes; then over the lanes
+      double S = 0.0;
+      const int64_t t = base + p;
+      int2 pr = make_int2(0, 0);
+      if (valid) {
+        pr = a.pairs[t / nev];
+        const double lam = a.lam[pr.x], Ti = a.T[pr.x];
+#pragma unroll
+        for (int k = 0; k < NN; ++k) {
+          const int j = pr.y * NN + k;
+          S += -lam * (a.T[j] - Ti) * h[k] + lam * a.q[j] * gg[k];
+        }
+      }
+      for (int o = G >> 1; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
+      if (valid && lg == 0) {
+        if (kind == K_GENERAL) near_value_general(a, pr.x, pr.y, (int)(t % nev), a.S + t);
+        else a.S[t] = S;
       }
     }
+    __syncwarp();
   }
 }
 
-__device__ double singular_value(const AdjArgs& a, int i, int e, const V2* nodes) {
+// slopes of the near integrals from their values
+__global__ void __launch_bounds__(128) adj_near_slope_kernel(const __grid_constant__ AdjArgs a) {
+  const int nn = a.g.nn, nev = near_values(nn), nc = 2 + 2 * nn;
+  const int64_t count = (int64_t)min(a.count[0], a.cap) * nc;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = t / nc;
+    const int c = (int)(t - p * nc);
+    const int2 pr = a.pairs[p];
+    const double* S = a.S + p * nev;
+    const double h = 1e-5 * a.g.elen[pr.y];
+    const int at = c < 2 ? 2 * pr.x + c : 2 * (pr.y * nn + ((c - 2) >> 1)) + (c & 1);
+    atomicAdd(a.gX + at, fd_slope(S[2 * c + 2], S[0], S[2 * c + 1], h));
+  }
+}
+
+// On-element integrals, node coordinates perturbed (the source is one of
+// them): four lanes per value with the rule's sample weights (singular_table),
+// 1 + 4 NN values per node, their differences within the CTA.  The rule run
+// step by step by one thread per node, 13 times over, took 2.5 ms at 1023
+// quadratic nodes.
+template <int NN>
+__global__ void __launch_bounds__(128) adj_singular_kernel(const __grid_constant__ AdjArgs a,
+                                                           const __grid_constant__ SingularTable<NN> tab) {
+  constexpr int NB = 8, NEV = 1 + 4 * NN;  // nodes per CTA, values per node
+  __shared__ double s_tab[sizeof(SingularTable<NN>) / 8];
+  __shared__ double s_S[NB * NEV];
+  for (int q = threadIdx.x; q < (int)(sizeof(tab) / 8); q += blockDim.x) s_tab[q] = ((const double*)&tab)[q];
+  __syncthreads();
+  const SingularTable<NN>& W = *(const SingularTable<NN>*)s_tab;
   const GeomDev& g = a.g;
-  const int nn = g.nn, ai = i - e * nn;
-  V2 geo[BEM_MAXGEO];
-  double h[BEM_MAXNN], gg[BEM_MAXNN];
   Physics ph{};
-  ph.kind = 0;
   ph.k = a.k;
-  const V2 nref{g.nx[e * nn], g.ny[e * nn]};
-  integrate_singular<1>(a.R, ph, nodes, geo, nodes[ai], a.R.leg_x[ai], nref, h, gg);
-  double s = 0.0;
-  for (int kk = 0; kk < nn; ++kk) {
-    const int j = e * nn + kk;
-    if (kk != ai) s += -a.lam[i] * (a.T[j] - a.T[i]) * h[kk];
-    s += a.lam[i] * a.q[j] * gg[kk];
-  }
-  return s;
-}
-
-// one thread per boundary node: its own element, node coordinates perturbed
-// (the source is one of them)
-__global__ void __launch_bounds__(64) adj_singular_kernel(AdjArgs a) {
-  const GeomDev& g = a.g;
-  const int nn = g.nn;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.n) return;
-  const int e = i / nn;
-  V2 nodes[BEM_MAXNN];
-  for (int kk = 0; kk < nn; ++kk) nodes[kk] = V2{g.px[e * nn + kk], g.py[e * nn + kk]};
-  const double h = 1e-5 * g.elen[e];
-  const double s0 = singular_value(a, i, e, nodes);
-  for (int kk = 0; kk < nn; ++kk) {
-    for (int d = 0; d < 2; ++d) {
-      double* c = d == 0 ? &nodes[kk].x : &nodes[kk].y;
-      const double c0 = *c;
-      *c = c0 + h;
-      const double sp = singular_value(a, i, e, nodes);
-      *c = c0 - h;
-      const double sm = singular_value(a, i, e, nodes);
-      *c = c0;
-      atomicAdd(a.gX + 2 * (e * nn + kk) + d, fd_slope(sm, s0, sp, h));
+  const coop::Consts kc = coop::make_consts<1>(ph);
+  const int l = threadIdx.x & 3;
+  for (int v0 = 0; v0 < NB * NEV; v0 += 32) {
+    const int v = v0 + (threadIdx.x >> 2);
+    const int vn = min(v / NEV, NB - 1), ev = v - vn * NEV;
+    const int i = min((int)blockIdx.x * NB + vn, g.n - 1);
+    const int e = i / NN, ai = i - e * NN;
+    V2 nodes[NN], pf{0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < NN; ++k) nodes[k] = V2{g.px[e * NN + k], g.py[e * NN + k]};
+    // node coordinate c as coordinate c + 2 of the near values
+    perturb<NN>(ev == 0 ? 0 : ev + 4, 1e-5 * g.elen[e], pf, nodes);
+#pragma unroll
+    for (int k = 0; k < NN; ++k)
+      if (k == ai) pf = nodes[k];
+    double X[NN], Y[NN];
+#pragma unroll
+    for (int k = 0; k < NN; ++k) {
+      X[k] = nodes[k].x;
+      Y[k] = nodes[k].y;
     }
+    const double nrx = g.nx[e * NN], nry = g.ny[e * NN];
+    const double lam = a.lam[i], Ti = a.T[i];
+    double ch[NN], cg[NN];
+#pragma unroll
+    for (int k = 0; k < NN; ++k) {
+      ch[k] = k == ai ? 0.0 : -lam * (a.T[e * NN + k] - Ti);
+      cg[k] = lam * a.q[e * NN + k];
+    }
+    double S = 0.0;
+    for (int q = l; q < BEM_NINTERP; q += 4) {
+      double rx, ry, dx, dy;
+      coop::nodal_point<NN>(X, Y, W.N[q], W.D[q], pf.x, pf.y, rx, ry, dx, dy);
+      const double J2 = fma(dx, dx, dy * dy), R2 = fma(rx, rx, ry * ry);
+      if (J2 < 1e-60 || R2 < 1e-60) continue;
+      const double flip = dy * nrx - dx * nry < 0 ? -1.0 : 1.0;
+      double U, T, wh = 0.0, wg = 0.0;
+      coop::kernel_values<1>(kc, rx, ry, flip * dy, -(flip * dx), &U, &T);
+#pragma unroll
+      for (int k = 0; k < NN; ++k) {
+        wh = fma(W.Wh[ai][q][k], ch[k], wh);
+        wg = fma(W.Wg[ai][q][k], cg[k], wg);
+      }
+      S = fma(wh, T, fma(wg, U * f64::sqrt(J2), S));
+    }
+    S += __shfl_xor_sync(0xffffffffu, S, 1);
+    S += __shfl_xor_sync(0xffffffffu, S, 2);
+    if (l == 0 && v < NB * NEV) s_S[v] = S;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < NB * 2 * NN; t += blockDim.x) {
+    const int vn = t / (2 * NN), c = t - vn * 2 * NN, i = blockIdx.x * NB + vn;
+    if (i >= g.n) continue;
+    const int e = i / NN;
+    const double* S = s_S + vn * NEV;
+    atomicAdd(a.gX + 2 * (e * NN + (c >> 1)) + (c & 1), fd_slope(S[2 * c + 2], S[0], S[2 * c + 1], 1e-5 * g.elen[e]));
   }
 }
 
@@ -387,9 +591,11 @@ extern "C" int bem_adjoint_laplace2d(bem_ctx* c, const bem_geom2d* g, double k, 
   rc = bem_stage_geom(c, g, npg, mem, gd, R);
   if (rc) return rc;
   const int cap = 32 * n + 1024;
-  int2* pairs = (int2*)c->get(bem_ctx::SLOT_PAIRS, sizeof(int2) * (size_t)cap);
-  int* cnt = (int*)c->get(bem_ctx::SLOT_COUNTERS, 64);
-  if (!pairs || !cnt) return BEM_ERR_NOMEM;
+  const int nev = 1 + 2 * (2 + 2 * gd.nn);
+  // near pairs and their values; the candidates and records are the assembly's
+  char* np = (char*)c->get(bem_ctx::SLOT_ADJ2, (sizeof(double) * nev + sizeof(int2)) * (size_t)cap);
+  int* cnt = (int*)c->get(bem_ctx::SLOT_COUNTERS, 64) + 4;
+  if (!np || !cnt) return BEM_ERR_NOMEM;
   cudaMemsetAsync(cnt, 0, 2 * sizeof(int), c->stream);
   cudaMemsetAsync(gX, 0, sizeof(double) * 5 * (size_t)N, c->stream);
   AdjArgs aa{};
@@ -403,14 +609,38 @@ extern "C" int bem_adjoint_laplace2d(bem_ctx* c, const bem_geom2d* g, double k, 
   aa.gX = gX;
   aa.gn = gn;
   aa.gJ = gJ;
-  aa.pairs = pairs;
+  aa.rows = (const float4*)c->slots[bem_ctx::SLOT_ROWS].p;
+  aa.elems = (const ElemRec*)c->slots[bem_ctx::SLOT_ELEMS].p;
+  aa.cand = (const int2*)c->slots[bem_ctx::SLOT_PAIRS].p;
+  aa.ncand = cnt - 4;
+  aa.ccap = (int)std::min<size_t>(c->slots[bem_ctx::SLOT_PAIRS].bytes / sizeof(int2), 0x7fffffff);
+  aa.S = (double*)np;
+  aa.pairs = (int2*)(np + sizeof(double) * nev * (size_t)cap);
   aa.count = cnt;
   aa.cap = cap;
-  adj_far_kernel<<<dim3((n + 31) / 32, (g->ne + 31) / 32), 256, 0, c->stream>>>(aa);
-  adj_near_kernel<<<(cap + 63) / 64 < 4096 ? (cap + 63) / 64 : 4096, 64, 0, c->stream>>>(aa);
-  adj_singular_kernel<<<(n + 63) / 64, 64, 0, c->stream>>>(aa);
+  adj_pairs_kernel<<<std::min((8 * n + 127) / 128, 152 * 16), 128, 0, c->stream>>>(aa);
+  adj_far_kernel<<<dim3((n + 127) / 128, (n + AF_ROWS - 1) / AF_ROWS), 128, 0, c->stream>>>(aa);
+  if (R.nearfield != 0) {
+    adj_near_general_kernel<<<4096, 64, 0, c->stream>>>(aa);
+  } else {
+    switch (gd.nn) {
+      case 2: adj_near_kernel<2><<<304, 128, 0, c->stream>>>(aa); break;
+      case 3: adj_near_kernel<3><<<304, 128, 0, c->stream>>>(aa); break;
+      case 4: adj_near_kernel<4><<<304, 128, 0, c->stream>>>(aa); break;
+      case 5: adj_near_kernel<5><<<304, 128, 0, c->stream>>>(aa); break;
+      case 6: adj_near_kernel<6><<<304, 128, 0, c->stream>>>(aa); break;
+    }
+  }
+  adj_near_slope_kernel<<<std::min((16 * n + 127) / 128, 152 * 16), 128, 0, c->stream>>>(aa);
+  switch (gd.nn) {
+    case 2: adj_singular_kernel<2><<<(n + 7) / 8, 128, 0, c->stream>>>(aa, singular_table<2>(R)); break;
+    case 3: adj_singular_kernel<3><<<(n + 7) / 8, 128, 0, c->stream>>>(aa, singular_table<3>(R)); break;
+    case 4: adj_singular_kernel<4><<<(n + 7) / 8, 128, 0, c->stream>>>(aa, singular_table<4>(R)); break;
+    case 5: adj_singular_kernel<5><<<(n + 7) / 8, 128, 0, c->stream>>>(aa, singular_table<5>(R)); break;
+    case 6: adj_singular_kernel<6><<<(n + 7) / 8, 128, 0, c->stream>>>(aa, singular_table<6>(R)); break;
+  }
   adj_chain_kernel<<<(g->ne + 127) / 128, 128, 0, c->stream>>>(aa);
-  count_launches(4);
+  count_launches(6);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return c->cuda_fail(e, "adjoint kernels");
   // gradient, J and the pair counters back through the pinned buffer

@@ -174,17 +174,6 @@ __global__ void pack_elems_kernel(GeomDev g, double near_factor, const unsigned 
   el[e] = r;
 }
 
-// Conservative box test of a source point (x, y) against an element record:
-// true when the pair is far for the exact FP64 test as well.  Explicit
-// round-to-nearest operations, so that the classification kernel and the far
-// kernel agree bit for bit.
-__device__ __forceinline__ bool box_far(float xh, float xl, float yh, float yl, const ElemRec& E) {
-  const float x = __fadd_rn(xh, xl), y = __fadd_rn(yh, yl);
-  const float dx = fmaxf(fmaxf(__fsub_rn(E.lox, x), __fsub_rn(x, E.hix)), 0.f);
-  const float dy = fmaxf(fmaxf(__fsub_rn(E.loy, y), __fsub_rn(y, E.hiy)), 0.f);
-  return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) > E.lim2;
-}
-
 // Possibly-near (point, element) pairs into the pair list: one thread per
 // point, the CTA's 256 elements staged in shared memory.  Each warp first
 // tests an element against the bounding box of its 32 points with the same

@@ -9,15 +9,6 @@
 
 namespace bem {
 
-// on-element rule of an element type with NN field nodes: geometry basis and
-// derivative at the 20 samples, sample weights of each field node's integrals
-// for each source node
-template <int NN>
-struct SingularTable {
-  double N[BEM_NINTERP][BEM_MAXGEO], D[BEM_NINTERP][BEM_MAXGEO];
-  double Wh[NN][BEM_NINTERP][NN], Wg[NN][BEM_NINTERP][NN];
-};
-
 // ---------------------------------------------------------------------------
 // near kernel: listed pairs, exact FP64 test, tanp3c or FP64 lumping
 // ---------------------------------------------------------------------------
@@ -170,8 +161,7 @@ __global__ void __launch_bounds__(128) near_kernel(const __grid_constant__ NearA
       const Slot& s = slots[valid ? p : 0];
       const int kind = valid ? s.kind : K_NONE;
       double h[NN * NC], gg[NN * NC];
-      integrate_group<NC, NN>(s, kind == K_TANGENT || kind == K_REALPOLE, R.npg, s_q, s_w, R.leg_x, R.leg_pw, ng, kc,
-                              lg, G, h, gg);
+      integrate_group<NC, NN>(s, kind == K_TANGENT || kind == K_REALPOLE, R.npg, s_q, s_w, R, ng, kc, lg, G, h, gg);
       int i = 0, e = 0;
       if (valid) {
         const int2 pr = a.pairs[s.id];
@@ -362,17 +352,27 @@ template <int NN>
 static void singular_weights(const Rules& R, SingularTable<NN>& W) {
   constexpr int M = BEM_NINTERP;
   using T = long double;
+  // geometry basis at the samples: the operations of shapefun_prod (its
+  // derivative sums contracted as the compiler does on the device)
+  const int ng = R.ngeo > 0 ? R.ngeo : NN;
+  const double* gx = R.ngeo > 0 ? R.geo_x : R.leg_x;
+  const double* gpw = R.ngeo > 0 ? R.geo_pw : R.leg_pw;
+  const double* gD = R.ngeo > 0 ? R.geo_D : R.leg_D;
   for (int q = 0; q < M; ++q) {
-    const int ng = R.ngeo > 0 ? R.ngeo : NN;
-    const double* mono = R.ngeo > 0 ? R.geo_mono : R.leg_mono;
-    for (int k = 0; k < BEM_MAXGEO; ++k) {
-      T v = 0, d = 0;
-      for (int c = ng - 1; c >= 0 && k < ng; --c) {
-        d = d * R.gi_x[q] + v;
-        v = v * R.gi_x[q] + mono[k * BEM_MAXGEO + c];
-      }
-      W.N[q][k] = (double)v;
-      W.D[q][k] = (double)d;
+    double* N = W.N[q];
+    double pre = 1.0, suf = 1.0;
+    for (int k = 0; k < ng; ++k) {
+      N[k] = gpw[k] * pre;
+      pre *= R.gi_x[q] - gx[k];
+    }
+    for (int k = ng - 1; k >= 0; --k) {
+      N[k] *= suf;
+      suf *= R.gi_x[q] - gx[k];
+    }
+    for (int k = 0; k < ng; ++k) {
+      double d = N[0] * gD[k];
+      for (int i = 1; i < ng; ++i) d = std::fma(N[i], gD[i * ng + k], d);
+      W.D[q][k] = d;
     }
   }
   for (int ai = 0; ai < NN; ++ai) {
@@ -486,14 +486,18 @@ void launch_near_pairs(const NearArgs& na, int nc, cudaStream_t st) {
   else launch_near_nc<4>(na, st);
 }
 
-// the table of an element type, built once per process (ngeo 0..6)
 template <int NN>
-static const SingularTable<NN>& singular_table(const Rules& R) {
+const SingularTable<NN>& singular_table(const Rules& R) {
   static SingularTable<NN> tab[BEM_MAXGEO + 1];
   static std::once_flag once[BEM_MAXGEO + 1];
   std::call_once(once[R.ngeo], [&] { singular_weights<NN>(R, tab[R.ngeo]); });
   return tab[R.ngeo];
 }
+template const SingularTable<2>& singular_table<2>(const Rules&);
+template const SingularTable<3>& singular_table<3>(const Rules&);
+template const SingularTable<4>& singular_table<4>(const Rules&);
+template const SingularTable<5>& singular_table<5>(const Rules&);
+template const SingularTable<6>& singular_table<6>(const Rules&);
 
 template <int NC, int NN>
 static void launch_singular_nn(const NearArgs& na, int n, cudaStream_t st) {

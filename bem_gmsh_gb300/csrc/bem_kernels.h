@@ -44,6 +44,30 @@ struct __align__(16) ElemRec {
   float lim2, pad0, pad1, pad2;
 };
 
+#ifdef __CUDACC__
+// Conservative box test of a source point (x, y) against an element record:
+// true when the pair is far for the exact FP64 test as well.  Explicit
+// round-to-nearest operations, so that every kernel agrees bit for bit.
+__device__ __forceinline__ bool box_far(float xh, float xl, float yh, float yl, const ElemRec& E) {
+  const float x = __fadd_rn(xh, xl), y = __fadd_rn(yh, yl);
+  const float dx = fmaxf(fmaxf(__fsub_rn(E.lox, x), __fsub_rn(x, E.hix)), 0.f);
+  const float dy = fmaxf(fmaxf(__fsub_rn(E.loy, y), __fsub_rn(y, E.hiy)), 0.f);
+  return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) > E.lim2;
+}
+#endif
+
+// on-element rule of an element type with NN field nodes: geometry basis and
+// derivative at the 20 samples, sample weights of each field node's integrals
+// for each source node (assemble_near.cu)
+template <int NN>
+struct SingularTable {
+  double N[BEM_NINTERP][BEM_MAXGEO], D[BEM_NINTERP][BEM_MAXGEO];
+  double Wh[NN][BEM_NINTERP][NN], Wg[NN][BEM_NINTERP][NN];
+};
+// the table of R's element type, built once per process
+template <int NN>
+const SingularTable<NN>& singular_table(const Rules& R);
+
 struct FarArgs {
   int nt, n, ne, nn;
   int64_t ld, ldg;

@@ -35,7 +35,8 @@ enum Kind { K_NONE = 0, K_TANGENT = 1, K_REALPOLE = 2, K_GENERAL = 3, K_FAR = 4,
 struct Slot {
   double z0, e0, At, Bt, e0At;
   double A[2], B[2], zt[2], et2[2], mid[2], h[2];  // per half
-  double cx[BEM_MAXGEO], cy[BEM_MAXGEO];           // geometry - source, coefficients of xi^d
+  double cx[BEM_MAXGEO], cy[BEM_MAXGEO];           // geometry - source, coefficients of xi^d (NODAL: the nodes)
+  double sx, sy;                                   // NODAL: the source
   double nrx, nry;                                 // normal of the element's first node
   int kind, np, chart, id;
 };
@@ -250,14 +251,38 @@ __device__ __forceinline__ void basis(const double* x, const double* pw, double 
   }
 }
 
+// Point (relative to the source) and tangent at the parent coordinate of
+// node interpolation weights N by Lagrange sums over absolute coordinates, in
+// the order of shape_geom.
+template <int NN>
+__device__ __forceinline__ void nodal_point(const double* X, const double* Y, const double* N, const double* dN,
+                                            double sx, double sy, double& px, double& py, double& dx, double& dy) {
+  px = N[0] * X[0];
+  py = N[0] * Y[0];
+  dx = dN[0] * X[0];
+  dy = dN[0] * Y[0];
+#pragma unroll
+  for (int k = 1; k < NN; ++k) {
+    px = fma(N[k], X[k], px);
+    py = fma(N[k], Y[k], py);
+    dx = fma(dN[k], X[k], dx);
+    dy = fma(dN[k], Y[k], dy);
+  }
+  px -= sx;
+  py -= sy;
+}
+
 // Sums over the rule of a slot of N_k T J w (h) and N_k U J w (g) by the
 // lanes lg = 0 .. G-1 of a group of G lanes (every lane of the warp calls
 // this with its own group's slot; `on` false: no work).  qs, ws: the Gauss
-// rule in shared memory; lx, lw: element nodes and product-form weights.
-template <int NC, int NN>
+// rule in shared memory.  NODAL: the element's nodes are its geometry and are
+// summed in absolute coordinates (nodal_point), for callers that difference
+// the integrals: the rounding of the coordinates, 2^-53 of their size and not
+// of the element's, then stays the one of the step-by-step rule.
+template <int NC, int NN, bool NODAL = false>
 __device__ __forceinline__ void integrate_group(const Slot& s, bool on, int npg, const double* qs, const double* ws,
-                                                const double* lx, const double* lw, int ng, const Consts& k, int lg,
-                                                int G, double (&h)[NN * NC], double (&g)[NN * NC]) {
+                                                const Rules& R, int ng, const Consts& k, int lg, int G,
+                                                double (&h)[NN * NC], double (&g)[NN * NC]) {
 #pragma unroll
   for (int c = 0; c < NN * NC; ++c) h[c] = g[c] = 0.0;
   const int m = on ? s.np * npg : 0;
@@ -267,9 +292,23 @@ __device__ __forceinline__ void integrate_group(const Slot& s, bool on, int npg,
     const bool act = q < m;
     if (!__any_sync(FULL, act)) break;
     double dx = 0.0, dy = 0.0, px = 0.0, py = 0.0, xi = 0.0, wx = 0.0;
+    double N[NN];
     if (act) {
       const int piece = q >= npg ? 1 : 0;
       rule_node(s, piece, qs[q - piece * npg], ws[q - piece * npg], xi, wx);
+      basis<NN>(R.leg_x, R.leg_pw, xi, N);
+    }
+    if (NODAL && act) {
+      double dN[NN];
+#pragma unroll
+      for (int j = 0; j < NN; ++j) {
+        dN[j] = N[0] * R.leg_D[j];
+#pragma unroll
+        for (int i = 1; i < NN; ++i) dN[j] = fma(N[i], R.leg_D[i * NN + j], dN[j]);
+      }
+      nodal_point<NN>(s.cx, s.cy, N, dN, s.sx, s.sy, px, py, dx, dy);
+    }
+    if (!NODAL && act) {
       // Horner for the point (relative to the source) and the tangent
       px = s.cx[ng - 1];
       py = s.cy[ng - 1];
@@ -286,9 +325,8 @@ __device__ __forceinline__ void integrate_group(const Slot& s, bool on, int npg,
     }
     if (act) {
       const double J = f64::sqrt(fma(dx, dx, dy * dy));
-      double U[4], T[4], N[NN];
+      double U[4], T[4];
       kernel_values<NC>(k, px, py, flip * dy, -(flip * dx), U, T);
-      basis<NN>(lx, lw, xi, N);
       const double wJ = wx * J;
 #pragma unroll
       for (int j = 0; j < NN; ++j) {

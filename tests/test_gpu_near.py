@@ -25,3 +25,33 @@ def test_near_and_own_entries(orc, ne, p, npg, kelvin):
     # the cancellation of the basis values
     assert np.max(np.abs(H - Hr)) <= 1e-12 * np.max(np.abs(Hr))
     assert np.max(np.abs(G - Gr)) <= 1e-12 * np.max(np.abs(Gr))
+
+
+@pytest.mark.parametrize("p, nearfield", [(1, 0), (3, 0), (4, 0), (2, 2)])
+def test_gradient_of_every_element_type(p, nearfield):
+    """dJ/dx of the adjoint call against central differences of its own J, for
+    the element types and the near-field map that take other kernels than the
+    quadratic tanp3c case."""
+    from bem_gmsh_gb300 import Laplace, _lib, from_nodes, star_adjoint_case
+    from bem_gmsh_gb300.api import adjoint_laplace
+    ctx = _lib.default_context()
+    dad, target = star_adjoint_case(12, p=p, seed=4)
+    qt = np.where(dad.BC == 0, 0.1 * target.collocation[:, 0], 0.0)
+    X = np.asarray(dad.collocation).reshape(dad.ne, p + 1, 2)
+
+    def J(Y):
+        return adjoint_laplace(from_nodes("fd", Y, p, Laplace(1.0), dad.BC, dad.BV), qt, npg=16, ctx=ctx)[0]
+
+    ctx.set_option(_lib.BEM_OPT_NEARFIELD, nearfield)
+    try:
+        g = adjoint_laplace(dad, qt, npg=16, ctx=ctx)[1].reshape(-1)
+        h = 1e-6
+        for c in list(np.argsort(-np.abs(g))[:3]) + [1, 2 * p + 2]:
+            Y = X.copy().reshape(-1)
+            Y[c] += h
+            up = J(Y.reshape(X.shape))
+            Y[c] -= 2 * h
+            # J to 1e-12 of itself over 2 h, and the differences' own h^2 terms
+            assert abs((up - J(Y.reshape(X.shape))) / (2 * h) - g[c]) <= 1e-5 * np.max(np.abs(g))
+    finally:
+        ctx.set_option(_lib.BEM_OPT_NEARFIELD, 0)
