@@ -55,3 +55,21 @@ def test_gradient_of_every_element_type(p, nearfield):
             assert abs((up - J(Y.reshape(X.shape))) / (2 * h) - g[c]) <= 1e-5 * np.max(np.abs(g))
     finally:
         ctx.set_option(_lib.BEM_OPT_NEARFIELD, 0)
+
+
+@pytest.mark.parametrize("ne, p, npg", [(24, 3, 8), (30, 2, 5), (60, 2, 8), (90, 1, 10), (300, 2, 16), (40, 2, 32)])
+def test_interior_far_rule(orc, ne, p, npg):
+    """Interior points from the middle to a thousandth of the radius from the
+    boundary, and on it: far pairs by the Gauss rule, the others by the map;
+    more elements than a round of the kernel takes, and fewer than a warp."""
+    from bem_gmsh_gb300.api import interior_laplace
+    dad = star_domain(ne, p=p, seed=ne)
+    ana = dad.cache["analytical"]
+    T, q = ana.u(dad.Nodes), ana.q(dad.Nodes, dad.normal)
+    pts = np.concatenate([[[0.0, 0.0]], 0.5 * dad.Nodes[::5], 0.9 * dad.Nodes[::7], 0.999 * dad.Nodes[::11],
+                          dad.Nodes[::29]])
+    got = interior_laplace(dad, pts, npg=npg, T=T, q=q)
+    ref = orc.interior_laplace(dad, pts, npg=npg, T=T, q=q)
+    # both rules within 3e-11 of a far integral (8 points and more; fewer
+    # points take the map everywhere)
+    assert np.max(np.abs(got - ref)) <= 1e-10 * np.max(np.abs(ref))
