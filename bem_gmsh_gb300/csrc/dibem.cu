@@ -17,6 +17,7 @@
 
 #include "bem_abi_internal.h"
 #include "bem_device.cuh"
+#include "fast64.cuh"
 
 namespace bem {
 namespace {
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(128) dibem_kelvin_kernel(int nt, const double*
   }
 }
 
-// radial integral of each RBF kind (`_dibem_phi_int2d`, DIBEM_GPU.jl:141-171)
+
 template <typename T>
 __device__ __forceinline__ T dibem_phi_int(int kind, T R, T kcond, T epsa) {
   const T R2 = R * R;
@@ -170,6 +171,63 @@ __device__ __forceinline__ T dibem_phi_int(int kind, T R, T kcond, T epsa) {
   }
 }
 
+// phi_int(R) / R^2 in FP64, up to the factor phi_int_scale: the powers of R
+// cancel before they are formed, so a pair needs no quotient (an FP64 quotient
+// is five and a half multiply-adds of GB300's small FP64 pipe)
+__device__ __forceinline__ double phi_int_over_r2(int kind, double R2, double lgR2, double epsa) {
+  if (kind == 10) return 1.0 - lgR2;
+  const double R = f64::sqrt(R2);
+  switch (kind) {
+    case 1: return R;
+    case 2: return R2 * (4.0 * f64::log(R + epsa) - 1.0);
+    case 3: return R2 * R;
+    case 4: return (R2 * R2) * (6.0 * f64::log(R + epsa) - 1.0);
+    case 5: return (R2 * R2) * R;
+    case 6: return (R2 * R2 * R2) * (8.0 * f64::log(R + epsa) - 1.0);
+    default: return (R2 * R2 * R2) * R;
+  }
+}
+__device__ __forceinline__ double phi_int_scale(int kind, double kcond) {
+  switch (kind) {
+    case 1: return 1.0 / 3.0;
+    case 2: return 1.0 / 16.0;
+    case 3: return 1.0 / 5.0;
+    case 4: return 1.0 / 36.0;
+    case 5: return 1.0 / 7.0;
+    case 6: return 1.0 / 64.0;
+    case 7: return 1.0 / 9.0;
+    default: return 1.0 / (8.0 * kPi * kcond);
+  }
+}
+
+// An element's box in FP32, rounded outwards, and its near limit widened by
+// more than the rounding of coordinates and distances: a point that the FP32
+// test calls far is far for the exact FP64 test too.  (The FP64 box test took
+// a third of the far kernel, the exact test for every pair half of the near
+// kernel.)
+struct Box32 {
+  float lox, loy, hix, hiy, lim;
+};
+__device__ __forceinline__ Box32 box32(const double* x, const double* y, int nn, double L, double nf) {
+  double lx = INFINITY, ly = INFINITY, hx = -INFINITY, hy = -INFINITY;
+  for (int q = 0; q < nn; ++q) {
+    lx = fmin(lx, x[q]);
+    ly = fmin(ly, y[q]);
+    hx = fmax(hx, x[q]);
+    hy = fmax(hy, y[q]);
+  }
+  Box32 b{__double2float_rd(lx), __double2float_rd(ly), __double2float_ru(hx), __double2float_ru(hy), 0.f};
+  const float m = fmaxf(fmaxf(fabsf(b.lox), fabsf(b.hix)), fmaxf(fabsf(b.loy), fabsf(b.hiy)));
+  b.lim = nf > 1e20 ? INFINITY : __double2float_ru(nf * L * (1.0 + 1e-5)) + 1e-6f * m;
+  return b;
+}
+// (px, py): the point rounded to FP32, pm = 1e-6 times its largest coordinate
+__device__ __forceinline__ bool surely_far(const Box32& b, float px, float py, float pm) {
+  const float dx = fmaxf(fmaxf(b.lox - px, px - b.hix), 0.f), dy = fmaxf(fmaxf(b.loy - py, py - b.hiy), 0.f);
+  const float lim = b.lim + pm;
+  return dx * dx + dy * dy > lim * lim;
+}
+
 // Far boundary sums IF, ID of the DIBEM domain integrals (restating
 // `_dibem_IFID_kernel!`, DIBEM_GPU.jl:234-270): for every collocation point
 // i and boundary node j with R > 1e-10, unless the pair (i, element of j) is
@@ -177,10 +235,11 @@ __device__ __forceinline__ T dibem_phi_int(int kind, T R, T kcond, T epsa) {
 // as the assembly),
 //   IF_i += phi_int(R) w_j (r . n_j) / R^2,  ID_i += rad(R) w_j (r . n_j) / R^2,
 // rad(R) = -(2 R^2 log R - R^2) / (8 pi k) (`_dibem_rad_id2d`, :173-177),
-// w_j = Jacobian_j * elem_weight_k.  Grid: x over 128-point row blocks, y
-// over 32-element chunks staged in shared memory; partial sums are added
-// atomically.  A conservative FP64 box test skips the exact near test for
-// pairs that are far by a margin.
+// w_j = Jacobian_j * elem_weight_k.  With rad(R) / R^2 = (1 - log R^2) / (8 pi k)
+// and phi_int(R) / R^2 by phi_int_over_r2 a pair is 27 FP64 operations for an
+// odd spline (it was 90; 4098 x 4098 pairs 2.48 -> 0.84 ms, FP64 issue bound).
+// Grid: x over 128-point row blocks, y over 32-element chunks staged in
+// shared memory; partial sums are added atomically.
 constexpr int IF_EC = 32;
 struct IfidRule {
   double ew[BEM_MAXNN];
@@ -191,7 +250,8 @@ __global__ void __launch_bounds__(128) dibem_ifid_kernel(GeomDev g, IfidRule rw,
                                                         double nf, T* __restrict__ IF, T* __restrict__ ID) {
   __shared__ double sx[IF_EC * BEM_MAXNN], sy[IF_EC * BEM_MAXNN];
   __shared__ T snx[IF_EC * BEM_MAXNN], sny[IF_EC * BEM_MAXNN], sw[IF_EC * BEM_MAXNN];
-  __shared__ double blo[IF_EC][2], bhi[IF_EC][2], blim2[IF_EC], belen[IF_EC];
+  __shared__ Box32 sbox[IF_EC];
+  __shared__ double belen[IF_EC];
   const int nn = g.nn;
   const int e0 = blockIdx.y * IF_EC;
   const int nel = min(IF_EC, g.ne - e0);
@@ -199,40 +259,27 @@ __global__ void __launch_bounds__(128) dibem_ifid_kernel(GeomDev g, IfidRule rw,
     const int j = e0 * nn + idx;
     sx[idx] = g.px[j];
     sy[idx] = g.py[j];
-    snx[idx] = (T)g.nx[j];
-    sny[idx] = (T)g.ny[j];
     sw[idx] = (T)(g.jac[j] * rw.ew[idx % nn]);
+    snx[idx] = (T)g.nx[j] * (sizeof(T) == 8 ? sw[idx] : T(1));  // FP64: times the weight
+    sny[idx] = (T)g.ny[j] * (sizeof(T) == 8 ? sw[idx] : T(1));
   }
+  __syncthreads();
   for (int el = threadIdx.x; el < nel; el += blockDim.x) {
-    double lx = INFINITY, ly = INFINITY, hx = -INFINITY, hy = -INFINITY;
-    for (int q = 0; q < nn; ++q) {
-      const int j = (e0 + el) * nn + q;
-      lx = fmin(lx, g.px[j]);
-      ly = fmin(ly, g.py[j]);
-      hx = fmax(hx, g.px[j]);
-      hy = fmax(hy, g.py[j]);
-    }
-    blo[el][0] = lx; blo[el][1] = ly;
-    bhi[el][0] = hx; bhi[el][1] = hy;
-    const double L = g.elen[e0 + el];
-    belen[el] = L;
-    const double lim = nf * L;
-    blim2[el] = nf > 1e20 ? INFINITY : lim * lim * (1.0 + 1e-12);
+    belen[el] = g.elen[e0 + el];
+    sbox[el] = box32(sx + el * nn, sy + el * nn, nn, belen[el], nf);
   }
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= g.nt) return;
   const V2 pf{g.px[i], g.py[i]};
   const T pxi = (T)pf.x, pyi = (T)pf.y;
+  const float fx = (float)pf.x, fy = (float)pf.y, fm = 1e-6f * fmaxf(fabsf(fx), fabsf(fy));
   T aF = T(0), aD = T(0);
-  const T rmin = T(1e-10);
   const T radc = T(1) / (T(8) * T(3.14159265358979323846) * kcond);
   for (int el = 0; el < nel; ++el) {
     const int e = e0 + el;
     if (i >= e * nn && i < (e + 1) * nn) continue;  // source on the element
-    const double dx = fmax(fmax(blo[el][0] - pf.x, pf.x - bhi[el][0]), 0.0);
-    const double dy = fmax(fmax(blo[el][1] - pf.y, pf.y - bhi[el][1]), 0.0);
-    if (!(dx * dx + dy * dy > blim2[el])) {
+    if (!surely_far(sbox[el], fx, fy, fm)) {
       V2 xg[BEM_MAXNN];
       for (int q = 0; q < nn; ++q) xg[q] = V2{sx[el * nn + q], sy[el * nn + q]};
       if (near_element(pf, xg, nn, belen[el], nf)) continue;
@@ -241,13 +288,26 @@ __global__ void __launch_bounds__(128) dibem_ifid_kernel(GeomDev g, IfidRule rw,
       const int s = el * nn + q;
       const T rx = (T)sx[s] - pxi, ry = (T)sy[s] - pyi;
       const T R2 = rx * rx + ry * ry;
-      const T R = sqrt(R2);
-      if (R > rmin) {
-        const T wJn = sw[s] * (rx * snx[s] + ry * sny[s]) / R2;
-        aF += dibem_phi_int<T>(rbf, R, kcond, epsa) * wJn;
-        aD += -(T(2) * R2 * log(R) - R2) * radc * wJn;
+      if constexpr (sizeof(T) == 4) {
+        // FP32: the products in the reference's order (quotients are cheap
+        // here, and the sums keep their rounding)
+        const T R = sqrt(R2);
+        if (R > T(1e-10)) {
+          const T wJn = sw[s] * (rx * snx[s] + ry * sny[s]) / R2;
+          aF += dibem_phi_int<T>(rbf, R, kcond, epsa) * wJn;
+          aD += -(T(2) * R2 * log(R) - R2) * radc * wJn;
+        }
+      } else if (R2 > T(1e-20)) {
+        const T rn = rx * snx[s] + ry * sny[s];
+        const T lg = f64::log(R2);
+        aF += phi_int_over_r2(rbf, R2, lg, epsa) * rn;
+        aD += (T(1) - lg) * rn;
       }
     }
+  }
+  if constexpr (sizeof(T) == 8) {
+    aF *= phi_int_scale(rbf, kcond);
+    aD *= radc;
   }
   atomicAdd(IF + i, aF);
   atomicAdd(ID + i, aD);
@@ -260,27 +320,57 @@ __global__ void __launch_bounds__(128) dibem_ifid_kernel(GeomDev g, IfidRule rw,
 // src/Core/DIBEM_common.jl:112-171: rule points y_q, normals tan2normal of
 // the tangent aligned with the element's first nodal normal, w_q J_q),
 //   IF_i += phi_int(R) w_q J_q (r . n_q) / R^2,  ID_i += rad(R) w_q J_q (r . n_q) / R^2
-// with r = y_q - x_i, points closer than 1e-14 skipped.  FP64.  The block's
-// 16 elements and their rule points are built once in shared memory; each
-// thread takes one point.
-constexpr int NR_EC = 16;
-__global__ void __launch_bounds__(128) dibem_near_kernel(GeomDev g, Rules R, int rbf, double kcond, double epsa,
-                                                         double nf, double* __restrict__ IF,
-                                                         double* __restrict__ ID) {
+// with r = y_q - x_i, points closer than 1e-14 skipped.  FP64.  A CTA takes
+// 128 points and 16 elements: its pairs are found first (nearly all CTAs have
+// none and leave), then the elements' rule points are built in shared memory
+// and 16 lanes take a pair's rule (a thread per point went through its
+// elements alone: 13 of a warp's 32 lanes had work at best; 1.39 ms at 4098
+// nodes, now 0.06).
+constexpr int NR_EC = 16, NR_PT = 128;
+__global__ void __launch_bounds__(NR_PT) dibem_near_kernel(const __grid_constant__ GeomDev g,
+                                                          const __grid_constant__ Rules R, int rbf, double kcond,
+                                                          double epsa, double nf, double* __restrict__ IF,
+                                                          double* __restrict__ ID) {
   __shared__ double sx[NR_EC * BEM_MAXNN], sy[NR_EC * BEM_MAXNN];
-  __shared__ double qy[NR_EC * BEM_MAXNPG][5];  // y.x, y.y, n.x, n.y, w J
+  __shared__ double qy[NR_EC * BEM_MAXNPG][4];  // y.x, y.y, n.x w J, n.y w J
+  __shared__ Box32 sbox[NR_EC];
   __shared__ double belen[NR_EC];
-  const int nn = g.nn, npg = R.npg;
+  __shared__ unsigned short s_pair[NR_PT * NR_EC];  // point * 16 + element
+  __shared__ int s_count;
+  const int nn = g.nn, npg = R.npg, t = threadIdx.x;
   const int e0 = blockIdx.y * NR_EC;
   const int nel = min(NR_EC, g.ne - e0);
-  for (int idx = threadIdx.x; idx < nel * nn; idx += blockDim.x) {
+  for (int idx = t; idx < nel * nn; idx += NR_PT) {
     sx[idx] = g.px[e0 * nn + idx];
     sy[idx] = g.py[e0 * nn + idx];
   }
-  for (int el = threadIdx.x; el < nel; el += blockDim.x) belen[el] = g.elen[e0 + el];
+  if (t == 0) s_count = 0;
   __syncthreads();
-  for (int t = threadIdx.x; t < nel * npg; t += blockDim.x) {
-    const int el = t / npg, q = t - el * npg;
+  if (t < nel) {
+    belen[t] = g.elen[e0 + t];
+    sbox[t] = box32(sx + t * nn, sy + t * nn, nn, belen[t], nf);
+  }
+  __syncthreads();
+  const int i = blockIdx.x * NR_PT + t;
+  if (i < g.nt) {
+    const V2 pf{g.px[i], g.py[i]};
+    const float fx = (float)pf.x, fy = (float)pf.y, fm = 1e-6f * fmaxf(fabsf(fx), fabsf(fy));
+    for (int el = 0; el < nel; ++el) {
+      const int e = e0 + el;
+      bool near = i >= e * nn && i < (e + 1) * nn;
+      if (!near && !surely_far(sbox[el], fx, fy, fm)) {
+        V2 xg[BEM_MAXNN];
+        for (int k = 0; k < nn; ++k) xg[k] = V2{sx[el * nn + k], sy[el * nn + k]};
+        near = near_element(pf, xg, nn, belen[el], nf);
+      }
+      if (near) s_pair[atomicAdd(&s_count, 1)] = (unsigned short)(t * NR_EC + el);
+    }
+  }
+  __syncthreads();
+  const int count = s_count;
+  if (count == 0) return;
+  for (int v = t; v < nel * npg; v += NR_PT) {
+    const int el = v / npg, q = v - el * npg;
     double L[BEM_MAXNN], dL[BEM_MAXNN];
     shapefun(R.leg_x, R.leg_bw, R.leg_D, nn, R.qsi[q], L, dL);
     double px = 0, py = 0, dx = 0, dy = 0;
@@ -290,46 +380,44 @@ __global__ void __launch_bounds__(128) dibem_near_kernel(GeomDev g, Rules R, int
       dx += dL[k] * sx[el * nn + k];
       dy += dL[k] * sy[el * nn + k];
     }
-    const double J = sqrt(dx * dx + dy * dy);
     const int j0 = (e0 + el) * nn;
-    const double rx = g.nx[j0], ry = g.ny[j0];
-    double ux = rx, uy = ry;
-    if (!(J < 1e-16)) { ux = dy / J; uy = -dx / J; }
-    if (ux * rx + uy * ry < 0) { ux = -ux; uy = -uy; }
-    qy[t][0] = px;
-    qy[t][1] = py;
-    qy[t][2] = ux;
-    qy[t][3] = uy;
-    qy[t][4] = J < 1e-16 ? 0.0 : R.w[q] * J;
+    const bool bad = sqrt(dx * dx + dy * dy) < 1e-16;
+    const double flip = dy * g.nx[j0] - dx * g.ny[j0] < 0 ? -R.w[q] : R.w[q];
+    qy[v][0] = px;
+    qy[v][1] = py;
+    qy[v][2] = bad ? 0.0 : flip * dy;
+    qy[v][3] = bad ? 0.0 : -(flip * dx);
   }
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.nt) return;
-  const V2 pf{g.px[i], g.py[i]};
-  const double radc = 1.0 / (8.0 * kPi * kcond);
-  double aF = 0.0, aD = 0.0;
-  for (int el = 0; el < nel; ++el) {
-    const int e = e0 + el;
-    const bool on = i >= e * nn && i < (e + 1) * nn;
-    if (!on) {
-      V2 xg[BEM_MAXNN];
-      for (int k = 0; k < nn; ++k) xg[k] = V2{sx[el * nn + k], sy[el * nn + k]};
-      if (!near_element(pf, xg, nn, belen[el], nf)) continue;
+  const double cF = phi_int_scale(rbf, kcond), cD = 1.0 / (8.0 * kPi * kcond);
+  const int lg = t & 15;
+  for (int p0 = 0; p0 < count; p0 += NR_PT / 16) {
+    const int p = p0 + (t >> 4);
+    double aF = 0.0, aD = 0.0;
+    int ip = 0;
+    if (p < count) {
+      const int pr = s_pair[p], el = pr & (NR_EC - 1);
+      ip = blockIdx.x * NR_PT + pr / NR_EC;
+      const double x = g.px[ip], y = g.py[ip];
+      for (int q = lg; q < npg; q += 16) {
+        const double* Y = qy[el * npg + q];
+        const double rx = Y[0] - x, ry = Y[1] - y;
+        const double R2 = rx * rx + ry * ry;
+        if (R2 < 1e-28) continue;
+        const double rn = rx * Y[2] + ry * Y[3], l = f64::log(R2);
+        aF += phi_int_over_r2(rbf, R2, l, epsa) * rn;
+        aD += (1.0 - l) * rn;
+      }
     }
-    for (int q = 0; q < npg; ++q) {
-      const double* Y = qy[el * npg + q];
-      if (Y[4] == 0.0) continue;
-      const double rx = Y[0] - pf.x, ry = Y[1] - pf.y;
-      const double R2 = rx * rx + ry * ry;
-      const double Rr = sqrt(R2);
-      if (Rr < 1e-14) continue;
-      const double wJn = Y[4] * ((Y[2] * rx + Y[3] * ry) / R2);
-      aF += dibem_phi_int<double>(rbf, Rr, kcond, epsa) * wJn;
-      aD += -(2.0 * R2 * log(Rr) - R2) * radc * wJn;
+    for (int o = 8; o > 0; o >>= 1) {
+      aF += __shfl_xor_sync(0xffffffffu, aF, o);
+      aD += __shfl_xor_sync(0xffffffffu, aD, o);
+    }
+    if (p < count && lg == 0) {
+      atomicAdd(IF + ip, aF * cF);
+      atomicAdd(ID + ip, aD * cD);
     }
   }
-  if (aF != 0.0) atomicAdd(IF + i, aF);
-  if (aD != 0.0) atomicAdd(ID + i, aD);
 }
 
 }  // namespace
