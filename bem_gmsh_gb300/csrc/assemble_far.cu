@@ -27,6 +27,7 @@
 #include "bem_kernels.h"
 #include "bem_prof.h"
 #include "df32.cuh"
+#include "near_coop.cuh"
 
 namespace bem {
 
@@ -68,6 +69,15 @@ __global__ void pack_nodes_kernel(GeomDev g, Rules R, Physics ph, NodeRec* nodes
     r.cH = (float)wjk;
   }
   nodes[j] = r;
+}
+
+// FP64 node record
+__global__ void pack_nodes_d_kernel(GeomDev g, Rules R, Physics ph, NodeD* nodes) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= g.n) return;
+  const double w = g.jac[j] * R.ew[j % g.nn];
+  const coop::Consts k = ph.kind == 0 ? coop::make_consts<1>(ph) : coop::Consts{1.0, 0.0, 1.0, 0.0};
+  nodes[j] = NodeD{g.nx[j] * (k.cT * w), g.ny[j] * (k.cT * w), k.cU * w, 0.0};
 }
 
 // double-float log table (one thread per entry)
@@ -325,6 +335,9 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
   __shared__ __align__(16) ElemRec s_el[BE];
   __shared__ __align__(16) unsigned char s_ndraw[BE * BEM_MAXNN * NDB];
   __shared__ __align__(16) float4 s_log[PREC == 3 ? df::kLogTable : 1];
+  // FP64: node coordinates beside the records
+  __shared__ double s_x[PREC == 1 || PREC == 2 ? BE * BEM_MAXNN : 1], s_y[PREC == 1 || PREC == 2 ? BE * BEM_MAXNN : 1];
+  const NodeD* s_ndd = (const NodeD*)s_ndraw;
   __shared__ __align__(8) uint64_t s_bar;
   const NodeRec* s_nd = (const NodeRec*)s_ndraw;
   const NodeDF* s_ndf = (const NodeDF*)s_ndraw;
@@ -346,6 +359,12 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
   }
   if constexpr (PREC == 3) {
     for (int i = tid; i < df::kLogTable; i += blockDim.x) s_log[i] = a.logtab[i];
+  }
+  if constexpr (PREC == 1 || PREC == 2) {
+    for (int i = tid; i < ne_t * nn; i += blockDim.x) {
+      s_x[i] = a.px[e0 * nn + i];
+      s_y[i] = a.py[e0 * nn + i];
+    }
   }
   __syncthreads();
   if (tid == 0) {
@@ -413,6 +432,7 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
     for (int r = 0; r < SPT * DOF * DOF; ++r) rs32[r] = df::f2{0.f, 0.f};
   }
 
+  const coop::Consts kc = coop::make_consts<NC>(a.ph);
   const size_t ld = (size_t)a.ld;
   const size_t ldg = (size_t)a.ldg;
   const bool vec_ok = a.vec_ok && (src0 + SPT <= a.nt);
@@ -528,12 +548,12 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
       continue;
     }
     for (int k = 0; k < nn; ++k) {
-      const NodeRec nd = s_nd[el * nn + k];
       const int j = e * nn + k;
       OutT hv[DOF][SPT * DOF], gv[DOF][SPT * DOF];  // [column dof b][row]
 #pragma unroll
       for (int s = 0; s < SPT; ++s) {
         if constexpr (PREC == 0) {
+          const NodeRec nd = s_nd[el * nn + k];
           float rx = (nd.xh - sxh[s]) + (nd.xl - sxl[s]);
           float ry = (nd.yh - syh[s]) + (nd.yl - syl[s]);
           float U[NC], Tk[NC];
@@ -546,10 +566,23 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
               gv[b][s * DOF + ar] = far[s] ? U[ar * DOF + b] : 0.f;
             }
         } else {
+          // 22 FP64 operations for a Laplace pair (fast64.cuh, constants
+          // folded into the record; it was 59: the compiler's logarithm and
+          // quotient), 46 for a Kelvin one.  FP64 issue bounds the kernel:
+          // 4100 x 4100 entries of H and G 1.62 -> 0.72 ms.
           double U[NC], Tk[NC];
           if (far[s]) {
-            far_eval_f64<NC>(a.ph, a.px[j] - sx[s], a.py[j] - sy[s], a.nx[j], a.ny[j],
-                             a.jac[j] * a.ew[k], U, Tk);
+            const NodeD& nd = s_ndd[el * nn + k];
+            const double rx = s_x[el * nn + k] - sx[s], ry = s_y[el * nn + k] - sy[s];
+            if constexpr (NC == 1) {
+              const double R2 = fma(rx, rx, ry * ry);
+              U[0] = nd.c * f64::log(R2);
+              Tk[0] = f64::div(fma(rx, nd.nx, ry * nd.ny), R2);
+            } else {
+              coop::kernel_values<NC>(kc, rx, ry, nd.nx, nd.ny, U, Tk);
+#pragma unroll
+              for (int c = 0; c < NC; ++c) U[c] *= nd.c;
+            }
           } else {
 #pragma unroll
             for (int c = 0; c < NC; ++c) U[c] = Tk[c] = 0.0;
@@ -767,7 +800,7 @@ static void launch_variant(const AsmRequest& q, cudaStream_t st) {
     if (side2) cudaStreamWaitEvent(st, q.ev_join2, 0);
     launch_finalize(fi, NC, g.nt, st);
   }
-  count_launches(g.n > 0 ? 9 : 8);
+  count_launches(PREC == 3 ? 8 : 9);
 }
 
 int launch_assembly(const AsmRequest& q, cudaStream_t st) {
@@ -786,7 +819,10 @@ int launch_assembly(const AsmRequest& q, cudaStream_t st) {
     if (q.prec == 2) cudaMemsetAsync(q.A32 + off, 0, cnt * 4, st);
   }
   pack_rows_kernel<<<(g.nt + 255) / 256, 256, 0, st>>>(g, q.rows);
-  pack_nodes_kernel<<<(g.n + 255) / 256, 256, 0, st>>>(g, q.R, q.ph, q.nodes);
+  if (q.prec == 0)
+    pack_nodes_kernel<<<(g.n + 255) / 256, 256, 0, st>>>(g, q.R, q.ph, q.nodes);
+  else if (q.prec != 3)
+    pack_nodes_d_kernel<<<(g.n + 255) / 256, 256, 0, st>>>(g, q.R, q.ph, (NodeD*)q.nodes);
   cudaMemsetAsync(q.absmax, 0, sizeof(unsigned long long), st);
   absmax_kernel<<<64, 256, 0, st>>>(g, q.absmax);
   pack_elems_kernel<<<(g.ne + 255) / 256, 256, 0, st>>>(g, q.near_factor, q.absmax, q.elems);

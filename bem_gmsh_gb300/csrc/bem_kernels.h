@@ -14,6 +14,12 @@ struct __align__(16) NodeRec {
   float cG, cH;          // folded kernel constants times J w
 };
 
+// 32-byte node record of the FP64 far field, in the place of a NodeRec.
+// Laplace: {n cT w, cU w, -}; Kelvin: {n w, w, -} (constants of coop::Consts).
+struct __align__(16) NodeD {
+  double nx, ny, c, pad;
+};
+
 // 64-byte node record of the double-float far field (Laplace): coordinates
 // as exact three-float splits, normal, kernel constants and boundary value
 // as hi + lo pairs (G = log(R2) cG, H = (r.n) / R2 cH).
