@@ -573,10 +573,14 @@ extern "C" int bem_adjoint_laplace2d(bem_ctx* c, const bem_geom2d* g, double k, 
     cudaMemcpyAsync(qt, q_target, sizeof(double) * N, cudaMemcpyDeviceToDevice, c->stream);
   }
   const int prec = (c->opt_far_df >= 1) ? 3 : 1;
-  rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b);
-  if (rc) return rc;
   bem_solve_stats st{};
-  rc = bem_solve_mixed_dev(c, N, A, ld, b, tol, max_iter, 1, u, &st);
+  for (int attempt = 0;; ++attempt) {
+    // (the solve checks the assembly's pair count; too short a list: again)
+    rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b, attempt == 0);
+    if (rc) return rc;
+    rc = bem_solve_mixed_dev(c, N, A, ld, b, tol, max_iter, 1, u, &st);
+    if (rc != BEM_RETRY) break;
+  }
   if (rc != BEM_OK && rc != BEM_ERR_NOT_CONVERGED) return rc;
   adj_split_kernel<<<1, 256, 0, c->stream>>>(n, dBC, dBV, u, qt, T, q, dJdu, Jd);
   // adjoint system A^T lambda = dJ/du

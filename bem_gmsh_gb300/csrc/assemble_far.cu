@@ -40,9 +40,7 @@ __device__ __forceinline__ void split_f(double v, float& hi, float& lo) {
 }
 
 // row record: x_hi, x_lo, y_hi, y_lo
-__global__ void pack_rows_kernel(GeomDev g, float4* rows) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.nt) return;
+__device__ __forceinline__ void pack_row(const GeomDev& g, int i, float4* rows) {
   float4 r;
   split_f(g.px[i], r.x, r.y);
   split_f(g.py[i], r.z, r.w);
@@ -52,9 +50,8 @@ __global__ void pack_rows_kernel(GeomDev g, float4* rows) {
 // node record (32 B): x_hi, x_lo, y_hi, y_lo, nx, ny, cG, cH
 // Laplace: G = log2(R2) * cG, H = (r.n) / R2 * cH
 // Kelvin : cG = cH = J w (the weight only)
-__global__ void pack_nodes_kernel(GeomDev g, Rules R, Physics ph, NodeRec* nodes) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.n) return;
+__device__ __forceinline__ void pack_node(const GeomDev& g, const Rules& R, const Physics& ph, int j,
+                                          NodeRec* nodes) {
   NodeRec r;
   split_f(g.px[j], r.xh, r.xl);
   split_f(g.py[j], r.yh, r.yl);
@@ -72,28 +69,17 @@ __global__ void pack_nodes_kernel(GeomDev g, Rules R, Physics ph, NodeRec* nodes
 }
 
 // FP64 node record
-__global__ void pack_nodes_d_kernel(GeomDev g, Rules R, Physics ph, NodeD* nodes) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.n) return;
+__device__ __forceinline__ void pack_node_d(const GeomDev& g, const Rules& R, const Physics& ph, int j,
+                                            NodeD* nodes) {
   const double w = g.jac[j] * R.ew[j % g.nn];
   const coop::Consts k = ph.kind == 0 ? coop::make_consts<1>(ph) : coop::Consts{1.0, 0.0, 1.0, 0.0};
   nodes[j] = NodeD{g.nx[j] * (k.cT * w), g.ny[j] * (k.cT * w), k.cU * w, 0.0};
 }
 
-// double-float log table (one thread per entry)
-__global__ void logtab_kernel(float4* t) {
-  const int i = threadIdx.x;
-  if (i < df::kLogTable) {
-    const df::LogEntry e = df::log_entry(i);
-    t[i] = make_float4(e.rc_h, e.rc_l, e.lc_h, e.lc_l);
-  }
-}
-
 // double-float node record (Laplace): G = log(R2) cG, H = (r.n) / R2 cH with
 // the constants of laplace_UT times J w, and the boundary value of the node
-__global__ void pack_nodes_df_kernel(GeomDev g, Rules R, Physics ph, const double* bv, NodeDF* nodes) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.n) return;
+__device__ __forceinline__ void pack_node_df(const GeomDev& g, const Rules& R, const Physics& ph, const double* bv,
+                                             int j, NodeDF* nodes) {
   NodeDF r;
   df::split3(g.px[j], r.xa, r.xb, r.xc);
   df::split3(g.py[j], r.ya, r.yb, r.yc);
@@ -116,9 +102,8 @@ __global__ void pack_nodes_df_kernel(GeomDev g, Rules R, Physics ph, const doubl
 // cU = J w / (2 prod1 mu), cUl = -(3 - 4 nu) / 2 cU (the log(1/R) term as
 // log(R2)), cT = -J w / prod1 with prod1 = 4 pi (1 - nu), and the node's two
 // boundary values
-__global__ void pack_nodes_dfk_kernel(GeomDev g, Rules R, Physics ph, const double* bv, NodeDFK* nodes) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.n) return;
+__device__ __forceinline__ void pack_node_dfk(const GeomDev& g, const Rules& R, const Physics& ph, const double* bv,
+                                              int j, NodeDFK* nodes) {
   NodeDFK r;
   df::split3(g.px[j], r.xa, r.xb, r.xc);
   df::split3(g.py[j], r.ya, r.yb, r.yc);
@@ -144,26 +129,11 @@ __global__ void pack_nodes_dfk_kernel(GeomDev g, Rules R, Physics ph, const doub
 
 // element record (32 B): conservative box of the element's nodes and the
 // squared near limit, widened so that a pair the box test calls far is far
-// for the exact FP64 test as well.
-// largest |coordinate| of the collocation points (non-negative doubles
-// order like their bit patterns)
-__global__ void absmax_kernel(GeomDev g, unsigned long long* out) {
-  unsigned long long m = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.nt; i += gridDim.x * blockDim.x) {
-    double v = fmax(fabs(g.px[i]), fabs(g.py[i]));
-    m = max(m, (unsigned long long)__double_as_longlong(v));
-  }
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
-// The margin covers the FP32 rounding of coordinates, box and distance
-// (a few 2^-24 relative to the coordinate scale) with room to spare.
-__global__ void pack_elems_kernel(GeomDev g, double near_factor, const unsigned long long* absmax,
-                                  ElemRec* el) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= g.ne) return;
-  const double abs_margin = 1e-6 * __longlong_as_double((long long)*absmax);
+// for the exact FP64 test as well.  The margin covers the FP32 rounding of
+// coordinates, box and distance (a few 2^-24 relative to the coordinates,
+// which for a near pair are at most the element's and the limit) with room to
+// spare.
+__device__ __forceinline__ void pack_elem(const GeomDev& g, double near_factor, int e, ElemRec* el) {
   double lox = INFINITY, loy = INFINITY, hix = -INFINITY, hiy = -INFINITY;
   for (int k = 0; k < g.nn; ++k) {
     double x = g.px[e * g.nn + k], y = g.py[e * g.nn + k];
@@ -173,7 +143,8 @@ __global__ void pack_elems_kernel(GeomDev g, double near_factor, const unsigned 
     hiy = fmax(hiy, y);
   }
   double lim = near_factor * g.elen[e];
-  double limw = lim * (1.0 + 1e-5) + abs_margin;
+  double reach = fmax(fmax(fabs(lox), fabs(hix)), fmax(fabs(loy), fabs(hiy))) + lim;
+  double limw = lim * (1.0 + 1e-5) + 1e-6 * reach;
   ElemRec r;
   r.lox = __double2float_rd(lox);
   r.loy = __double2float_rd(loy);
@@ -184,19 +155,62 @@ __global__ void pack_elems_kernel(GeomDev g, double near_factor, const unsigned 
   el[e] = r;
 }
 
+// Everything an assembly sets up, in one launch (it was six kernels and four
+// memsets: 25 us of launches before the first pair): row, node and element
+// records, the double-float log table (one entry per thread of the last
+// block), zeroed row sums, right-hand side and counters.
+struct PackArgs {
+  GeomDev g;
+  Rules R;
+  Physics ph;
+  double near_factor;
+  int prec, dof;
+  const double* bv;
+  float4* rows;
+  void* nodes;
+  ElemRec* elems;
+  float4* logtab;
+  double *rowsum, *b;
+  int* counters;
+};
+__global__ void __launch_bounds__(256) pack_kernel(const __grid_constant__ PackArgs a) {
+  const GeomDev& g = a.g;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 2) a.counters[i] = 0;
+  if (i < g.nt) {
+    pack_row(g, i, a.rows);
+    for (int c = 0; c < a.dof * a.dof; ++c) a.rowsum[(size_t)i * a.dof * a.dof + c] = 0.0;
+    if (a.b)
+      for (int c = 0; c < a.dof; ++c) a.b[(size_t)i * a.dof + c] = 0.0;
+  }
+  if (i < g.n) {
+    if (a.prec == 0) pack_node(g, a.R, a.ph, i, (NodeRec*)a.nodes);
+    else if (a.prec != 3) pack_node_d(g, a.R, a.ph, i, (NodeD*)a.nodes);
+    else if (a.dof == 1) pack_node_df(g, a.R, a.ph, a.bv, i, (NodeDF*)a.nodes);
+    else pack_node_dfk(g, a.R, a.ph, a.bv, i, (NodeDFK*)a.nodes);
+  }
+  if (i < g.ne) pack_elem(g, a.near_factor, i, a.elems);
+  if (a.prec == 3 && blockIdx.x == gridDim.x - 1 && threadIdx.x < df::kLogTable) {
+    const df::LogEntry e = df::log_entry(threadIdx.x);
+    a.logtab[threadIdx.x] = make_float4(e.rc_h, e.rc_l, e.lc_h, e.lc_l);
+  }
+}
+
 // Possibly-near (point, element) pairs into the pair list: one thread per
-// point, the CTA's 256 elements staged in shared memory.  Each warp first
+// point, the CTA's 64 elements staged in shared memory (256 of them made a
+// chain of 20 us on any mesh).  Each warp first
 // tests an element against the bounding box of its 32 points with the same
 // operations: IEEE subtraction is monotonic, so a box distance above the
 // limit means every point of the warp is far by the per-point test, and the
 // 32 point tests are skipped.
+constexpr int CL_EC = 64;
 __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, const float4* __restrict__ rows,
                                                             const ElemRec* __restrict__ elems, int nn,
                                                             int* pair_count, int2* pairs, int pair_cap) {
-  __shared__ ElemRec s_e[256];
+  __shared__ ElemRec s_e[CL_EC];
   const int i = blockIdx.x * 256 + threadIdx.x;
-  const int e0 = blockIdx.y * 256;
-  const int nel = min(256, ne - e0);
+  const int e0 = blockIdx.y * CL_EC;
+  const int nel = min(CL_EC, ne - e0);
   if ((int)threadIdx.x < nel) s_e[threadIdx.x] = elems[e0 + threadIdx.x];
   __syncthreads();
   const bool valid = i < nt;
@@ -728,17 +742,10 @@ static void launch_variant(const AsmRequest& q, cudaStream_t st) {
   fa.ph = q.ph;
   fa.rows = q.rows; fa.nodes = q.nodes; fa.elems = q.elems;
   fa.nodes_df = q.nodes_df; fa.logtab = q.logtab;
-  if constexpr (PREC == 3) {
-    logtab_kernel<<<1, 160, 0, st>>>(q.logtab);
-    if constexpr (NC == 1) {
-      pack_nodes_df_kernel<<<(g.n + 255) / 256, 256, 0, st>>>(g, q.R, q.ph, q.bv, q.nodes_df);
-    } else {
-      pack_nodes_dfk_kernel<<<(g.n + 255) / 256, 256, 0, st>>>(g, q.R, q.ph, q.bv, (NodeDFK*)q.nodes_df);
-      const df::f2 c1 = df::from_double(1 - 2 * q.ph.nu);
-      fa.c1h = c1.h;
-      fa.c1l = c1.l;
-    }
-    count_launches(2);
+  if constexpr (PREC == 3 && NC == 4) {
+    const df::f2 c1 = df::from_double(1 - 2 * q.ph.nu);
+    fa.c1h = c1.h;
+    fa.c1l = c1.l;
   }
   fa.px = g.px; fa.py = g.py; fa.nx = g.nx; fa.ny = g.ny; fa.jac = g.jac;
   for (int k = 0; k < BEM_MAXNN; ++k) fa.ew[k] = q.R.ew[k];
@@ -766,7 +773,7 @@ static void launch_variant(const AsmRequest& q, cudaStream_t st) {
   // writes its own entries; row sums are atomic)
   {
     KScope ks(st, KC_NEAR);
-    dim3 cg((g.nt + 255) / 256, (g.ne + 255) / 256);
+    dim3 cg((g.nt + 255) / 256, (g.ne + CL_EC - 1) / CL_EC);
     near_classify_kernel<<<cg, 256, 0, st>>>(g.nt, g.ne, q.rows, q.elems, g.nn, q.counters, q.pairs, q.pair_cap);
   }
   const bool side = q.aux != nullptr && g.n > 0;
@@ -800,16 +807,13 @@ static void launch_variant(const AsmRequest& q, cudaStream_t st) {
     if (side2) cudaStreamWaitEvent(st, q.ev_join2, 0);
     launch_finalize(fi, NC, g.nt, st);
   }
-  count_launches(PREC == 3 ? 8 : 9);
+  count_launches(6);
 }
 
 int launch_assembly(const AsmRequest& q, cudaStream_t st) {
   const GeomDev& g = q.g;
   const int dof = q.ph.kind == 0 ? 1 : 2;
   if (g.nt <= 0 || g.n <= 0 || g.ne <= 0) return (int)cudaErrorInvalidValue;
-  cudaMemsetAsync(q.rowsum, 0, sizeof(double) * (size_t)g.nt * dof * dof, st);
-  cudaMemsetAsync(q.counters, 0, 2 * sizeof(int), st);
-  if (q.fused) cudaMemsetAsync(q.b, 0, sizeof(double) * (size_t)g.nt * dof, st);
   // columns of internal points: zero except the diagonal (finalize)
   if (g.nt > g.n) {
     size_t esz = (q.prec == 0) ? 4 : 8;
@@ -818,14 +822,22 @@ int launch_assembly(const AsmRequest& q, cudaStream_t st) {
     cudaMemsetAsync((char*)q.H + off * esz, 0, cnt * esz, st);
     if (q.prec == 2) cudaMemsetAsync(q.A32 + off, 0, cnt * 4, st);
   }
-  pack_rows_kernel<<<(g.nt + 255) / 256, 256, 0, st>>>(g, q.rows);
-  if (q.prec == 0)
-    pack_nodes_kernel<<<(g.n + 255) / 256, 256, 0, st>>>(g, q.R, q.ph, q.nodes);
-  else if (q.prec != 3)
-    pack_nodes_d_kernel<<<(g.n + 255) / 256, 256, 0, st>>>(g, q.R, q.ph, (NodeD*)q.nodes);
-  cudaMemsetAsync(q.absmax, 0, sizeof(unsigned long long), st);
-  absmax_kernel<<<64, 256, 0, st>>>(g, q.absmax);
-  pack_elems_kernel<<<(g.ne + 255) / 256, 256, 0, st>>>(g, q.near_factor, q.absmax, q.elems);
+  PackArgs pa{};
+  pa.g = g;
+  pa.R = q.R;
+  pa.ph = q.ph;
+  pa.near_factor = q.near_factor;
+  pa.prec = q.prec;
+  pa.dof = dof;
+  pa.bv = q.bv;
+  pa.rows = q.rows;
+  pa.nodes = q.prec == 3 ? (void*)q.nodes_df : (void*)q.nodes;
+  pa.elems = q.elems;
+  pa.logtab = q.logtab;
+  pa.rowsum = q.rowsum;
+  pa.b = q.fused ? q.b : nullptr;
+  pa.counters = q.counters;
+  pack_kernel<<<(g.nt + 255) / 256, 256, 0, st>>>(pa);
   const int key = q.ph.kind * 100 + q.prec * 10 + q.fused;
   switch (key) {
     case 0: launch_variant<1, 0, false>(q, st); break;

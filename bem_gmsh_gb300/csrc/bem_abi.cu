@@ -181,6 +181,24 @@ char* bem_ctx::pinned(size_t bytes) {
   return pin;
 }
 
+char* bem_ctx::pinned_out(size_t bytes) {
+  if (pout_bytes >= bytes) return pout;
+  if (pout) {
+    cudaStreamSynchronize(stream);
+    cudaFreeHost(pout);
+  }
+  pout = nullptr;
+  pout_bytes = 0;
+  const size_t want = (bytes + bytes / 8 + 4095) / 4096 * 4096;
+  if (cudaHostAlloc((void**)&pout, want, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    pout = nullptr;
+    return nullptr;
+  }
+  pout_bytes = want;
+  return pout;
+}
+
 char* bem_ctx::solver_words() {
   if (!swords && cudaHostAlloc((void**)&swords, 1024, cudaHostAllocDefault) != cudaSuccess) {
     cudaGetLastError();
@@ -261,6 +279,7 @@ extern "C" int bem_ctx_destroy(bem_ctx* c) {
     if (b.p) cudaFree(b.p);
   if (c->pin) cudaFreeHost(c->pin);
   if (c->swords) cudaFreeHost(c->swords);
+  if (c->pout) cudaFreeHost(c->pout);
   if (c->pin_ev) cudaEventDestroy(c->pin_ev);
   for (auto e : c->tev)
     if (e) cudaEventDestroy(e);
@@ -388,7 +407,16 @@ int bem_stage_geom(bem_ctx* c, const bem_geom2d* g, int npg, int mem, GeomDev& g
 
 // Runs one assembly (device pointers already set in q), retrying once with
 // a larger pair list if the first estimate overflowed.
-int bem_run_assembly(bem_ctx* c, AsmRequest& q) {
+int bem_assembly_result(bem_ctx* c, const int* counts) {
+  if (counts[1] != 0) {
+    c->last_error = "bulk-copy wait timed out in the far-field kernel";
+    return BEM_ERR_INTERNAL;
+  }
+  c->pair_cap_hint = std::max(c->pair_cap_hint, counts[0] + counts[0] / 4 + 1024);
+  return counts[0] <= c->asm_cap ? BEM_OK : BEM_RETRY;
+}
+
+int bem_run_assembly(bem_ctx* c, AsmRequest& q, bool later) {
   const int nt = q.g.nt;
   const int dof = q.ph.kind == 0 ? 1 : 2;
   q.rows = (float4*)c->get(bem_ctx::SLOT_ROWS, sizeof(float4) * (size_t)nt);
@@ -397,8 +425,8 @@ int bem_run_assembly(bem_ctx* c, AsmRequest& q) {
   q.rowsum = (double*)c->get(bem_ctx::SLOT_ROWSUM, sizeof(double) * (size_t)nt * dof * dof);
   q.gdiag = (double*)c->get(bem_ctx::SLOT_GDIAG, sizeof(double) * (size_t)q.g.n * dof * dof);
   q.counters = (int*)c->get(bem_ctx::SLOT_COUNTERS, 64);
-  q.absmax = (unsigned long long*)((char*)q.counters + 32);
   if (!q.rows || !q.nodes || !q.elems || !q.rowsum || !q.gdiag || !q.counters) return BEM_ERR_NOMEM;
+  c->asm_count = nullptr;
   if (!c->asm_stream) {
     int lo = 0, hi = 0;
     cudaDeviceGetStreamPriorityRange(&lo, &hi);
@@ -420,28 +448,27 @@ int bem_run_assembly(bem_ctx* c, AsmRequest& q) {
     q.logtab = (float4*)c->get(bem_ctx::SLOT_LOGTAB, sizeof(float4) * 136);
     if (!q.nodes_df || !q.logtab) return BEM_ERR_NOMEM;
   }
-  int cap = c->pair_cap_hint > 0 ? c->pair_cap_hint : nt * 16 + 4096;
+  int cap = std::max(c->pair_cap_hint, nt * 16 + 4096);
   for (int attempt = 0; attempt < 3; ++attempt) {
     q.pairs = (int2*)c->get(bem_ctx::SLOT_PAIRS, sizeof(int2) * (size_t)cap);
     if (!q.pairs) return BEM_ERR_NOMEM;
     q.pair_cap = cap;
     int rc = bem::launch_assembly(q, c->stream);
     if (rc != 0) return c->cuda_fail((cudaError_t)rc, "launch_assembly");
-    // pair count and far-kernel status through the pinned buffer
-    int* hc = (int*)c->pinned(64);
+    c->asm_cap = cap;
+    if (later) {
+      c->asm_count = q.counters;
+      return BEM_OK;
+    }
+    // pair count and far-kernel status through the page-locked words
+    int* hc = (int*)c->solver_words();
     if (!hc) return BEM_ERR_NOMEM;
     cudaMemcpyAsync(hc, q.counters, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return c->cuda_fail(e, "assembly");
-    if (hc[1] != 0) {
-      c->last_error = "bulk-copy wait timed out in the far-field kernel";
-      return BEM_ERR_INTERNAL;
-    }
-    if (hc[0] <= cap) {
-      c->pair_cap_hint = std::max(c->pair_cap_hint, hc[0] + hc[0] / 4 + 1024);
-      return BEM_OK;
-    }
-    cap = hc[0] + hc[0] / 4 + 1024;
+    rc = bem_assembly_result(c, hc);
+    if (rc != BEM_RETRY) return rc;
+    cap = c->pair_cap_hint;
   }
   return BEM_ERR_INTERNAL;
 }
@@ -517,7 +544,7 @@ extern "C" int bem_assemble_kelvin2d(bem_ctx* c, const bem_geom2d* g, double mu,
 // ---------------------------------------------------------------------------
 int bem_assemble_system_dev(bem_ctx* c, const bem_geom2d* g, const Physics& ph, const int32_t* BC,
                             const double* BV, int npg, double nf, int mem, int prec, double* A,
-                            int64_t lda, float* A32, double* b) {
+                            int64_t lda, float* A32, double* b, bool later) {
   int rc = bem_check_geom(g, npg, nf);
   if (rc) return rc;
   const int dof = ph.kind == 0 ? 1 : 2;
@@ -536,7 +563,7 @@ int bem_assemble_system_dev(bem_ctx* c, const bem_geom2d* g, const Physics& ph, 
   q.ldg = lda;
   q.A32 = A32;
   q.b = b;
-  return bem_run_assembly(c, q);
+  return bem_run_assembly(c, q, later);
 }
 
 extern "C" int bem_assemble_system2d(bem_ctx* c, const bem_geom2d* g, int kind, double prm0,

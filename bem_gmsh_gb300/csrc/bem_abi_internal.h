@@ -30,6 +30,9 @@ struct bem_ctx {
   std::string last_error;
   Buf slots[NSLOT];
   int pair_cap_hint = 0;
+  // the assembly not yet checked (bem_run_assembly with `later`), else null
+  const int* asm_count = nullptr;
+  int asm_cap = 0;
   int opt_tcgen05 = 2;  // BEM_OPT_TCGEN05: trailing updates on tcgen05 (2: persistent kernel)
   int opt_tc_reserve = 0;  // BEM_OPT_TC_RESERVE: SMs the persistent kernel leaves free
   int opt_far_df = 1;   // BEM_OPT_FAR_DF
@@ -79,6 +82,11 @@ struct bem_ctx {
   // (apart from the staging buffer, whose next use waits for its last copy);
   // NULL on allocation failure
   char* solver_words();
+  // Grow-only page-locked buffer for a solve's solution (the staging buffer
+  // would first wait for the inputs' copy).  NULL on allocation failure.
+  char* pinned_out(size_t bytes);
+  char* pout = nullptr;
+  size_t pout_bytes = 0;
   char* swords = nullptr;
   char* pin = nullptr;
   size_t pin_bytes = 0;
@@ -115,7 +123,14 @@ void bem_build_rules(const bem_geom2d* g, int npg, const double* ew_host, bem::R
 int bem_stage_geom(bem_ctx* c, const bem_geom2d* g, int npg, int mem, bem::GeomDev& gd,
                    bem::Rules& R, int64_t nb = 0, const int32_t* BC = nullptr, const double* BV = nullptr,
                    const int32_t** dBC = nullptr, const double** dBV = nullptr);
-int bem_run_assembly(bem_ctx* c, bem::AsmRequest& q);
+// Runs one assembly.  With `later`, nothing is waited for: the pair count and
+// the far kernel's status (asm_count, two device ints) are checked by the
+// solve that follows, with bem_assembly_result.
+int bem_run_assembly(bem_ctx* c, bem::AsmRequest& q, bool later = false);
+// BEM_OK; BEM_RETRY when the pair list was too short (the next assembly of
+// the context has a longer one); BEM_ERR_INTERNAL
+constexpr int BEM_RETRY = 1000;
+int bem_assembly_result(bem_ctx* c, const int* counts);
 int bem_assemble_system_dev(bem_ctx* c, const bem_geom2d* g, const bem::Physics& ph,
                             const int32_t* BC, const double* BV, int npg, double nf, int mem,
-                            int prec, double* A, int64_t lda, float* A32, double* b);
+                            int prec, double* A, int64_t lda, float* A32, double* b, bool later = false);

@@ -165,7 +165,6 @@ struct AsmRequest {
   int* counters;  // [0] pair count, [1] status
   int2* pairs;
   int pair_cap;
-  unsigned long long* absmax;  // scratch: largest |coordinate|
   // optional side stream for the on-element kernel (runs beside the far and
   // near kernels; joined before the diagonal), with its fork/join events
   cudaStream_t aux = nullptr, aux2 = nullptr;

@@ -53,9 +53,10 @@ void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, dou
 // ints at info.
 void gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
                     int* hinfo, cudaStream_t st);
-// v = r / |r| (zeros for r = 0), x = 0 when given; *host = |r|^2
+// v = r / |r| (zeros for r = 0), x = 0 when given; *host = |r|^2; hcnt: the
+// two ints at cnt, when given
 void normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
-                 cudaStream_t st);
+                 cudaStream_t st, const int* cnt = nullptr, int* hcnt = nullptr);
 // x += Z[:, 0:m] y (y on the host, m <= 32), w = b
 void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
               cudaStream_t st);

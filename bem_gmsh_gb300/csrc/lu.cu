@@ -922,10 +922,11 @@ __global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
   }
 }
 
-// v = r / |r|, |r|^2 to the host; x (when given) zeroed
+// v = r / |r|, |r|^2 to the host; x (when given) zeroed, cnt's two ints copied
 __global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
     k_normalize(const double* __restrict__ r, int N, double* __restrict__ v, double* __restrict__ x,
-                double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo) {
+                double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo,
+                const int* __restrict__ cnt, int* __restrict__ hcnt) {
   __shared__ GsShared s;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int chunk = (N + GS_CTAS - 1) / GS_CTAS, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
@@ -943,6 +944,10 @@ __global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
     *host = n2;
     hinfo[0] = info[0];
     hinfo[1] = info[1];
+    if (cnt) {
+      hcnt[0] = cnt[0];
+      hcnt[1] = cnt[1];
+    }
   }
 }
 
@@ -1954,9 +1959,9 @@ void gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, doubl
   k_gram_schmidt<<<GS_CTAS, GS_THREADS, 0, st>>>(V, ldv, N, m, w, vn, host, info, hinfo);
 }
 void normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
-                 cudaStream_t st) {
+                 cudaStream_t st, const int* cnt, int* hcnt) {
   count_launches(1);
-  k_normalize<<<GS_CTAS, GS_THREADS, 0, st>>>(r, N, v, x, host, info, hinfo);
+  k_normalize<<<GS_CTAS, GS_THREADS, 0, st>>>(r, N, v, x, host, info, hinfo, cnt, hcnt);
 }
 void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
               cudaStream_t st) {

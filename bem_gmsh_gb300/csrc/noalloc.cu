@@ -120,7 +120,6 @@ extern "C" int bem_assemble_laplace2d_noalloc(const bem_geom2d* geom, double k, 
   q.rowsum = (double*)(base + kOffRowsum);
   q.gdiag = (double*)(base + kOffGdiag);
   q.counters = (int*)(base + kOffCounters);
-  q.absmax = (unsigned long long*)(base + kOffCounters + 32);
   q.pairs = (int2*)(base + kOffPairs);
   q.pair_cap = kPairCap;
   int lrc = bem::launch_assembly(q, st);

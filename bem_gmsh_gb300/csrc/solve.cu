@@ -100,7 +100,7 @@ struct Timer {
 struct SolvePin {
   double* hh;
   double* dot;
-  int* info;  // 4 ints: after the factorization, after the last iteration
+  int* info;  // 2 ints after the factorization, 2 after the last iteration, the assembly's 2
 };
 bool solve_pin(bem_ctx* c, SolvePin& p) {
   double* d = (double*)c->solver_words();
@@ -131,6 +131,8 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   const int m = 30;  // restart length
   cudaStream_t st = c->stream;
   c->mixed_fail = bem_ctx::MIXED_OK;
+  const int* asm_count = c->asm_count;
+  c->asm_count = nullptr;
   float* A32 = (float*)c->get(bem_ctx::SLOT_LU0, sizeof(float) * (size_t)Npad * Npad);
   double* cs = (double*)c->get(bem_ctx::SLOT_LU1, sizeof(double) * (size_t)N);
   float* Dinv = (float*)c->get(bem_ctx::SLOT_LU2, sizeof(float) * bem::lu_dinv_floats(K));
@@ -167,8 +169,7 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   // inverses, sweep couplings)
   // info[16], info[17]: tile counter of the persistent bulk updates
   auto factor = [&]() -> int {
-    cudaMemsetAsync(info, 0, 2 * sizeof(int), st);
-    cudaMemsetAsync(info + 16, 0, 2 * sizeof(int), st);
+    cudaMemsetAsync(info, 0, 18 * sizeof(int), st);
     bem::lu_prepare(A64, lda, N, Npad, cs, A32, Npad, st);
     int r;
     if (lookahead)
@@ -237,7 +238,7 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   // first iteration is queued behind the factorization before anything of
   // either is known.  x = 0 at the start, so the first residual is b.
   std::vector<double> H((m + 1) * m), cg(m), sg(m), gvec(m + 1), y(m);
-  bem::normalize64(b, N, V, x, pin.dot, info, pin.info, st);
+  bem::normalize64(b, N, V, x, pin.dot, info, pin.info, st, asm_count, pin.info + 4);
   int iters = 0, prc = 0;
   bool converged = false, first = true;
   double bnorm = 0.0, beta = 0.0, prev_beta = INFINITY, relres = 1.0;
@@ -254,6 +255,10 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
       if (e != cudaSuccess) return c->cuda_fail(e, first ? "factor" : "refinement");
       if (first) {
         first = false;
+        if (asm_count) {
+          const int ar = bem_assembly_result(c, pin.info + 4);
+          if (ar != BEM_OK) return ar;
+        }
         if (stats) stats->t_factor_ms = tf.ms();
         if (pin.info[1]) {
           c->last_error = "tensor-core GEMM wait timed out in the LU";
@@ -454,6 +459,7 @@ extern "C" int bem_solve_system(bem_ctx* c, int64_t n, const double* A, int64_t 
   if (mem != BEM_MEM_HOST && mem != BEM_MEM_DEVICE) return BEM_ERR_INVALID;
   if (!(tol > 0) || max_iter < 1) return BEM_ERR_INVALID;
   CallScope cscope(c);
+  c->asm_count = nullptr;
   cudaSetDevice(c->device);
   const int N = (int)n;
   if (stats) std::memset(stats, 0, sizeof(*stats));
@@ -526,17 +532,26 @@ extern "C" int bem_solve2d(bem_ctx* c, const bem_geom2d* g, int kind, double prm
   ta.start(c->stream);
   // the FP64 comparison path keeps FP64 arithmetic throughout
   const int prec = (mode == BEM_SOLVE_MIXED && c->opt_far_df >= 1) ? 3 : 1;
-  rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b);
+  // the mixed solve checks the assembly's pair count with its own first
+  // results; one that had too short a list is run again
+  rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b,
+                               mode == BEM_SOLVE_MIXED);
   ta.stop(c->stream);
   if (rc) return rc;
-  double t_asm = ta.ms();
   double* hx = nullptr;
   if (mem == BEM_MEM_HOST) {
-    hx = (double*)c->pinned(sizeof(double) * (size_t)N);
+    hx = (double*)c->pinned_out(sizeof(double) * (size_t)N);
     if (!hx) return BEM_ERR_NOMEM;
   }
   if (mode == BEM_SOLVE_MIXED) {
     rc = bem_solve_mixed_safe(c, N, A, ld, true, b, tol, max_iter, dx, stats, hx);
+    if (rc == BEM_RETRY) {
+      ta.start(c->stream);
+      rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b);
+      ta.stop(c->stream);
+      if (rc) return rc;
+      rc = bem_solve_mixed_safe(c, N, A, ld, true, b, tol, max_iter, dx, stats, hx);
+    }
   } else {
     rc = bem_solve_fp64_dev(c, N, A, ld, b, dx, stats);
     if (hx && (rc == BEM_OK || rc == BEM_ERR_NOT_CONVERGED)) {
@@ -545,7 +560,7 @@ extern "C" int bem_solve2d(bem_ctx* c, const bem_geom2d* g, int kind, double prm
       if (e != cudaSuccess) return c->cuda_fail(e, "copy x to host");
     }
   }
-  if (stats) stats->t_assemble_ms = t_asm;
+  if (stats) stats->t_assemble_ms = ta.ms();
   if (rc != BEM_OK && rc != BEM_ERR_NOT_CONVERGED) return rc;
   if (hx) std::memcpy(x, hx, sizeof(double) * N);
   return rc;
