@@ -577,11 +577,6 @@ __device__ __forceinline__ bool trsv_sweep(TrsvShared& sh, float* Ds, const floa
   if (t == 0) sh.bad = 0;
   float mreg[LU_NB / 2];
   if (owner) {
-    const float* Db = Dinv + (size_t)b * 2 * LU_NB * LU_NB + (UPPER ? LU_NB * LU_NB : 0);
-    for (int idx = t; idx < LU_NB * LU_NB; idx += blockDim.x) {
-      int rr = idx & (LU_NB - 1), c = idx >> 7;
-      Ds[c * (LU_NB + 1) + rr] = Db[rr + (size_t)c * LU_NB];
-    }
     // this thread's half row of the coupling to the adjacent block
     if (nj > 0) {
       const float* Mb = Mc + (size_t)(2 * b + (UPPER ? 1 : 0)) * LU_NB * LU_NB;
@@ -719,12 +714,14 @@ __device__ __forceinline__ bool trsv_sweep(TrsvShared& sh, float* Ds, const floa
   }
   // z_b = D_b (r_b - ...)
   if (t < LU_NB) sh.ys[t] = sum;
+  if (UPPER) cp_async_wait<0>();
+  else cp_async_wait<1>();
   __syncthreads();
   float o0 = 0.f, o1 = 0.f;
 #pragma unroll 16
   for (int q = half * (LU_NB / 2); q < (half + 1) * (LU_NB / 2); q += 2) {
-    o0 += Ds[q * (LU_NB + 1) + row] * sh.ys[q];
-    o1 += Ds[(q + 1) * (LU_NB + 1) + row] * sh.ys[q + 1];
+    o0 += Ds[q * LU_NB + row] * sh.ys[q];
+    o1 += Ds[(q + 1) * LU_NB + row] * sh.ys[q + 1];
   }
   sh.part[half][row] = o0 + o1;
   __syncthreads();
@@ -766,11 +763,23 @@ __global__ void __launch_bounds__(256) k_trsv(const float* __restrict__ A, int64
                                               unsigned long long* t0, unsigned long long* t1, unsigned long long* p0,
                                               unsigned long long* p1, int P, int epoch, int wepoch, int wait_limit,
                                               int* err) {
-  extern __shared__ float Ds[];  // the block's inverse, [col][row], LU_NB * (LU_NB + 1)
+  extern __shared__ __align__(16) float Ds[];  // the inverses of the CTA's two blocks, [col][row]
   __shared__ TrsvShared sh;
+  // both inverses are on their way before the first wait (scalar loads of
+  // one at the start of each sweep were 5 us of every application)
+  if ((int)blockIdx.x % P == P - 1) {
+    const int bi = (int)blockIdx.x / P;
+    const float* D0 = Dinv + (size_t)bi * 2 * LU_NB * LU_NB;
+    const float* D1 = Dinv + ((size_t)(K - 1 - bi) * 2 + 1) * LU_NB * LU_NB;
+    for (int q = 4 * threadIdx.x; q < LU_NB * LU_NB; q += 4 * blockDim.x) cp_async16(Ds + q, D0 + q);
+    cp_async_commit();
+    for (int q = 4 * threadIdx.x; q < LU_NB * LU_NB; q += 4 * blockDim.x) cp_async16(Ds + LU_NB * LU_NB + q, D1 + q);
+    cp_async_commit();
+  }
   bool ok = trsv_sweep<false>(sh, Ds, A, ld, K, Dinv, Mc, v, N, nullptr, t0, p0, P, epoch, wepoch, wait_limit, cs, z, w);
   __syncthreads();
-  if (ok) ok = trsv_sweep<true>(sh, Ds, A, ld, K, Dinv, Mc, v, N, t0, t1, p1, P, epoch, wepoch, wait_limit, cs, z, w);
+  if (ok) ok = trsv_sweep<true>(sh, Ds + LU_NB * LU_NB, A, ld, K, Dinv, Mc, v, N, t0, t1, p1, P, epoch, wepoch, wait_limit, cs, z, w);
+  cp_async_wait<0>();
   if (!ok && threadIdx.x == 0) atomicExch(err, 1);
 }
 
@@ -819,17 +828,18 @@ __global__ void __launch_bounds__(32 * GV_WARPS) k_gemv64(const double* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Gram-Schmidt step of the refinement in one cluster of eight CTAs.
+// Gram-Schmidt step of the refinement in one cluster of 8 or 16 CTAs.
 // The vectors are short (N <= 10^4 doubles, all in L2) and the arithmetic is
 // small; what cost was the launches: three dot products, two updates, a
 // normalization, three memsets and a copy to the host, about 30 us of stream
-// time per iteration.  Eight SMs hold an eighth of the rows each; the partial
-// sums meet through distributed shared memory, one cluster barrier per
-// reduction, and the coefficients go straight to the host's page-locked
-// words.  8 us at N = 8193 with five vectors (FP64 issue of eight SMs), 5 us
-// at N = 160.
+// time per iteration.  Each SM holds a slice of the rows; the partial sums
+// meet through distributed shared memory, one cluster barrier per reduction,
+// and the coefficients go straight to the host's page-locked words.  Four
+// warps per CTA, one per scheduler: a warp's FP64 add takes 64 cycles of its
+// scheduler whatever it adds, so more warps only lengthen the reductions
+// (with 16 of them a step took 15 us at N = 1023; now 8).
 // ---------------------------------------------------------------------------
-constexpr int GS_CTAS = 8, GS_THREADS = 512, GS_MAXV = 32;
+constexpr int GS_CTAS = 16, GS_THREADS = 128, GS_MAXV = 32;
 
 struct GsShared {
   double warp[GS_THREADS / 32][GS_MAXV];
@@ -859,62 +869,63 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 __device__ __forceinline__ void gs_reduce(GsShared& s, int m, int buf) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, nc = (int)cl.num_blocks();
   __syncthreads();
-  if (t < m * GS_CTAS) {
-    const int q = t % m, to = t / m;
-    double v = 0.0;
+  for (int v = t; v < m * nc; v += GS_THREADS) {
+    const int q = v % m, to = v / m;
+    double x = 0.0;
 #pragma unroll
-    for (int w = 0; w < GS_THREADS / 32; ++w) v += s.warp[w][q];
-    *cl.map_shared_rank(&s.part[buf][cl.block_rank()][q], to) = v;
+    for (int w = 0; w < GS_THREADS / 32; ++w) x += s.warp[w][q];
+    *cl.map_shared_rank(&s.part[buf][cl.block_rank()][q], to) = x;
   }
   cl.sync();
   if (t < m) {
-    double v = 0.0;
-#pragma unroll
-    for (int r = 0; r < GS_CTAS; ++r) v += s.part[buf][r][t];
-    s.h[t] = v;
+    double x = 0.0;
+    for (int r = 0; r < nc; ++r) x += s.part[buf][r][t];
+    s.h[t] = x;
   }
   __syncthreads();
 }
 
 // w -= V (V^T w) twice (classical Gram-Schmidt with reorthogonalization),
-// vn = w / |w|.  host: [0..31] and [32..61] the two passes' coefficients,
-// [62] |w|^2; hinfo: the two LU status words.
-__global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
+// vn = w / |w|.  The second pass's sums include |w|^2 before that pass, and
+// |w|^2 after it is that minus the squared coefficients (they are rounding
+// next to it).  host: [0..31] and [32..61] the two passes' coefficients, [62]
+// |w|^2; hinfo: the two LU status words.
+__global__ void __launch_bounds__(GS_THREADS)
     k_gram_schmidt(const double* __restrict__ V, int64_t ldv, int N, int m, double* w, double* __restrict__ vn,
                    double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo) {
   __shared__ GsShared s;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int chunk = (N + GS_CTAS - 1) / GS_CTAS, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
+  const int chunk = (N + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
   for (int pass = 0; pass < 2; ++pass) {
-    for (int q0 = 0; q0 < m; q0 += 8) {
+    const int cnt = m + pass;  // the second pass's last value is |w|^2
+    for (int q0 = 0; q0 < cnt; q0 += 8) {
       double acc[8] = {};
       for (int i = i0 + t; i < i1; i += GS_THREADS) {
-        const double wi = w[i];
+        double wi = w[i];
+        if (pass == 1 && q0 == 0) {
+          for (int q = 0; q < m; ++q) wi = fma(-V[i + (size_t)q * ldv], s.h[q], wi);
+          w[i] = wi;
+        }
 #pragma unroll
         for (int q = 0; q < 8; ++q)
-          if (q0 + q < m) acc[q] = fma(V[i + (size_t)(q0 + q) * ldv], wi, acc[q]);
+          if (q0 + q < cnt) acc[q] = fma(q0 + q < m ? V[i + (size_t)(q0 + q) * ldv] : wi, wi, acc[q]);
       }
       const double v = warp_sum8(acc, lane);
       if ((lane & 3) == 0) s.warp[warp][q0 + (lane >> 2)] = v;
     }
-    gs_reduce(s, m, pass);
+    gs_reduce(s, cnt, pass);
     if (blockIdx.x == 0 && t < m) host[32 * pass + t] = s.h[t];
-    for (int i = i0 + t; i < i1; i += GS_THREADS) {
-      double a = w[i];
-      for (int q = 0; q < m; ++q) a = fma(-V[i + (size_t)q * ldv], s.h[q], a);
-      w[i] = a;
-    }
-    __syncthreads();
   }
-  double acc = 0.0;
-  for (int i = i0 + t; i < i1; i += GS_THREADS) acc = fma(w[i], w[i], acc);
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) s.warp[warp][0] = acc;
-  gs_reduce(s, 1, 0);
-  const double n2 = s.h[0], sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
-  for (int i = i0 + t; i < i1; i += GS_THREADS) vn[i] = w[i] * sc;
+  double n2 = s.h[m];
+  for (int q = 0; q < m; ++q) n2 = fma(-s.h[q], s.h[q], n2);
+  const double sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+  for (int i = i0 + t; i < i1; i += GS_THREADS) {
+    double a = w[i];
+    for (int q = 0; q < m; ++q) a = fma(-V[i + (size_t)q * ldv], s.h[q], a);
+    vn[i] = a * sc;
+  }
   if (blockIdx.x == 0 && t == 0) {
     host[62] = n2;
     hinfo[0] = info[0];
@@ -923,13 +934,13 @@ __global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
 }
 
 // v = r / |r|, |r|^2 to the host; x (when given) zeroed, cnt's two ints copied
-__global__ void __cluster_dims__(GS_CTAS, 1, 1) __launch_bounds__(GS_THREADS)
+__global__ void __launch_bounds__(GS_THREADS)
     k_normalize(const double* __restrict__ r, int N, double* __restrict__ v, double* __restrict__ x,
                 double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo,
                 const int* __restrict__ cnt, int* __restrict__ hcnt) {
   __shared__ GsShared s;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int chunk = (N + GS_CTAS - 1) / GS_CTAS, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
+  const int chunk = (N + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
   double acc = 0.0;
   for (int i = i0 + t; i < i1; i += GS_THREADS) acc = fma(r[i], r[i], acc);
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -1912,12 +1923,12 @@ int lu_solve_vec(const float* A, int64_t ld, int N, int Npad, const float* Dinv,
     int dev = 0, nsm = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int dsm = (int)(sizeof(float) * LU_NB * (LU_NB + 1));
+    const int dsm = (int)(sizeof(float) * 2 * LU_NB * LU_NB);
     cudaFuncSetAttribute(k_trsv, cudaFuncAttributeMaxDynamicSharedMemorySize, dsm);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trsv, 256, dsm);
     max_coresident = nsm * per;
   });
-  const size_t dsm = sizeof(float) * LU_NB * (LU_NB + 1);
+  const size_t dsm = sizeof(float) * 2 * LU_NB * LU_NB;
   if (K > max_coresident) {  // too many block rows to keep resident: step-wise launches
     k_to_f32<<<(Npad + 255) / 256, 256, 0, st>>>(v, N, Npad, rf);
     lu_solve_vec_steps(A, ld, Npad, Dinv, rf, rf + Npad, st);
@@ -1953,15 +1964,38 @@ void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, dou
   k_gemv64<<<dim3(rb, (N + cols - 1) / cols), 32 * GV_WARPS, 0, st>>>(A, lda, N, x, y, alpha, cols);
 }
 
+// one cluster: 16 CTAs (beyond the portable size) from N = 4096 on, where a
+// slice's FP64 arithmetic outweighs the wider barrier; else 8
+template <class... P, class... X>
+static void gs_launch(void (*kern)(P...), int N, cudaStream_t st, X... args) {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaFuncSetAttribute(k_gram_schmidt, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(k_normalize, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
+  const unsigned nc = N >= 4096 ? GS_CTAS : 8;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = nc;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nc);
+  cfg.blockDim = dim3(GS_THREADS);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 void gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
                     int* hinfo, cudaStream_t st) {
   count_launches(1);
-  k_gram_schmidt<<<GS_CTAS, GS_THREADS, 0, st>>>(V, ldv, N, m, w, vn, host, info, hinfo);
+  gs_launch(k_gram_schmidt, N, st, V, ldv, N, m, w, vn, host, info, hinfo);
 }
 void normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
                  cudaStream_t st, const int* cnt, int* hcnt) {
   count_launches(1);
-  k_normalize<<<GS_CTAS, GS_THREADS, 0, st>>>(r, N, v, x, host, info, hinfo, cnt, hcnt);
+  gs_launch(k_normalize, N, st, r, N, v, x, host, info, hinfo, cnt, hcnt);
 }
 void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
               cudaStream_t st) {
