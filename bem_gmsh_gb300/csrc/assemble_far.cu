@@ -202,7 +202,9 @@ __global__ void __launch_bounds__(256) pack_kernel(const __grid_constant__ PackA
 // tests an element against the bounding box of its 32 points with the same
 // operations: IEEE subtraction is monotonic, so a box distance above the
 // limit means every point of the warp is far by the per-point test, and the
-// 32 point tests are skipped.
+// 32 point tests are skipped.  The hits of all the warp's elements take one
+// place in the list: an atomic with its return per element made a serial
+// chain of memory latencies (14 to 23 us, whatever the mesh).
 constexpr int CL_EC = 64;
 __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, const float4* __restrict__ rows,
                                                             const ElemRec* __restrict__ elems, int nn,
@@ -224,6 +226,8 @@ __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, cons
     by0 = fminf(by0, __shfl_xor_sync(0xffffffffu, by0, o));
     by1 = fmaxf(by1, __shfl_xor_sync(0xffffffffu, by1, o));
   }
+  // hit masks of element el: lane el % 32, word el / 32
+  unsigned m0 = 0, m1 = 0;
   for (int el = 0; el < nel; ++el) {
     const ElemRec E = s_e[el];
     const float dx = fmaxf(fmaxf(__fsub_rn(E.lox, bx1), __fsub_rn(bx0, E.hix)), 0.f);
@@ -232,16 +236,28 @@ __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, cons
     // (a point on the element itself belongs to the on-element kernel)
     const bool need = valid && (i < (e0 + el) * nn || i >= (e0 + el + 1) * nn) && !box_far(r.x, r.y, r.z, r.w, E);
     const unsigned m = __ballot_sync(0xffffffffu, need);
-    if (m) {
-      const int leader = __ffs(m) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(pair_count, __popc(m));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (need) {
-        const int slot = base + __popc(m & ((1u << lane) - 1));
-        if (slot < pair_cap) pairs[slot] = make_int2(i, e0 + el);
-      }
-    }
+    if (lane == (el & 31)) (el < 32 ? m0 : m1) = m;
+  }
+  const int cnt = __popc(m0) + __popc(m1);
+  int inc = cnt;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, inc, 31);
+  if (total == 0) return;  // warp-uniform
+  int base = 0;
+  if (lane == 0) base = atomicAdd(pair_count, total);
+  base = __shfl_sync(0xffffffffu, base, 0) + inc - cnt;
+  for (unsigned busy = __ballot_sync(0xffffffffu, cnt != 0); busy; busy &= busy - 1) {
+    const int src = __ffs(busy) - 1;
+    const unsigned a0 = __shfl_sync(0xffffffffu, m0, src), a1 = __shfl_sync(0xffffffffu, m1, src);
+    const int first = __shfl_sync(0xffffffffu, base, src);
+    const unsigned below = (1u << lane) - 1;
+    int slot = first + __popc(a0 & below);
+    if ((a0 >> lane & 1) && slot < pair_cap) pairs[slot] = make_int2(i, e0 + src);
+    slot = first + __popc(a0) + __popc(a1 & below);
+    if ((a1 >> lane & 1) && slot < pair_cap) pairs[slot] = make_int2(i, e0 + 32 + src);
   }
 }
 

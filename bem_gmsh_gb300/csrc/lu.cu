@@ -39,6 +39,13 @@ namespace bem {
 // (float)(a * 2^s).  Values whose result leaves the normal FP32 range (not
 // met by a scaled column other than for zeros) take the FP64 instructions
 // (df::scale_to_f32).
+//
+// V: loads in flight per thread and round.  HELD: one round covers the column
+// (N <= 512 V), which then stays in registers and is read once; V is chosen
+// by N, because with V fixed at 16 a column of 2049 rows issued 4 times its
+// instructions (25 us at N = 2049, now 14) and one of 8193 took a second
+// round for one row (189 us, now 138; its bytes take 120).
+template <int V, bool HELD>
 __global__ void __launch_bounds__(512) k_equilibrate(const double* __restrict__ A, int64_t lda, int N, int Npad,
                                                      double* __restrict__ cs, float* __restrict__ A32,
                                                      int64_t ld32) {
@@ -50,11 +57,8 @@ __global__ void __launch_bounds__(512) k_equilibrate(const double* __restrict__ 
   }
   const unsigned long long* col = (const unsigned long long*)(A + (size_t)j * lda);
   constexpr unsigned long long ABS = 0x7FFFFFFFFFFFFFFFull;
-  // 16 independent loads in flight per thread and round
-  constexpr int V = 16;
-  unsigned long long mx = 0;
+  unsigned long long v[V], mx = 0;
   for (int base = 0; base < N; base += V * 512) {
-    unsigned long long v[V];
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       const int i = base + q * 512 + t;
@@ -62,6 +66,7 @@ __global__ void __launch_bounds__(512) k_equilibrate(const double* __restrict__ 
     }
 #pragma unroll
     for (int q = 0; q < V; ++q) mx = max(mx, v[q] & ABS);
+    if constexpr (HELD) break;
   }
   for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   __shared__ unsigned long long sw[16];
@@ -80,17 +85,26 @@ __global__ void __launch_bounds__(512) k_equilibrate(const double* __restrict__ 
   }
   __syncthreads();
   const int sh = ssh;
-  for (int base = 0; base < Npad; base += V * 512) {
-    unsigned long long v[V];
+  if constexpr (HELD) {
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const int i = base + q * 512 + t;
-      v[q] = i < N ? col[i] : 0ull;
-    }
-#pragma unroll
-    for (int q = 0; q < V; ++q) {
-      const int i = base + q * 512 + t;
+      const int i = q * 512 + t;
       if (i < Npad) out[i] = df::scale_to_f32(__longlong_as_double((long long)v[q]), sh);
+    }
+    // padding rows beyond the round
+    for (int i = V * 512 + t; i < Npad; i += 512) out[i] = 0.f;
+  } else {
+    for (int base = 0; base < Npad; base += V * 512) {
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        const int i = base + q * 512 + t;
+        v[q] = i < N ? col[i] : 0ull;
+      }
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        const int i = base + q * 512 + t;
+        if (i < Npad) out[i] = df::scale_to_f32(__longlong_as_double((long long)v[q]), sh);
+      }
     }
   }
 }
@@ -505,9 +519,11 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 //   z_b = D_b (r_b - sum over the other solved blocks),  y_b = z_b - M_b y_prev
 // the sweep's dependent step is one 128 x 128 product; z_b is formed while
 // the previous block is still being solved.  One CTA per (block, side,
-// 64 x 64 quadrant), 4 x 4 outputs per thread.
-constexpr int CPL_LD = 64 + 4;
-constexpr int CPL_SMEM = (int)sizeof(float) * 2 * LU_NB * CPL_LD;
+// 64 x 64 quadrant), 4 x 4 outputs per thread; the operands come in 16-byte
+// asynchronous copies, all in flight at once (scalar loads took 16 of the
+// kernel's 22 us, which every solve pays before its first sweep).
+constexpr int CPL_LD = 64 + 4, CPL_LQ = LU_NB + 4;
+constexpr int CPL_SMEM = (int)sizeof(float) * (LU_NB * CPL_LD + 64 * CPL_LQ);
 
 __global__ void __launch_bounds__(256) k_lu_couplings(const float* __restrict__ A, int64_t ld, int K,
                                                       const float* __restrict__ Dinv, float* __restrict__ Mc) {
@@ -516,28 +532,39 @@ __global__ void __launch_bounds__(256) k_lu_couplings(const float* __restrict__ 
   if (side == 0 ? b == 0 : b == K - 1) return;
   const int qr = (quad & 1) * 64, qc = (quad >> 1) * 64;
   float* P = cs_;                   // D_b rows [qr, qr + 64): P[k][r]
-  float* Q = cs_ + LU_NB * CPL_LD;  // coupling block columns [qc, qc + 64): Q[k][c]
+  float* Q = cs_ + LU_NB * CPL_LD;  // coupling block columns [qc, qc + 64): Q[c][k]
   const float* Pg = Dinv + (size_t)b * 2 * LU_NB * LU_NB + (side ? LU_NB * LU_NB : 0);
   const int qb = side ? b + 1 : b - 1;
   const float* Qg = A + (size_t)b * LU_NB + (size_t)qb * LU_NB * ld;
-  for (int idx = t; idx < LU_NB * 64; idx += 256) {
-    const int r = idx & 63, k = idx >> 6;
-    P[k * CPL_LD + r] = Pg[qr + r + (size_t)k * LU_NB];  // D_b(qr + r, k), column-major
-    const int k2 = idx & (LU_NB - 1), c = idx >> 7;
-    Q[k2 * CPL_LD + c] = Qg[k2 + (size_t)(qc + c) * ld];  // block(k2, qc + c), coalesced reads
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int idx = t + 256 * i;
+    const int r = 4 * (idx & 15), k = idx >> 4;
+    cp_async16(&P[k * CPL_LD + r], Pg + qr + r + (size_t)k * LU_NB);  // D_b(qr + r, k), column-major
+    const int k2 = 4 * (idx & 31), c = idx >> 5;
+    cp_async16(&Q[c * CPL_LQ + k2], Qg + k2 + (size_t)(qc + c) * ld);  // block(k2, qc + c)
   }
+  cp_async_commit();
+  cp_async_wait<0>();
   __syncthreads();
   const int r0 = 4 * (t & 15), c0 = 4 * (t >> 4);
   float acc[4][4] = {};
-#pragma unroll 4
-  for (int k = 0; k < LU_NB; ++k) {
-    const float4 a = *(const float4*)&P[k * CPL_LD + r0];
-    const float4 q = *(const float4*)&Q[k * CPL_LD + c0];
-    const float av[4] = {a.x, a.y, a.z, a.w}, qv[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll 2
+  for (int k = 0; k < LU_NB; k += 4) {
+    float4 q[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j) q[j] = *(const float4*)&Q[(c0 + j) * CPL_LQ + k];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], qv[j], acc[i][j]);
+    for (int kk = 0; kk < 4; ++kk) {
+      const float4 a = *(const float4*)&P[(k + kk) * CPL_LD + r0];
+      const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float qv = kk == 0 ? q[j].x : kk == 1 ? q[j].y : kk == 2 ? q[j].z : q[j].w;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][j] = fmaf(av[i], qv, acc[i][j]);
+      }
+    }
   }
   float* Mo = Mc + (size_t)(2 * b + side) * LU_NB * LU_NB;
 #pragma unroll
@@ -996,7 +1023,16 @@ void lu_prepare(const double* A64, int64_t lda, int N, int Npad, double* cs, flo
                 cudaStream_t st) {
   KScope ks(st, KC_LU_PREP);
   count_launches(1);
-  k_equilibrate<<<Npad, 512, 0, st>>>(A64, lda, N, Npad, cs, A32, ld32);
+  const int v = (N + 511) / 512;
+  auto k = v <= 1   ? k_equilibrate<1, true>
+           : v <= 2 ? k_equilibrate<2, true>
+           : v <= 3 ? k_equilibrate<3, true>
+           : v <= 5 ? k_equilibrate<5, true>
+           : v <= 9 ? k_equilibrate<9, true>
+           : v <= 13 ? k_equilibrate<13, true>
+           : v <= 17 ? k_equilibrate<17, true>
+                     : k_equilibrate<16, false>;
+  k<<<Npad, 512, 0, st>>>(A64, lda, N, Npad, cs, A32, ld32);
 }
 
 // ---------------------------------------------------------------------------
@@ -1010,21 +1046,24 @@ void lu_prepare(const double* A64, int64_t lda, int N, int Npad, double* cs, flo
 //      32 rows below them (lane: row jb + 16 + 32 w + lane), so no barrier
 //      is needed between columns; the pivot rows reach the lanes two at a
 //      time through a double-buffered pair of rows in shared memory (every
-//      lane forms row c+1 after column c itself).  Warp 1 then
-//      inverts the unit-lower 16 x 16 block (one column per lane).
-//   B  block row of U: U[p, >p] = Linv_pp A[p, >p].  Column block p of L\U
-//      and its lower sub-block inverse are final and are written out; warp 4
-//      inverts the upper 16 x 16 block beside the next panel's factorization
-//      (its columns of S no longer change).
-//   C  the trailing update A22 -= L21 U12 on 4 x 4 register tiles.
-// 24 block barriers in all.  In the look-ahead LU the block first gets the
-// previous step's update of itself (the thin update leaves the block out):
-// A_kk -= L_{k,k-1} U_{k-1,k} with that step's tensor-core operands, TMA
-// loads and tcgen05 MMAs into TMEM (3xTF32) while the block loads, then one
-// TMEM read per thread (the same update on mma.sync took 12 of the kernel's
-// 45 us; as a separate one-tile launch it cost a launch on the chain).  73 KB
-// of shared memory (201 KB with the update's four operand stages) and the
-// whole register file (512 threads x 128): the kernel runs alone on an SM
+//      lane forms row c+1 after column c itself).
+//   B  block row of U: U[p, >p] = L_pp^{-1} A[p, >p], one thread per column,
+//      substitution in registers (400 cycles; four threads per column times
+//      the inverse of L_pp took 3000, bound by shared-memory loads).  Column
+//      block p of L\U is final and is written out; warps 4 and 5 invert its
+//      16 x 16 blocks beside the next panel's factorization (its columns of S
+//      no longer change).
+//   C  the trailing update A22 -= L21 U12: the next panel's columns by all
+//      warps on 4 x 2 tiles, the rest by warps 6-15 on 4 x 4 tiles beside the
+//      next panel's factorization (which it slows from 2450 to 3000 cycles).
+// 26.6 us a step of the look-ahead LU (with block barriers after every phase
+// and B through the inverse of L_pp 28 to 30), 4.5 of them set-up and the
+// block's own update: A_kk -= L_{k,k-1} U_{k-1,k} (the thin update leaves the
+// block out) with the previous step's tensor-core operands, TMA loads and
+// tcgen05 MMAs into TMEM (3xTF32) while the block loads, then one TMEM read
+// per thread (the same update on mma.sync took 12 us; as a separate one-tile
+// launch it cost a launch on the chain).  67 KB of shared memory (195 KB with
+// the update's four operand stages) and the whole register file (512 threads x 128): the kernel runs alone on an SM
 // (capped at 64 registers to share an SM with a bulk-update tile it measured
 // 40 % slower).  A and ld must allow 16-byte accesses (ld % 4 == 0, 16-byte
 // aligned A).
@@ -1032,9 +1071,8 @@ void lu_prepare(const double* A64, int64_t lda, int N, int Npad, double* cs, flo
 constexpr int DB = LU_SB;       // panel width
 constexpr int TLD = LU_NB + 4;  // shared leading dimension
 // shared floats of the diagonal kernel: L\U, four warps' double-buffered
-// pairs of pivot rows, the 16 x 16 scratch of the lower inverse, the two
-// sub-block inverses
-constexpr int DIAG_SMEM = (int)sizeof(float) * (LU_NB * TLD + 4 * 4 * DB + 16 * 20 + 4 * DB * DB);
+// pairs of pivot rows
+constexpr int DIAG_SMEM = (int)sizeof(float) * (LU_NB * TLD + 4 * 4 * DB);
 // with the block's own update: two operand stages of the tensor-core update
 // (1024-byte aligned), their barriers and the TMEM address
 constexpr int DIAG_PRE_STAGES = 4;
@@ -1099,8 +1137,6 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
   extern __shared__ __align__(1024) float dsm[];
   float* S = dsm;                       // A -> L\U
   float* rowbuf = S + LU_NB * TLD;      // [warp 0-3][parity][2 rows][16]
-  float* Ls = rowbuf + 4 * 4 * DB;      // 16 x 16 unit lower, column-major, ld 20
-  float* LiP = Ls + 16 * 20;            // [parity][Linv_pp, Uinv_pp], column-major, ld 16
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const size_t off = (size_t)k * LU_NB;
   float* Ab = A + off + off * ld;
@@ -1139,6 +1175,9 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     tmem = *s_tmem;
+    // launched ahead of the end of the kernel before it (the panels): nothing
+    // of theirs is read above this line
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int NCH = LU_NB / BK;
     const uint32_t full0 = bars, empty0 = bars + 8 * DIAG_PRE_STAGES, done = bars + 8 * 2 * DIAG_PRE_STAGES;
     if (warp == 0 && lane == 0) {
@@ -1224,16 +1263,11 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
   }
   int bad = 0;
   // phase A of panel jb (warps 0-3): factor rows jb.. of columns jb..jb+15,
-  // warp 1 then inverts the unit-lower 16 x 16 block into Li
-  auto factor_panel = [&](int jb, float* Li) {
-    float PT[DB], PB[DB];
+  // given in registers (PT: row jb + lane, lanes < 16; PB: row jb + 16 + 32
+  // warp + lane), and write them to S
+  auto factor_panel = [&](int jb, float (&PT)[DB], float (&PB)[DB]) {
     const int rb = jb + DB + 32 * warp + lane;
     const bool tv = lane < DB, bv = rb < LU_NB;
-#pragma unroll
-    for (int c = 0; c < DB; ++c) {
-      PT[c] = tv ? S[(jb + c) * TLD + jb + lane] : 0.f;
-      PB[c] = bv ? S[(jb + c) * TLD + rb] : 0.f;
-    }
     // two columns per step: pivot rows c and c+1 go out together, and every
     // lane forms row c+1 after column c itself (the same operations lane c+1
     // performs on its own copy), so one broadcast serves two columns; the
@@ -1299,34 +1333,40 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
     if (warp == 0 && tv) {
 #pragma unroll
       for (int c = 0; c < DB; ++c) S[(jb + c) * TLD + jb + lane] = PT[c];
-    } else if (warp == 1) {
-      // inverse of the unit-lower 16 x 16 block, lane c < 16 solving for
-      // column c by column-oriented forward substitution
-      if (tv) {
+    }
+  };
+  auto load_panel = [&](int jb, float (&PT)[DB], float (&PB)[DB]) {
+    const int rt = jb + (lane & (DB - 1)), rb = min(jb + DB + 32 * warp + lane, LU_NB - 1);
 #pragma unroll
-        for (int q = 0; q < DB; ++q) Ls[q * 20 + lane] = PT[q];
-      }
-      __syncwarp();
-      float x[DB];
+    for (int c = 0; c < DB; ++c) {
+      PT[c] = S[(jb + c) * TLD + rt];
+      PB[c] = S[(jb + c) * TLD + rb];
+    }
+  };
+  // trailing update of the 16 columns after panel jb, 4 x 2 tiles by all
+  // threads: nothing else runs meanwhile, because its shared-memory loads are
+  // its time (the next panel's factorization waits for it)
+  auto next_columns = [&](int jb) {
+    const int nr = (LU_NB - jb - DB) / 4;
+    const float* Pb = S + jb * TLD + jb + DB;
+    float* Cb = S + (jb + DB) * TLD + jb + DB;
+    const int r0 = 4 * (t % nr), cc = 2 * (t / nr);
+    if (cc < DB) {
+      float acc[4][2] = {};
+      tile_mm<2>(Pb, S + (jb + DB) * TLD + jb, r0, cc, 0, DB, acc);
 #pragma unroll
-      for (int i = 0; i < DB; ++i) x[i] = (i == lane) ? 1.f : 0.f;
-#pragma unroll
-      for (int q = 0; q < DB - 1; ++q) {
-#pragma unroll
-        for (int i = q + 1; i < DB; ++i) x[i] = fmaf(-Ls[q * 20 + i], x[q], x[i]);
-      }
-      if (tv) {
-#pragma unroll
-        for (int i4 = 0; i4 < DB; i4 += 4)
-          *(float4*)&Li[lane * DB + i4] = make_float4(x[i4], x[i4 + 1], x[i4 + 2], x[i4 + 3]);
+      for (int j = 0; j < 2; ++j) {
+        float4 cv = *(float4*)&Cb[(cc + j) * TLD + r0];
+        cv.x -= acc[0][j]; cv.y -= acc[1][j]; cv.z -= acc[2][j]; cv.w -= acc[3][j];
+        *(float4*)&Cb[(cc + j) * TLD + r0] = cv;
       }
     }
   };
   // trailing update S[r, c] -= L21[r, :] U12[:, c] of panel jb for rows
-  // [jb+16, 128) and the columns [c0, c1) (multiples of 4), by `nth`
-  // threads numbered from `tid`
-  auto trailing = [&](int jb, int c0, int c1, int tid, int nth) {
-    const int nr = (LU_NB - jb - DB) / 4, ncl = (c1 - c0) / 4;
+  // [jb+16, 128) and the columns [c0, 128) on 4 x 4 tiles, by `nth` threads
+  // numbered from `tid`
+  auto trailing = [&](int jb, int c0, int tid, int nth) {
+    const int nr = (LU_NB - jb - DB) / 4, ncl = (LU_NB - c0) / 4;
     const float* Pb = S + jb * TLD + jb + DB;  // L21(r, q)
     const float* Qb = S + c0 * TLD + jb;       // U12(q, c)
     float* Cb = S + c0 * TLD + jb + DB;
@@ -1343,79 +1383,92 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
     }
   };
   // The phases are pipelined: after the block row of U of panel p, warps
-  // 0-3 update only panel p+1's columns, meet at a 128-thread named barrier
-  // and factor panel p+1 while warps 4-15 store panel p and apply the rest
-  // of its trailing update.  The 16 x 16 inverses are double-buffered by
-  // panel parity (panel p's are stored while panel p+1's are formed).
-  if (warp < 4) factor_panel(0, LiP);
-  __syncthreads();
-  for (int p = 0; p < LU_NB / DB; ++p) {
+  // 0-3 update only panel p+1's columns and factor them while warps 4-15
+  // store panel p, invert its 16 x 16 blocks (warps 4 and 5) and apply the
+  // rest of its trailing update.
+  // 16 x 16 sub-block inverses, lane c < 16 solving for column c: unit-lower
+  // by column-oriented forward substitution, upper by back substitution;
+  // inverse(i, c) = out[c * 16 + i]
+  auto invert = [&](int p, bool upper) {
+    const float* Sp = S + p * DB * TLD + p * DB;
+    float x[DB];
+#pragma unroll
+    for (int i = 0; i < DB; ++i) x[i] = (i == lane) ? 1.f : 0.f;
+    if (!upper) {
+#pragma unroll
+      for (int q = 0; q < DB - 1; ++q)
+#pragma unroll
+        for (int i = q + 1; i < DB; ++i) x[i] = fmaf(-Sp[q * TLD + i], x[q], x[i]);
+    } else {
+#pragma unroll
+      for (int q = DB - 1; q >= 0; --q) {
+        x[q] *= rcp_nr(Sp[q * TLD + q]);
+#pragma unroll
+        for (int i = 0; i < q; ++i) x[i] = fmaf(-Sp[q * TLD + i], x[q], x[i]);
+      }
+    }
+    if (lane < DB) {
+      float* out = SIk + p * 2 * DB * DB + (upper ? DB * DB : 0) + lane * DB;
+#pragma unroll
+      for (int i4 = 0; i4 < DB; i4 += 4)
+        *(float4*)&out[i4] = make_float4(x[i4], x[i4 + 1], x[i4 + 2], x[i4 + 3]);
+    }
+  };
+  for (int p = -1; p < LU_NB / DB; ++p) {
     const int jb = p * DB;
-    float* Li = LiP + (p & 1) * 2 * DB * DB;
-    // ---- B: block row of U, U[p, >p] = Linv_pp A[p, >p]: four threads
-    // per column (lanes 4m .. 4m+3 of one warp), rows 4 (t % 4) .. +3 each;
-    // the column is read whole before any of its four threads writes ----
-    {
-      const int c = jb + DB + (t >> 2), i0 = 4 * (t & 3);
-      const bool on = c < LU_NB;
-      float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
-      if (on) {
+    if (p >= 0) {
+      // ---- B: block row of U, U[p, >p] = L_pp^{-1} A[p, >p]: one thread per
+      // column, forward substitution in registers, L from broadcast loads ----
+      const int c = jb + DB + t;
+      if (c < LU_NB) {
         float v[DB];
 #pragma unroll
         for (int q4 = 0; q4 < DB; q4 += 4) {
-          const float4 a = *(const float4*)&S[c * TLD + jb + q4];
-          v[q4] = a.x; v[q4 + 1] = a.y; v[q4 + 2] = a.z; v[q4 + 3] = a.w;
+          const float4 x = *(const float4*)&S[c * TLD + jb + q4];
+          v[q4] = x.x; v[q4 + 1] = x.y; v[q4 + 2] = x.z; v[q4 + 3] = x.w;
         }
 #pragma unroll
-        for (int q = 0; q < DB; ++q) {
-          const float4 l = *(const float4*)&Li[q * DB + i0];
-          o0 = fmaf(l.x, v[q], o0);
-          o1 = fmaf(l.y, v[q], o1);
-          o2 = fmaf(l.z, v[q], o2);
-          o3 = fmaf(l.w, v[q], o3);
+        for (int q = 0; q < DB - 1; ++q) {
+          float l[DB];
+#pragma unroll
+          for (int q4 = (q + 1) / 4 * 4; q4 < DB; q4 += 4) {
+            const float4 x = *(const float4*)&S[(jb + q) * TLD + jb + q4];
+            l[q4] = x.x; l[q4 + 1] = x.y; l[q4 + 2] = x.z; l[q4 + 3] = x.w;
+          }
+#pragma unroll
+          for (int i = q + 1; i < DB; ++i) v[i] = fmaf(-l[i], v[q], v[i]);
         }
+#pragma unroll
+        for (int q4 = 0; q4 < DB; q4 += 4)
+          *(float4*)&S[c * TLD + jb + q4] = make_float4(v[q4], v[q4 + 1], v[q4 + 2], v[q4 + 3]);
       }
-      __syncwarp();
-      if (on) *(float4*)&S[c * TLD + jb + i0] = make_float4(o0, o1, o2, o3);
+      __syncthreads();
+      // ---- C1: the next panel's columns ----
+      if (p + 1 < LU_NB / DB) next_columns(jb);
+      __syncthreads();
     }
-    __syncthreads();
     if (warp < 4) {
       if (p + 1 < LU_NB / DB) {
-        // ---- C1: the next panel's columns; then A of panel p+1 ----
-        trailing(jb, jb + DB, jb + 2 * DB, t, 128);
+        // ---- A of the next panel ----
+        float PT[DB], PB[DB];
+        load_panel(jb + DB, PT, PB);
+        // every warp has read the pivot rows before one writes them back
         asm volatile("bar.sync 1, 128;" ::: "memory");
-        factor_panel(jb + DB, LiP + ((p + 1) & 1) * 2 * DB * DB);
+        factor_panel(jb + DB, PT, PB);
       }
-    } else {
-      // ---- store column block p of L\U and its lower inverse; the upper
-      // inverse (warp 4, beside the next panel's factorization); C2 ----
+    } else if (p >= 0) {
+      // ---- store column block p of L\U, its inverses; C2 ----
       if (warp == 4) {
-        // inverse of the upper 16 x 16 block, lane c < 16 solving for column
-        // c by column-oriented back substitution; Uinv(i, c) = Ui[c * 16 + i]
-        float x[DB];
-#pragma unroll
-        for (int i = 0; i < DB; ++i) x[i] = (i == lane) ? 1.f : 0.f;
-#pragma unroll
-        for (int q = DB - 1; q >= 0; --q) {
-          const float* uc = S + (jb + q) * TLD + jb;
-          x[q] *= rcp_nr(uc[q]);
-#pragma unroll
-          for (int i = 0; i < q; ++i) x[i] = fmaf(-uc[i], x[q], x[i]);
-        }
-        if (lane < DB) {
-          float* Ug = SIk + p * 2 * DB * DB + DB * DB;
-#pragma unroll
-          for (int i4 = 0; i4 < DB; i4 += 4)
-            *(float4*)&Ug[lane * DB + i4] = make_float4(x[i4], x[i4 + 1], x[i4 + 2], x[i4 + 3]);
-        }
+        invert(p, true);
+      } else if (warp == 5) {
+        invert(p, false);
       } else {
-        for (int idx = t - 160; idx < DB * 32; idx += 352) {
+        for (int idx = t - 192; idx < DB * 32; idx += 320) {
           const int cs = jb + (idx >> 5), r4 = 4 * (idx & 31);
           *(float4*)(Ab + r4 + (size_t)cs * ld) = *(const float4*)&S[cs * TLD + r4];
         }
-        for (int idx = t - 160; idx < DB * DB; idx += 352) SIk[p * 2 * DB * DB + idx] = Li[idx];
+        if (jb + 2 * DB < LU_NB) trailing(jb, jb + 2 * DB, t - 192, 320);
       }
-      if (jb + 2 * DB < LU_NB) trailing(jb, jb + 2 * DB, LU_NB, t - 128, 384);
     }
     __syncthreads();
   }
@@ -1474,6 +1527,8 @@ __global__ void __launch_bounds__(256) k_panels(const float* __restrict__ Dk, in
   float* Xp = Si + LU_SI / 2;        // the current sub-block X_p (16 x 32)
   const int t = threadIdx.x;
   const int side = blockIdx.y;
+  // the next diagonal block may take its SM and set up meanwhile
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const int idx = t + 256 * i, r4 = 4 * (idx & 31), kx = idx >> 5;
@@ -1743,9 +1798,10 @@ static float* sub_inverses(float* Dinv, int Npad, int k) {
 }
 
 // diagonal block k; with P (the plan of step k-1), the block first gets
-// that step's update on the tensor cores
+// that step's update on the tensor cores; early: the launch is ordered before
+// its predecessor in the stream ends (programmatic dependent launch)
 static void diag_block(float* A, int64_t ld, int Npad, float* Dinv, int* info, int k, cudaStream_t st,
-                       const TcPlan* P = nullptr) {
+                       const TcPlan* P = nullptr, bool early = false) {
   KScope kd(st, KC_LU_DIAG);
   static const CUtensorMap none{};
   DiagPre pre{0, 0, 0};
@@ -1757,8 +1813,17 @@ static void diag_block(float* A, int64_t ld, int Npad, float* Dinv, int* info, i
     m[2] = (const CUtensorMap*)P->mB128;
     m[3] = (const CUtensorMap*)P->mBlo128;
   }
-  k_diag_lu<<<1, 512, pre.on ? DIAG_SMEM_PRE : DIAG_SMEM, st>>>(A, ld, k, sub_inverses(Dinv, Npad, 0), info, *m[0],
-                                                              *m[1], *m[2], *m[3], pre);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = pre.on ? DIAG_SMEM_PRE : DIAG_SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_diag_lu, A, ld, k, sub_inverses(Dinv, Npad, 0), info, *m[0], *m[1], *m[2], *m[3], pre);
   count_launches(1);
 }
 
@@ -1822,6 +1887,8 @@ int lu_factor(float* A, int64_t ld, int Npad, float* Dinv, int* info, int x3, cu
   return (int)cudaGetLastError();
 }
 
+constexpr int LU_EARLY = 3072;  // see below
+
 // Lookahead-1 schedule on three streams.  `la` (the critical path) factors
 // diagonal block k+1 after applying step k's update to the block itself
 // (inside the diagonal kernel), then its panels; `tl` meanwhile applies the rest of step k's thin update (block
@@ -1831,6 +1898,15 @@ int lu_factor(float* A, int64_t ld, int Npad, float* Dinv, int* info, int x3, cu
 // of all diagonal blocks in one launch.  evP[k]: panels of step k ready;
 // evT[k]: bulk update of step k done; evR[k]: thin update of step k done.
 // tc[2]: plans with separate lo/transposed buffers for even and odd steps.
+//
+// Once at most LU_EARLY columns remain, the bulk update (14 us at 2048) is
+// shorter than the diagonal block (26 us) it runs beside, so `la` waits for
+// it before the panels instead of before the next diagonal block.  With no
+// wait between panels and diagonal block, the latter is launched as the
+// panels' programmatic dependent: its set-up (4.8k cycles: TMEM, barriers,
+// the first instruction lines) and launch overlap the panels.  n = 1024 /
+// 2048 / 4096: 0.344 / 0.691 / 1.437 ms without, 0.309 / 0.622 / 1.386 with
+// (limit 2048: 1.396, 4096: 1.41; at 8192 the bulk update bounds both).
 int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, cudaStream_t st,
                         cudaStream_t la, cudaEvent_t fork, cudaEvent_t* evP, cudaEvent_t* evT,
                         cudaStream_t tl, cudaEvent_t* evR, const TcPlan* tc, int* err, int* ctr) {
@@ -1845,20 +1921,16 @@ int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, 
   for (int k = 0; k + 1 < K; ++k) {
     const int rem = Npad - (k + 1) * LU_NB;
     const TcPlan& P = tc[k & 1];
-    if (k >= 1) cudaStreamWaitEvent(la, evT[k - 1], 0);
+    const bool early = rem <= LU_EARLY, next_early = rem - LU_NB <= LU_EARLY;
+    if (k >= 1 && !early) cudaStreamWaitEvent(la, evT[k - 1], 0);
     // thin update of step k without the diagonal block: needs panels k
     // (evP[k]) and the bulk update of step k-1
     cudaStreamWaitEvent(tl, evP[k], 0);
     if (k >= 1) cudaStreamWaitEvent(tl, evT[k - 1], 0);
     thin_part(A, ld, k, rem, LU_NB, rem - LU_NB, true, tl);
     cudaEventRecord(evR[k], tl);
-    {
-      KScope crit(la, KC_LU_CRIT);
-      diag_block(A, ld, Npad, Dinv, info, k + 1, la, &P);
-      cudaStreamWaitEvent(la, evR[k], 0);
-      panels(A, ld, Npad, Dinv, k + 1, la, &tc[(k + 1) & 1]);
-    }
-    cudaEventRecord(evP[k + 1], la);
+    KScope crit(la, KC_LU_CRIT);
+    diag_block(A, ld, Npad, Dinv, info, k + 1, la, &P, early);
     cudaStreamWaitEvent(st, evP[k], 0);
     if (rem > LU_NB) {
       KScope trail(st, KC_LU_TRAIL);
@@ -1867,6 +1939,10 @@ int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, 
       if (e) return e;
     }
     cudaEventRecord(evT[k], st);
+    cudaStreamWaitEvent(la, evR[k], 0);
+    if (next_early) cudaStreamWaitEvent(la, evT[k], 0);
+    panels(A, ld, Npad, Dinv, k + 1, la, &tc[(k + 1) & 1]);
+    cudaEventRecord(evP[k + 1], la);
   }
   cudaStreamWaitEvent(st, evP[K - 1], 0);
   // all block inverses in one launch once the factorization is done
