@@ -892,12 +892,20 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
   return s;
 }
 
-// s.h[0..m) = the cluster's sums of the per-warp sums in s.warp
-__device__ __forceinline__ void gs_reduce(GsShared& s, int m, int buf) {
+// Distributed shared memory may be touched only once every CTA of the cluster
+// runs: all threads arrive at the kernel's start and wait before the first
+// remote write (the work in between hides the barrier).
+__device__ __forceinline__ void gs_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void gs_started() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
+// s.h[0..m) = the cluster's sums of the per-warp sums in s.warp; first: the
+// kernel's first call
+__device__ __forceinline__ void gs_reduce(GsShared& s, int m, int buf, bool first) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int t = threadIdx.x, nc = (int)cl.num_blocks();
   __syncthreads();
+  if (first) gs_started();
   for (int v = t; v < m * nc; v += GS_THREADS) {
     const int q = v % m, to = v / m;
     double x = 0.0;
@@ -923,6 +931,7 @@ __global__ void __launch_bounds__(GS_THREADS)
     k_gram_schmidt(const double* __restrict__ V, int64_t ldv, int N, int m, double* w, double* __restrict__ vn,
                    double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo) {
   __shared__ GsShared s;
+  gs_arrive();
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int chunk = (N + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
   for (int pass = 0; pass < 2; ++pass) {
@@ -942,7 +951,7 @@ __global__ void __launch_bounds__(GS_THREADS)
       const double v = warp_sum8(acc, lane);
       if ((lane & 3) == 0) s.warp[warp][q0 + (lane >> 2)] = v;
     }
-    gs_reduce(s, cnt, pass);
+    gs_reduce(s, cnt, pass, pass == 0);
     if (blockIdx.x == 0 && t < m) host[32 * pass + t] = s.h[t];
   }
   double n2 = s.h[m];
@@ -966,13 +975,14 @@ __global__ void __launch_bounds__(GS_THREADS)
                 double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo,
                 const int* __restrict__ cnt, int* __restrict__ hcnt) {
   __shared__ GsShared s;
+  gs_arrive();
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int chunk = (N + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * chunk, i1 = min(N, i0 + chunk);
   double acc = 0.0;
   for (int i = i0 + t; i < i1; i += GS_THREADS) acc = fma(r[i], r[i], acc);
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) s.warp[warp][0] = acc;
-  gs_reduce(s, 1, 0);
+  gs_reduce(s, 1, 0, true);
   const double n2 = s.h[0], sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
   for (int i = i0 + t; i < i1; i += GS_THREADS) {
     v[i] = r[i] * sc;
