@@ -1488,11 +1488,15 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
   }
 }
 
-constexpr int PW = 32;  // slice width
-constexpr int PXLD = PW + 4;
-// shared floats of the panel kernel: the factored block, the slice, one
-// side's eight 16 x 16 sub-block inverses
-constexpr int PANEL_SMEM = (int)sizeof(float) * (LU_NB * TLD + LU_NB * PXLD + LU_SI / 2 + DB * PW);
+// shared floats of the panel kernel for slices of W vectors: the 28 blocks of
+// one triangle and the 8 inverses (16 x 16, leading dimension 20: four lanes'
+// 16-byte rows on different banks), the exchange rows
+constexpr int PBL = 20;
+constexpr int PBS = DB * PBL;
+constexpr int PANEL_BLOCKS = 28;
+constexpr int panel_smem(int W) {
+  return (int)sizeof(float) * ((PANEL_BLOCKS + LU_NB / DB) * PBS + W * DB);
+}
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -1505,11 +1509,17 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Panels of diagonal block k by blocked triangular solves with its factored
 // block Dk (L unit lower and U upper, leading dimension ldk) and its 16 x 16
 // sub-block inverses SIk (from k_diag_lu):
-//   blockIdx.y == 0: columns [32 x, 32 x + 32) of B (128 rows): X = L^{-1} B.
+//   blockIdx.y == 0: columns [W x, W x + W) of B (128 rows): X = L^{-1} B.
 //     For each sub-block p: X_p = Linv_pp B_p, then B_q -= L_qp X_p (q > p).
-//   blockIdx.y == 1: rows [32 x, 32 x + 32) of Ap (128 columns): X = Ap U^{-1}.
+//   blockIdx.y == 1: rows [W x, W x + W) of Ap (128 columns): X = Ap U^{-1}.
 //     For each sub-block p: X_p = B_p Uinv_pp, then B_q -= X_p U_pq (q > p).
-// ident: the slices start as the corresponding part of the identity (not
+// Both are W vectors of 128 entries.  A half-warp keeps four vectors in
+// registers (lane i: entries 16 s + i), so X_p passes between its lanes only
+// and there is no block barrier after the load; an entry of L or U read from
+// shared memory serves four vectors.  The registers move up one sub-block per
+// step, which keeps the loop rolled: a kernel this short pays for every
+// instruction line it fetches.
+// ident: the vectors start as the corresponding part of the identity (not
 // read), which gives the full inverses L^{-1} and U^{-1} of the block for the
 // triangular sweeps.  B and Ap have leading dimension ld.  blockIdx.z
 // offsets Dk, SIk and B/Ap by z times zsD, zsSI and zsX (all diagonal blocks
@@ -1521,187 +1531,137 @@ __device__ __forceinline__ float tf32_low(float x) {
   return x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
 }
 
-__global__ void __launch_bounds__(256) k_panels(const float* __restrict__ Dk, int64_t ldk,
-                                                const float* __restrict__ SIk, float* B, float* Ap, int64_t ld,
-                                                int ident, int64_t zsD, int64_t zsSI, int64_t zsX,
-                                                float* __restrict__ Lt, float* __restrict__ Ltlo,
-                                                float* __restrict__ Ulo) {
+// c -= M x (SUB) or c = M x for one 16 x 16 block and this lane's entry i of
+// four vectors; M(i, q) = m[q * PBL + i] (side 0) or m[i * PBL + q] (side 1)
+template <int SIDE, bool SUB>
+__device__ __forceinline__ void panel_mm(const float* m, int i, const float4 (&x)[DB], float (&c)[4]) {
+  float l[DB];
+  if constexpr (SIDE == 0) {
+#pragma unroll
+    for (int q = 0; q < DB; ++q) l[q] = m[q * PBL + i];
+  } else {
+#pragma unroll
+    for (int q = 0; q < DB; q += 4) {
+      const float4 f = *(const float4*)&m[i * PBL + q];
+      l[q] = f.x; l[q + 1] = f.y; l[q + 2] = f.z; l[q + 3] = f.w;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < DB; ++q) {
+    const float f = SUB ? -l[q] : l[q];
+    c[0] = fmaf(f, x[q].x, c[0]);
+    c[1] = fmaf(f, x[q].y, c[1]);
+    c[2] = fmaf(f, x[q].z, c[2]);
+    c[3] = fmaf(f, x[q].w, c[3]);
+  }
+}
+
+// offset of block (row-block r, column-block c) of the strict triangle
+// (side 0: r > c; side 1: r < c) in the packed list, by p = min(r, c) and
+// s = |r - c| = 1 .. 7 - p
+__device__ __forceinline__ int panel_block(int p, int s) { return (p * (15 - p) / 2 + s - 1) * PBS; }
+
+template <int SIDE, int W>
+__device__ __forceinline__ void panel_slice(const float* Ms, const float* Si, float* xb, float* X0, int64_t ld,
+                                            bool ident, int x0, float* __restrict__ Lt, float* __restrict__ Ltlo,
+                                            float* __restrict__ Ulo) {
+  constexpr int NS = LU_NB / DB;
+  const int t = threadIdx.x, lane = t & 31, i = lane & 15, v0 = 8 * (t >> 5) + 4 * (lane >> 4);
+  float x[NS][4];
+  // side 0: entry r of vector c at X0[r + c * ld]; side 1: X0[c + r * ld]
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const int r = DB * s + i;
+    if (ident) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[s][j] = r == x0 + v0 + j ? 1.f : 0.f;
+    } else if constexpr (SIDE == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[s][j] = __ldcg(X0 + r + (size_t)(v0 + j) * ld);
+    } else {
+      const float4 f = __ldcg((const float4*)(X0 + v0 + (size_t)r * ld));
+      x[s][0] = f.x; x[s][1] = f.y; x[s][2] = f.z; x[s][3] = f.w;
+    }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  float4* mine = (float4*)xb + (t >> 5) * 32 + (lane >> 4);  // row q of this half-warp: mine[2 q]
+#pragma unroll 1
+  for (int p = 0; p < NS; ++p) {
+    float4 b[DB];
+    __syncwarp();
+    mine[2 * i] = make_float4(x[0][0], x[0][1], x[0][2], x[0][3]);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < DB; ++q) b[q] = mine[2 * q];
+    float X[4] = {0.f, 0.f, 0.f, 0.f};
+    panel_mm<SIDE, false>(Si + p * PBS, i, b, X);
+    __syncwarp();
+    mine[2 * i] = make_float4(X[0], X[1], X[2], X[3]);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < DB; ++q) b[q] = mine[2 * q];
+#pragma unroll
+    for (int s = 1; s < NS; ++s) {
+      if (p + s < NS) panel_mm<SIDE, true>(Ms + panel_block(p, s), i, b, x[s]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[s - 1][j] = x[s][j];
+    }
+    const int r = DB * p + i;
+    if constexpr (SIDE == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        X0[r + (size_t)(v0 + j) * ld] = X[j];
+        if (Ulo) Ulo[(size_t)(x0 + v0 + j) * LU_NB + r] = tf32_low(X[j]);
+      }
+    } else {
+      *(float4*)(X0 + v0 + (size_t)r * ld) = make_float4(X[0], X[1], X[2], X[3]);
+      if (Lt) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          Lt[(size_t)(x0 + v0 + j) * LU_NB + r] = X[j];
+          Ltlo[(size_t)(x0 + v0 + j) * LU_NB + r] = tf32_low(X[j]);
+        }
+      }
+    }
+  }
+}
+
+template <int W>
+__global__ void __launch_bounds__(4 * W) k_panels(const float* __restrict__ Dk, int64_t ldk,
+                                                  const float* __restrict__ SIk, float* B, float* Ap, int64_t ld,
+                                                  int ident, int64_t zsD, int64_t zsSI, int64_t zsX,
+                                                  float* __restrict__ Lt, float* __restrict__ Ltlo,
+                                                  float* __restrict__ Ulo) {
   extern __shared__ __align__(16) float psm[];
+  // the next diagonal block may take its SM and set up meanwhile
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   Dk += blockIdx.z * zsD;
   SIk += blockIdx.z * zsSI;
   B += blockIdx.z * zsX;
   Ap += blockIdx.z * zsX;
-  float* Ms = psm;                   // factored block, column-major, ld TLD
-  float* Xs = psm + LU_NB * TLD;     // the slice
-  float* Si = Xs + LU_NB * PXLD;     // [p][16 x 16], column-major
-  float* Xp = Si + LU_SI / 2;        // the current sub-block X_p (16 x 32)
-  const int t = threadIdx.x;
-  const int side = blockIdx.y;
-  // the next diagonal block may take its SM and set up meanwhile
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int idx = t + 256 * i, r4 = 4 * (idx & 31), kx = idx >> 5;
-    cp_async16(&Ms[kx * TLD + r4], Dk + r4 + (size_t)kx * ldk);
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int idx = t + 256 * i, p = idx >> 6, e4 = 4 * (idx & 63);
-    cp_async16(&Si[p * DB * DB + e4], SIk + p * 2 * DB * DB + side * DB * DB + e4);
-  }
-  if (side == 0) {
-    // slice [col][row], ld TLD: Xs[c * TLD + r]
-    float* Bb = B + (size_t)blockIdx.x * PW * ld;
-    if (ident) {
-      for (int idx = t; idx < PW * LU_NB; idx += 256) {
-        const int r = idx & (LU_NB - 1), c = idx >> 7;
-        Xs[c * TLD + r] = (r == (int)blockIdx.x * PW + c) ? 1.f : 0.f;
-      }
+  float* Ms = psm;                         // the triangle's blocks, [column][row]
+  float* Si = Ms + PANEL_BLOCKS * PBS;     // inverses
+  float* Xb = Si + LU_NB / DB * PBS;
+  const int t = threadIdx.x, side = blockIdx.y, x0 = blockIdx.x * W;
+  // 16-byte quarter columns: 64 per block
+  for (int idx = t; idx < (PANEL_BLOCKS + LU_NB / DB) * 64; idx += 4 * W) {
+    const int blk = idx >> 6, c = (idx >> 2) & 15, r4 = 4 * (idx & 3);
+    if (blk < PANEL_BLOCKS) {
+      int p = 0, s = blk;  // blk = p (15 - p) / 2 + s - 1
+      while (s >= 7 - p) s -= 7 - p, ++p;
+      const int lo = DB * p, hi = DB * (p + s + 1);
+      const int row = side ? lo : hi, col = side ? hi : lo;
+      cp_async16(&Ms[blk * PBS + c * PBL + r4], Dk + row + r4 + (size_t)(col + c) * ldk);
     } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int idx = t + 256 * i, k4 = 4 * (idx & 31), c = idx >> 5;
-        cp_async16(&Xs[c * TLD + k4], Bb + k4 + (size_t)c * ld);
-      }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    for (int p = 0; p < LU_NB / DB; ++p) {
-      const int jb = p * DB;
-      const float* Li = Si + p * DB * DB;  // Linv_pp(i, q) = Li[q * 16 + i]
-      {
-        // X_p = Linv_pp B_p into Xp[c][16]: thread -> column t / 8, rows
-        // 2 (t % 8) .. +1
-        const int c = t >> 3, r2 = 2 * (t & 7);
-        float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-        for (int q = 0; q < DB; ++q) {
-          const float b = Xs[c * TLD + jb + q];
-          o0 = fmaf(Li[q * DB + r2], b, o0);
-          o1 = fmaf(Li[q * DB + r2 + 1], b, o1);
-        }
-        Xp[c * DB + r2] = o0;
-        Xp[c * DB + r2 + 1] = o1;
-      }
-      __syncthreads();
-      // rows jb.. of the slice take X_p (two values per thread)
-      {
-        const int c = t >> 3, r2 = 2 * (t & 7);
-        Xs[c * TLD + jb + r2] = Xp[c * DB + r2];
-        Xs[c * TLD + jb + r2 + 1] = Xp[c * DB + r2 + 1];
-      }
-      // B_q -= L_qp X_p: thread -> row jb + 16 + (t % 128), 16 columns
-      const int i = jb + DB + (t & (LU_NB - 1));
-      if (i < LU_NB) {
-        float l[DB];
-#pragma unroll
-        for (int q = 0; q < DB; ++q) l[q] = Ms[(jb + q) * TLD + i];
-        const int cb = (t >> 7) * (PW / 2);
-#pragma unroll 4
-        for (int cc = 0; cc < PW / 2; ++cc) {
-          const int c = cb + cc;
-          const float* xp = Xp + c * DB;
-          float acc = Xs[c * TLD + i];
-#pragma unroll
-          for (int q4 = 0; q4 < DB; q4 += 4) {
-            const float4 x = *(const float4*)&xp[q4];
-            acc = fmaf(-l[q4], x.x, acc);
-            acc = fmaf(-l[q4 + 1], x.y, acc);
-            acc = fmaf(-l[q4 + 2], x.z, acc);
-            acc = fmaf(-l[q4 + 3], x.w, acc);
-          }
-          Xs[c * TLD + i] = acc;
-        }
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int idx = t + 256 * i, r4 = 4 * (idx & 31), c = idx >> 5;
-      const float4 v = *(const float4*)&Xs[c * TLD + r4];
-      *(float4*)&Bb[r4 + (size_t)c * ld] = v;
-      if (Ulo)
-        *(float4*)&Ulo[(size_t)(blockIdx.x * PW + c) * LU_NB + r4] =
-            make_float4(tf32_low(v.x), tf32_low(v.y), tf32_low(v.z), tf32_low(v.w));
-    }
-  } else {
-    // slice [col][row], ld PXLD: Xs[c * PXLD + r], 32 rows
-    float* Ab = Ap + (size_t)blockIdx.x * PW;
-    if (ident) {
-      for (int idx = t; idx < PW * LU_NB; idx += 256) {
-        const int r = idx & (PW - 1), c = idx >> 5;
-        Xs[c * PXLD + r] = ((int)blockIdx.x * PW + r == c) ? 1.f : 0.f;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int idx = t + 256 * i, r4 = 4 * (idx & 7), kx = idx >> 3;
-        cp_async16(&Xs[kx * PXLD + r4], Ab + r4 + (size_t)kx * ld);
-      }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    const int r = t & (PW - 1), g = t >> 5;
-    for (int p = 0; p < LU_NB / DB; ++p) {
-      const int jb = p * DB;
-      const float* Ui = Si + p * DB * DB;  // Uinv_pp(q, c) = Ui[c * 16 + q]
-      {
-        // X_p = B_p Uinv_pp into Xp[c][32]: thread -> row t % 32, columns
-        // 2 (t / 32) .. +1
-        const int c2 = 2 * g;
-        float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-        for (int q = 0; q < DB; ++q) {
-          const float b = Xs[(jb + q) * PXLD + r];
-          o0 = fmaf(b, Ui[c2 * DB + q], o0);
-          o1 = fmaf(b, Ui[(c2 + 1) * DB + q], o1);
-        }
-        Xp[c2 * PW + r] = o0;
-        Xp[(c2 + 1) * PW + r] = o1;
-      }
-      __syncthreads();
-      // B_q -= X_p U_pq: thread -> row t % 32, columns jb + 16 + t / 32 + 8 m;
-      // columns jb.. of the slice take X_p
-      float x[DB];
-#pragma unroll
-      for (int q = 0; q < DB; ++q) x[q] = Xp[q * PW + r];
-      Xs[(jb + 2 * g) * PXLD + r] = Xp[2 * g * PW + r];
-      Xs[(jb + 2 * g + 1) * PXLD + r] = Xp[(2 * g + 1) * PW + r];
-      for (int c = jb + DB + g; c < LU_NB; c += 8) {
-        const float* up = Ms + c * TLD + jb;
-        float acc = Xs[c * PXLD + r];
-#pragma unroll
-        for (int q4 = 0; q4 < DB; q4 += 4) {
-          const float4 u = *(const float4*)&up[q4];
-          acc = fmaf(-x[q4], u.x, acc);
-          acc = fmaf(-x[q4 + 1], u.y, acc);
-          acc = fmaf(-x[q4 + 2], u.z, acc);
-          acc = fmaf(-x[q4 + 3], u.w, acc);
-        }
-        Xs[c * PXLD + r] = acc;
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int idx = t + 256 * i, r4 = 4 * (idx & 7), c = idx >> 3;
-      *(float4*)(Ab + r4 + (size_t)c * ld) = *(const float4*)&Xs[c * PXLD + r4];
-    }
-    if (Lt) {
-      // row-major copies for the tensor-core operands: thread -> row t / 8,
-      // columns 4 (t % 8) + 32 j
-      const int rr = t >> 3, c4 = 4 * (t & 7);
-      const size_t row = (size_t)blockIdx.x * PW + rr;
-#pragma unroll
-      for (int j = 0; j < LU_NB / 32; ++j) {
-        const int c = 32 * j + c4;
-        const float4 v = make_float4(Xs[c * PXLD + rr], Xs[(c + 1) * PXLD + rr], Xs[(c + 2) * PXLD + rr],
-                                     Xs[(c + 3) * PXLD + rr]);
-        *(float4*)&Lt[row * LU_NB + c] = v;
-        *(float4*)&Ltlo[row * LU_NB + c] = make_float4(tf32_low(v.x), tf32_low(v.y), tf32_low(v.z), tf32_low(v.w));
-      }
+      const int p = blk - PANEL_BLOCKS;
+      cp_async16(&Si[p * PBS + c * PBL + r4], SIk + (2 * p + side) * DB * DB + c * DB + r4);
     }
   }
+  if (side == 0)
+    panel_slice<0, W>(Ms, Si, Xb, B + (size_t)x0 * ld, ld, ident, x0, Lt, Ltlo, Ulo);
+  else
+    panel_slice<1, W>(Ms, Si, Xb, Ap + x0, ld, ident, x0, Lt, Ltlo, Ulo);
 }
 
 // ---------------------------------------------------------------------------
@@ -1798,7 +1758,8 @@ static void lu_attrs_once() {
                        (int)gemm_mma_smem());
   cudaFuncSetAttribute(k_gemm_mma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)gemm_mma_smem());
-  cudaFuncSetAttribute(k_panels, cudaFuncAttributeMaxDynamicSharedMemorySize, PANEL_SMEM);
+  cudaFuncSetAttribute(k_panels<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem(32));
+  cudaFuncSetAttribute(k_panels<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem(64));
   cudaFuncSetAttribute(k_thin_update, cudaFuncAttributeMaxDynamicSharedMemorySize, THIN_SMEM);
 }
 
@@ -1837,6 +1798,13 @@ static void diag_block(float* A, int64_t ld, int Npad, float* Dinv, int* info, i
   count_launches(1);
 }
 
+// Slices of 32 vectors while they are at most one per SM (2 x 2432 / 32 = 152),
+// the shortest chain; beyond that of 64, whose loaded block serves twice the
+// vectors.  LU of 2048 / 4096 / 8192 columns: 0.587 / 1.310 / 4.375 ms, with 64
+// throughout 0.620 / 1.357 / 4.420, with 32 throughout 0.585 / 1.327 / 4.422
+// (with the slice in shared memory and 16 block barriers 0.622 / 1.384 / 4.506).
+constexpr int PANEL_NARROW = 2432;
+
 // the two panels of diagonal block k: U12 = L^{-1} A12, L21 = A21 U^{-1};
 // with a plan, also the step's tensor-core operands (Lt, Ltlo, Ulo)
 static void panels(float* A, int64_t ld, int Npad, float* Dinv, int k, cudaStream_t st,
@@ -1847,9 +1815,12 @@ static void panels(float* A, int64_t ld, int Npad, float* Dinv, int k, cudaStrea
   float* A12 = A + kk + (kk + LU_NB) * ld;
   float* A21 = A + (kk + LU_NB) + kk * ld;
   KScope kp(st, KC_LU_PANELS);
-  k_panels<<<dim3(rem / PW, 2), 256, PANEL_SMEM, st>>>(A + kk + kk * ld, ld, sub_inverses(Dinv, Npad, k), A12,
-                                                       A21, ld, 0, 0, 0, 0, P ? P->Lt : nullptr,
-                                                       P ? P->Ltlo : nullptr, P ? P->Ulo : nullptr);
+  const bool wide = rem > PANEL_NARROW;
+  const int W = wide ? 64 : 32;
+  auto kern = wide ? k_panels<64> : k_panels<32>;
+  kern<<<dim3(rem / W, 2), 4 * W, panel_smem(W), st>>>(A + kk + kk * ld, ld, sub_inverses(Dinv, Npad, k), A12, A21,
+                                                       ld, 0, 0, 0, 0, P ? P->Lt : nullptr, P ? P->Ltlo : nullptr,
+                                                       P ? P->Ulo : nullptr);
   count_launches(1);
 }
 
@@ -1858,7 +1829,7 @@ static void panels(float* A, int64_t ld, int Npad, float* Dinv, int k, cudaStrea
 static void block_inverses(float* A, int64_t ld, int Npad, float* Dinv, int k0, int nk, cudaStream_t st) {
   const size_t kk = (size_t)k0 * LU_NB;
   float* Lo = Dinv + (size_t)k0 * 2 * LU_NB * LU_NB;
-  k_panels<<<dim3(LU_NB / PW, 2, nk), 256, PANEL_SMEM, st>>>(
+  k_panels<32><<<dim3(LU_NB / 32, 2, nk), 128, panel_smem(32), st>>>(
       A + kk + kk * ld, ld, sub_inverses(Dinv, Npad, k0), Lo, Lo + LU_NB * LU_NB, LU_NB, 1,
       (int64_t)LU_NB * (ld + 1), LU_SI, 2 * LU_NB * LU_NB, nullptr, nullptr, nullptr);
   count_launches(1);
@@ -2104,8 +2075,8 @@ void diag_selftest(float* A1, float* A2, int64_t ld, float* D1, float* D2, float
     static const CUtensorMap none{};
     k_diag_lu<<<1, 512, DIAG_SMEM, st>>>(A1, ld, 0, SI, info, none, none, none, none, DiagPre{0, 0, 0});
   }
-  k_panels<<<dim3(LU_NB / PW, 2), 256, PANEL_SMEM, st>>>(A1, ld, SI, D1, D1 + LU_NB * LU_NB, LU_NB, 1, 0, 0, 0,
-                                                        nullptr, nullptr, nullptr);
+  k_panels<32><<<dim3(LU_NB / 32, 2), 128, panel_smem(32), st>>>(A1, ld, SI, D1, D1 + LU_NB * LU_NB, LU_NB, 1, 0, 0, 0,
+                                                                nullptr, nullptr, nullptr);
   k_diag_factor_rb<<<1, 512, sizeof(float) * LU_NB * DLD, st>>>(A2, ld, 0, D2, info);
   count_launches(3);
 }
