@@ -9,9 +9,6 @@
 // 1-7 the polyharmonic splines R, R^2 log(R+e), R^3, R^4 log(R+e), R^5,
 // R^6 log(R+e), R^7, kind 10 the fundamental solution.  Entries with
 // i == j or R^2 <= eps^2 stay zero.  Outputs column-major (Julia layout).
-// Each thread writes 16 bytes (2 FP64 or 4 FP32 rows) of each of its CTA's
-// 32 columns, so a warp stores contiguous 512-byte segments: the FP32 kernel
-// is bound by the HBM write of F and D, the FP64 one by FP64 issue.
 #include <cfloat>
 #include <cmath>
 
@@ -22,139 +19,153 @@
 namespace bem {
 namespace {
 
+// FP64 through the short functions (fast64.cuh), FP32 through the platform's
+__device__ __forceinline__ double fd_log(double x) { return f64::log(x); }
+__device__ __forceinline__ float fd_log(float x) { return logf(x); }
+__device__ __forceinline__ double fd_sqrt(double x) { return f64::sqrt(x); }
+__device__ __forceinline__ float fd_sqrt(float x) { return sqrtf(x); }
+__device__ __forceinline__ double fd_rcp(double x) { return f64::rcp(x); }
+__device__ __forceinline__ float fd_rcp(float x) { return 1.f / x; }
+
 template <typename T>
 __device__ __forceinline__ T dibem_phi(int kind, T R, T kcond, T epsa) {
   const T R2 = R * R;
   switch (kind) {
     case 1: return R;
-    case 2: return R2 * log(R + epsa);
+    case 2: return R2 * fd_log(R + epsa);
     case 3: return R2 * R;
-    case 4: return (R2 * R2) * log(R + epsa);
+    case 4: return (R2 * R2) * fd_log(R + epsa);
     case 5: return R2 * R2 * R;
-    case 6: return (R2 * R2 * R2) * log(R + epsa);
+    case 6: return (R2 * R2 * R2) * fd_log(R + epsa);
     case 7: return R2 * R2 * R2 * R;
-    default: return -log(R) / (T(2) * T(3.14159265358979323846) * kcond);
+    default: return -fd_log(R) / (T(2) * T(3.14159265358979323846) * kcond);
   }
 }
 
-// columns per CTA: the CTA's row and column coordinates are converted to T
-// once (on GB300 the FP64-to-FP32 conversion runs on the slow FP64 pipe)
-constexpr int JPC = 32;
-
-// Laplace: F, D (nt x nt)
+// F (nt x nt) and D: Laplace (DOF 1) nt x nt, Kelvin (DOF 2) 2nt x 2nt with
+// node-major blocks u11 u12; u12 u22.  Every entry depends on R or on products
+// of two components of x_j - x_i, so both matrices are symmetric to the bit:
+// a CTA forms the TB x TB tile (I, J), I >= J, once, stores it, and stores its
+// transpose as tile (J, I) through shared memory.  A warp stores 32
+// consecutive rows of a column whatever the leading dimension (a thread with
+// 16 bytes of each column, as before, stored element by element when it was
+// odd: 8193 points in FP32 145 us, now 108; the write alone takes 80, the rest
+// is issue, 82 instructions for an entry and its mirror).  FP64 is bound by its
+// arithmetic, which this halves (4095 points: Laplace 2.55 -> 0.63 ms, Kelvin
+// 1.84 -> 0.66, with the short logarithm and square root).  One kernel per phi
+// and a path without bounds for inner tiles took the FP32 one from 125 to 108.
+// Tile rows r and nb - 1 - r share blockIdx.y.
 template <typename T>
-__global__ void __launch_bounds__(128) dibem_laplace_kernel(int nt, const double* __restrict__ px,
-                                                            const double* __restrict__ py, T kcond, int kind,
-                                                            T epsa, T eps2, T* F, int64_t ldf, T* D, int64_t ldd) {
-  constexpr int RPT = 16 / sizeof(T);
-  __shared__ T sx[JPC], sy[JPC];
-  const int j0 = blockIdx.y * JPC;
-  const int nj = min(JPC, nt - j0);
-  if ((int)threadIdx.x < nj) {
-    sx[threadIdx.x] = (T)px[j0 + threadIdx.x];
-    sy[threadIdx.x] = (T)py[j0 + threadIdx.x];
-  }
-  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * RPT;
-  T xi[RPT], yi[RPT];
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-    const int i = min(i0 + r, nt - 1);
-    xi[r] = (T)px[i];
-    yi[r] = (T)py[i];
-  }
-  __syncthreads();
-  if (i0 >= nt) return;
-  // -log(R) / (2 pi k) with the constant's reciprocal formed once (per-entry
-  // FP64 divisions run on GB300's small FP64 pipe)
-  const T dcoef = T(1) / (T(2) * T(3.14159265358979323846) * kcond);
-  const bool vec = (i0 + RPT <= nt) && ((ldf | ldd) % RPT == 0) && (((uintptr_t)F | (uintptr_t)D) % 16 == 0);
-  for (int jj = 0; jj < nj; ++jj) {
-    const int j = j0 + jj;
-    const T xj = sx[jj], yj = sy[jj];
-    T f[RPT], d[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const int i = i0 + r;
-      f[r] = T(0);
-      d[r] = T(0);
-      if (i < nt && i != j) {
-        const T rx = xj - xi[r], ry = yj - yi[r];
-        const T R2 = rx * rx + ry * ry;
-        if (R2 > eps2) {
-          const T R = sqrt(R2);
-          d[r] = -log(R) * dcoef;
-          f[r] = dibem_phi<T>(kind, R, kcond, epsa);
-        }
-      }
-    }
-    T* Fc = F + i0 + (size_t)j * ldf;
-    T* Dc = D + i0 + (size_t)j * ldd;
-    if (vec) {
-      if constexpr (sizeof(T) == 8) {
-        *(double2*)Fc = make_double2(f[0], f[1]);
-        *(double2*)Dc = make_double2(d[0], d[1]);
-      } else {
-        *(float4*)Fc = make_float4(f[0], f[1], f[2], f[3]);
-        *(float4*)Dc = make_float4(d[0], d[1], d[2], d[3]);
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < RPT; ++r)
-        if (i0 + r < nt) {
-          Fc[r] = f[r];
-          Dc[r] = d[r];
-        }
-    }
-  }
-}
+struct FdArgs {
+  int nt, nb;
+  const double *px, *py;
+  T prm0, prm1, epsa, eps2;
+  T *F, *D;
+  int64_t ldf, ldd;
+};
 
-// Kelvin: F (nt x nt), D (2nt x 2nt, node-major 2x2 blocks u11 u12; u12 u22)
-template <typename T>
-__global__ void __launch_bounds__(128) dibem_kelvin_kernel(int nt, const double* __restrict__ px,
-                                                           const double* __restrict__ py, T mu, T nu, int kind,
-                                                           T epsa, T eps2, T* F, int64_t ldf, T* D, int64_t ldd) {
-  __shared__ T sx[JPC], sy[JPC];
-  const int j0 = blockIdx.y * JPC;
-  const int nj = min(JPC, nt - j0);
-  if ((int)threadIdx.x < nj) {
-    sx[threadIdx.x] = (T)px[j0 + threadIdx.x];
-    sy[threadIdx.x] = (T)py[j0 + threadIdx.x];
-  }
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const T xi = (T)px[min(i, nt - 1)], yi = (T)py[min(i, nt - 1)];
-  __syncthreads();
-  if (i >= nt) return;
+// one tile and its transpose; EDGE: it may reach beyond the last point or
+// hold the diagonal
+template <typename T, int DOF, int TB, int KIND, bool EDGE>
+__device__ __forceinline__ void dibem_fd_tile(const FdArgs<T>& a, int I, int J, T (*tr)[TB][TB + 1], const T* sx,
+                                              const T* sy, T xi, T yi) {
+  constexpr int NV = DOF == 1 ? 2 : 4, STEP = 256 / TB;
+  const int t = threadIdx.x, row = t & (TB - 1), c0 = t / TB;
   const T pi = T(3.14159265358979323846);
-  const T prod1 = T(4) * pi * (T(1) - nu);
-  const T inv_base = T(1) / (T(2) * prod1 * mu);
-  for (int jj = 0; jj < nj; ++jj) {
-    const int j = j0 + jj;
-    T f = T(0), u11 = T(0), u12 = T(0), u22 = T(0);
-    if (i != j) {
-      const T rx = sx[jj] - xi, ry = sy[jj] - yi;
-      const T R2 = rx * rx + ry * ry;
-      if (R2 > eps2) {
-        const T R = sqrt(R2);
-        f = dibem_phi<T>(kind, R, T(1), epsa);
-        // U of the 2-D Kelvin solution (`_kelvin2d_UT`, Elasticity/Fundamental.jl)
-        const T invR = T(1) / R;
-        const T dr1 = rx * invR, dr2 = ry * invR;
-        const T prod2 = (T(3) - T(4) * nu) * (-log(R));
-        u11 = (prod2 + dr1 * dr1) * inv_base;
-        u12 = (dr1 * dr2) * inv_base;
-        u22 = (prod2 + dr2 * dr2) * inv_base;
-      }
+  // Laplace: -log(R) / (2 pi k) with the constant's reciprocal formed once;
+  // Kelvin: prm0 = mu, prm1 = nu
+  const T coef = DOF == 1 ? T(1) / (T(2) * pi * a.prm0) : T(1) / (T(2) * (T(4) * pi * (T(1) - a.prm1)) * a.prm0);
+  auto put = [&](T* f, T* d, const T (&v)[NV]) {
+    *f = v[0];
+    if constexpr (DOF == 1) {
+      *d = v[1];
+    } else {
+      d[0] = v[1];
+      d[1] = v[2];
+      d[a.ldd] = v[2];
+      d[a.ldd + 1] = v[3];
     }
-    F[i + (size_t)j * ldf] = f;
-    T* c0 = D + 2 * (size_t)i + (size_t)(2 * j) * ldd;
-    T* c1 = c0 + ldd;
-    c0[0] = u11;
-    c0[1] = u12;
-    c1[0] = u12;
-    c1[1] = u22;
+  };
+  {
+    const int i = I * TB + row;
+    T* f = a.F + i + (size_t)(J * TB + c0) * a.ldf;
+    T* d = a.D + (size_t)DOF * i + (size_t)(J * TB + c0) * DOF * a.ldd;
+#pragma unroll 4
+    for (int c = c0; c < TB; c += STEP, f += STEP * a.ldf, d += STEP * DOF * a.ldd) {
+      const int j = J * TB + c;
+      T v[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) v[q] = T(0);
+      const T rx = sx[c] - xi, ry = sy[c] - yi;
+      const T R2 = rx * rx + ry * ry;
+      if ((!EDGE || i != j) && R2 > a.eps2) {
+        const T R = fd_sqrt(R2);
+        v[0] = dibem_phi<T>(KIND, R, DOF == 1 ? a.prm0 : T(1), a.epsa);
+        if constexpr (DOF == 1) {
+          v[1] = -fd_log(R) * coef;
+        } else {
+          // U of the 2-D Kelvin solution (`_kelvin2d_UT`, Elasticity/Fundamental.jl)
+          const T invR = fd_rcp(R);
+          const T dr1 = rx * invR, dr2 = ry * invR;
+          const T prod2 = (T(3) - T(4) * a.prm1) * (-fd_log(R));
+          v[1] = (prod2 + dr1 * dr1) * coef;
+          v[2] = (dr1 * dr2) * coef;
+          v[3] = (prod2 + dr2 * dr2) * coef;
+        }
+      }
+      if (!EDGE || (i < a.nt && j < a.nt)) put(f, d, v);
+#pragma unroll
+      for (int q = 0; q < NV; ++q) tr[q][c][row] = v[q];
+    }
+  }
+  if (EDGE && I == J) return;
+  __syncthreads();
+  {
+    const int j = J * TB + row;
+    T* f = a.F + j + (size_t)(I * TB + c0) * a.ldf;
+    T* d = a.D + (size_t)DOF * j + (size_t)(I * TB + c0) * DOF * a.ldd;
+#pragma unroll 4
+    for (int c = c0; c < TB; c += STEP, f += STEP * a.ldf, d += STEP * DOF * a.ldd) {
+      T v[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) v[q] = tr[q][row][c];
+      if (!EDGE || (I * TB + c < a.nt && j < a.nt)) put(f, d, v);
+    }
   }
 }
 
+template <typename T, int DOF, int TB, int KIND>
+__global__ void __launch_bounds__(256) dibem_fd_kernel(const __grid_constant__ FdArgs<T> a) {
+  __shared__ T tr[DOF == 1 ? 2 : 4][TB][TB + 1];
+  __shared__ T sx[TB], sy[TB];
+  const int y = blockIdx.y, x = blockIdx.x;
+  const int I = x <= y ? y : a.nb - 1 - y, J = x <= y ? x : x - y - 1;
+  if (x > y && I <= y) return;  // the middle row of an odd count pairs with itself
+  const int t = threadIdx.x, i = min(I * TB + (t & (TB - 1)), a.nt - 1);
+  if (t < TB) {
+    const int j = min(J * TB + t, a.nt - 1);
+    sx[t] = (T)a.px[j];
+    sy[t] = (T)a.py[j];
+  }
+  const T xi = (T)a.px[i], yi = (T)a.py[i];
+  __syncthreads();
+  if (I == J || (I + 1) * TB > a.nt)
+    dibem_fd_tile<T, DOF, TB, KIND, true>(a, I, J, tr, sx, sy, xi, yi);
+  else
+    dibem_fd_tile<T, DOF, TB, KIND, false>(a, I, J, tr, sx, sy, xi, yi);
+}
+
+template <typename T, int DOF, int TB>
+void launch_fd(int nt, const double* px, const double* py, double prm0, double prm1, int kind, double epsa, T eps,
+               T* F, int64_t ldf, T* D, int64_t ldd, cudaStream_t st) {
+  const int nb = (nt + TB - 1) / TB;
+  const FdArgs<T> a{nt, nb, px, py, (T)prm0, (T)prm1, (T)epsa, eps * eps, F, D, ldf, ldd};
+  void (*const k[8])(FdArgs<T>) = {dibem_fd_kernel<T, DOF, TB, 1>, dibem_fd_kernel<T, DOF, TB, 2>,
+                                   dibem_fd_kernel<T, DOF, TB, 3>, dibem_fd_kernel<T, DOF, TB, 4>,
+                                   dibem_fd_kernel<T, DOF, TB, 5>, dibem_fd_kernel<T, DOF, TB, 6>,
+                                   dibem_fd_kernel<T, DOF, TB, 7>, dibem_fd_kernel<T, DOF, TB, 10>};
+  k[kind == 10 ? 7 : kind - 1]<<<dim3(nb + 1, (nb + 1) / 2), 256, 0, st>>>(a);
+}
 
 template <typename T>
 __device__ __forceinline__ T dibem_phi_int(int kind, T R, T kcond, T epsa) {
@@ -505,23 +516,17 @@ extern "C" int bem_dibem_fd2d(bem_ctx* c, int nt, const double* px, const double
     dF = o0;
     dD = o1;
   }
+  // tiles of 64 only where four bytes a value keep two of them in 33 KB
   if (kind == 0) {
-    const int rpt = (int)(16 / esz);
-    dim3 grid((unsigned)((n + 128 * rpt - 1) / (128 * rpt)), (unsigned)((n + JPC - 1) / JPC));
     if (dtype == BEM_F64)
-      dibem_laplace_kernel<double><<<grid, 128, 0, c->stream>>>(nt, dx, dy, prm0, rbf, epsa, DBL_EPSILON * DBL_EPSILON,
-                                                               (double*)dF, lf, (double*)dD, lD);
+      launch_fd<double, 1, 32>(nt, dx, dy, prm0, 0, rbf, epsa, DBL_EPSILON, (double*)dF, lf, (double*)dD, lD, c->stream);
     else
-      dibem_laplace_kernel<float><<<grid, 128, 0, c->stream>>>(nt, dx, dy, (float)prm0, rbf, (float)epsa,
-                                                              FLT_EPSILON * FLT_EPSILON, (float*)dF, lf, (float*)dD, lD);
+      launch_fd<float, 1, 64>(nt, dx, dy, prm0, 0, rbf, epsa, FLT_EPSILON, (float*)dF, lf, (float*)dD, lD, c->stream);
   } else {
-    dim3 grid((unsigned)((n + 127) / 128), (unsigned)((n + JPC - 1) / JPC));
     if (dtype == BEM_F64)
-      dibem_kelvin_kernel<double><<<grid, 128, 0, c->stream>>>(nt, dx, dy, prm0, prm1, rbf, epsa,
-                                                              DBL_EPSILON * DBL_EPSILON, (double*)dF, lf, (double*)dD, lD);
+      launch_fd<double, 2, 32>(nt, dx, dy, prm0, prm1, rbf, epsa, DBL_EPSILON, (double*)dF, lf, (double*)dD, lD, c->stream);
     else
-      dibem_kelvin_kernel<float><<<grid, 128, 0, c->stream>>>(nt, dx, dy, (float)prm0, (float)prm1, rbf, (float)epsa,
-                                                             FLT_EPSILON * FLT_EPSILON, (float*)dF, lf, (float*)dD, lD);
+      launch_fd<float, 2, 32>(nt, dx, dy, prm0, prm1, rbf, epsa, FLT_EPSILON, (float*)dF, lf, (float*)dD, lD, c->stream);
   }
   count_launches(1);
   cudaError_t e = cudaGetLastError();
