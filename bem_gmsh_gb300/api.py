@@ -30,7 +30,7 @@ def geom_struct(dad: BEMdata, device: bool = False):
     """Pack a BEMdata into the C struct `bem_geom2d`.
 
     device=False: host numpy arrays (BEM_MEM_HOST).  device=True: the arrays
-    are copied once to CUDA tensors (BEM_MEM_DEVICE).  Returns (struct, keep)
+    are copied once to CUDA memory (BEM_MEM_DEVICE).  Returns (struct, keep)
     where `keep` holds the arrays alive."""
     arrs = dict(
         px=np.ascontiguousarray(dad.collocation[:, 0], dtype=np.float64),
@@ -44,7 +44,10 @@ def geom_struct(dad: BEMdata, device: bool = False):
         ew=np.ascontiguousarray(dad.elem_weight, dtype=np.float64))
     if device:
         import torch
-        arrs = {k: torch.from_numpy(v).cuda() for k, v in arrs.items()}
+        # one copy of all arrays: nine small ones took 140 us more
+        block = torch.from_numpy(np.concatenate(list(arrs.values()))).cuda()
+        parts = torch.split(block, [v.size for v in arrs.values()])
+        arrs = dict(zip(arrs, parts))
         ptr = {k: (v.data_ptr() if v.numel() else None) for k, v in arrs.items()}
     else:
         ptr = {k: (v.ctypes.data if v.size else None) for k, v in arrs.items()}

@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -33,7 +34,24 @@ namespace {
 // double-double arithmetic, bem_crmath.cuh): the tanp3c map amplifies a
 // one-ulp change of a node, so every implementation of the assembly must use
 // the same bits, and correct rounding is the one platform-independent choice.
-void gauss_legendre(int n, double* x, double* w) { bem::crm::gauss_legendre_cr(n, x, w); }
+// The rule of an order is computed once per process (16 points take 16 us, 32
+// take 59; three rules a call were 40 us and more before its first launch).
+void gauss_legendre(int n, double* x, double* w) {
+  constexpr int MOST = 64;
+  struct Rule {
+    std::once_flag once;
+    double x[MOST], w[MOST];
+  };
+  static Rule rules[MOST + 1];
+  if (n < 1 || n > MOST) {
+    bem::crm::gauss_legendre_cr(n, x, w);
+    return;
+  }
+  Rule& r = rules[n];
+  std::call_once(r.once, [&] { bem::crm::gauss_legendre_cr(n, r.x, r.w); });
+  std::memcpy(x, r.x, sizeof(double) * n);
+  std::memcpy(w, r.w, sizeof(double) * n);
+}
 
 // differentiation matrix of a barycentric basis (Interpolation.jl:193-213)
 void diff_matrix(const double* x, const double* bw, int n, double* D) {
