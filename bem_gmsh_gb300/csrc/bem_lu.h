@@ -99,7 +99,15 @@ void tc_split(const TcPlan& p, int k, cudaStream_t st);
 // for a static tile order; launches sharing ctr must not overlap.
 int tc_gemm_sub(const TcPlan& p, int k, int ro, int co, int M, int N, int* err, cudaStream_t st,
                 int* ctr = nullptr);
-// ctr: two zeroed device ints for the bulk updates' tile counter (or null)
+// The update C -= L U of the trailing matrix from block `org` on by step k and,
+// with q (step k + 1's plan), by step k + 1 in the same pass over C.  strips:
+// only its first block column and row, without the diagonal block.  Plans of
+// variant 2.
+int tc_update(const TcPlan& p, const TcPlan* q, int k, int org, bool strips, int* err, cudaStream_t st,
+              int* ctr = nullptr);
+// ctr: two zeroed device ints for the bulk updates' tile counter (or null);
+// tc: LU_PLANS plans with buffers of their own, step k uses tc[k % LU_PLANS]
+constexpr int LU_PLANS = 4;
 int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, cudaStream_t st,
                         cudaStream_t la, cudaEvent_t fork, cudaEvent_t* evP, cudaEvent_t* evT,
                         cudaStream_t tl, cudaEvent_t* evR, const TcPlan* tc, int* err, int* ctr = nullptr);

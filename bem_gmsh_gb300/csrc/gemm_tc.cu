@@ -62,6 +62,36 @@ struct TcArgs {
   int cx0, cy0;   // C map (persistent kernel): row and column of C(0, 0)
   int* ctr;       // persistent kernel: {next tile, CTAs done} (zero at launch),
                   // or null for the static order t = blockIdx.x + i gridDim.x
+  // persistent kernel: a second product of 128 in k added to the same tile
+  // (ay1, bx1, bly1 as ay0, bx0, bly0, with the second set of maps)
+  int two;
+  int ay1, bx1, bly1;
+  // persistent kernel: only the first block column (from its second block row
+  // on) and the first block row (from its second block column on) of C
+  int strips;
+};
+
+// the persistent kernel's tiles
+struct Tiles {
+  int mt, n, count, strips;
+  __device__ explicit Tiles(const TcArgs& a) : mt(a.M / BM), n(a.N), strips(a.strips) {
+    count = strips ? mt - 1 + (n - BM + BN - 1) / BN : mt * ((n + BN - 1) / BN);
+  }
+  // origin and column end of tile t
+  __device__ void at(int t, int& m0, int& n0, int& n1) const {
+    n1 = n;
+    if (!strips) {
+      m0 = (t % mt) * BM;
+      n0 = (t / mt) * BN;
+    } else if (t < mt - 1) {
+      m0 = (t + 1) * BM;
+      n0 = 0;
+      n1 = BM;
+    } else {
+      m0 = 0;
+      n0 = BM + (t - (mt - 1)) * BN;
+    }
+  }
 };
 
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_gemm_tc(const __grid_constant__ CUtensorMap mA,
@@ -343,7 +373,10 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
                                                           const __grid_constant__ CUtensorMap mAlo,
                                                           const __grid_constant__ CUtensorMap mB,
                                                           const __grid_constant__ CUtensorMap mBlo,
-                                                          const __grid_constant__ CUtensorMap mC, TcArgs a) {
+                                                          const __grid_constant__ CUtensorMap mC,
+                                                          const __grid_constant__ CUtensorMap mA1,
+                                                          const __grid_constant__ CUtensorMap mAlo1,
+                                                          const __grid_constant__ CUtensorMap mBlo1, TcArgs a) {
   extern __shared__ __align__(1024) uint8_t dsm[];
   const uint32_t base_u = smem_u32(dsm);
   const uint32_t tiles = (base_u + 1023u) & ~1023u;
@@ -367,7 +400,8 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
   volatile int* s_tile = (volatile int*)(misc + 8 * NBAR + 24);
   volatile int* s_etile = (volatile int*)(misc + 8 * NBAR + 24 + 4 * P_TRING);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int MT = a.M / BM, NT = (a.N + BN - 1) / BN, T = MT * NT;
+  const Tiles til(a);
+  const int T = til.count;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < P_STAGES; ++i) {
@@ -402,6 +436,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *s_tmem;
   constexpr int NCH = LU_NB / BK;
+  const int nchunk = a.two ? 2 * NCH : NCH;
 
   if (warp == 0 && lane == 0) {
     // operand producer; it also claims the tiles (from the global counter
@@ -416,16 +451,25 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
       s_tile[slot] = t;
       mbar_arrive(tile_full + 8 * slot);
       if (t < 0) break;
-      const int m0 = (t % MT) * BM, n0 = (t / MT) * BN;
-      for (int c = 0; c < NCH && !*s_fail; ++c, ++opc) {
+      int m0, n0, n1;
+      til.at(t, m0, n0, n1);
+      for (int c = 0; c < nchunk && !*s_fail; ++c, ++opc) {
         const int s = opc % P_STAGES;
         if (opc >= P_STAGES && !pwait(op_empty + 8 * s, ((opc / P_STAGES) - 1) & 1, s_fail)) break;
         const uint32_t st = tiles + s * STAGE_BYTES;
         mbar_expect_tx(op_full + 8 * s, STAGE_BYTES);
-        tma_load_2d(st, &mA, c * BK, a.ay0 + m0, op_full + 8 * s);
-        tma_load_2d(st + A_BYTES, &mAlo, c * BK, a.ay0 + m0, op_full + 8 * s);
-        tma_load_2d(st + 2 * A_BYTES, &mB, a.bx0 + c * BK, a.by0 + n0, op_full + 8 * s);
-        tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mBlo, a.blx0 + c * BK, a.bly0 + n0, op_full + 8 * s);
+        if (c < NCH) {
+          tma_load_2d(st, &mA, c * BK, a.ay0 + m0, op_full + 8 * s);
+          tma_load_2d(st + A_BYTES, &mAlo, c * BK, a.ay0 + m0, op_full + 8 * s);
+          tma_load_2d(st + 2 * A_BYTES, &mB, a.bx0 + c * BK, a.by0 + n0, op_full + 8 * s);
+          tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mBlo, a.blx0 + c * BK, a.bly0 + n0, op_full + 8 * s);
+        } else {
+          const int k = (c - NCH) * BK;
+          tma_load_2d(st, &mA1, k, a.ay1 + m0, op_full + 8 * s);
+          tma_load_2d(st + A_BYTES, &mAlo1, k, a.ay1 + m0, op_full + 8 * s);
+          tma_load_2d(st + 2 * A_BYTES, &mB, a.bx1 + k, a.by0 + n0, op_full + 8 * s);
+          tma_load_2d(st + 2 * A_BYTES + B_BYTES, &mBlo1, k, a.bly1 + n0, op_full + 8 * s);
+        }
         s_cnt[0] = opc + 1;
       }
     }
@@ -435,8 +479,9 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
     for (int it = 0;; ++it) {
       const int t = take_tile(tile_full, tile_empty, s_tile, it, s_fail);
       if (t < 0) break;
-      const int m0 = (t % MT) * BM, n0 = (t / MT) * BN;
-      const int nch = min(P_NCHUNK, (a.N - n0 + P_CW - 1) / P_CW);
+      int m0, n0, n1;
+      til.at(t, m0, n0, n1);
+      const int nch = min(P_NCHUNK, (n1 - n0 + P_CW - 1) / P_CW);
       for (int ch = 0; ch < nch && !*s_fail; ++ch, ++cc) {
         const int b = cc % P_CBUF;
         if (cc >= P_CBUF && !pwait(c_empty + 8 * b, ((cc / P_CBUF) - 1) & 1, s_fail)) break;
@@ -456,7 +501,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + (uint32_t)(b * BN);
       bool ok = true;
-      for (int c = 0; c < NCH; ++c, ++opc) {
+      for (int c = 0; c < nchunk; ++c, ++opc) {
         const int s = opc % P_STAGES;
         if (!pwait(op_full + 8 * s, (opc / P_STAGES) & 1, s_fail)) { ok = false; break; }
         s_cnt[2] = opc + 1;
@@ -491,12 +536,13 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
       asm volatile("bar.sync 1, 128;" ::: "memory");
       const int t = *s_etile;
       if (t < 0) break;
-      const int m0 = (t % MT) * BM, n0 = (t / MT) * BN;
+      int m0, n0, n1;
+      til.at(t, m0, n0, n1);
       const int b = it & 1;
       const int okt = pwait_warp(acc_full + 8 * b, (it >> 1) & 1, s_fail, lane);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * BN);
-      const int nch = min(P_NCHUNK, (a.N - n0 + P_CW - 1) / P_CW);
+      const int nch = min(P_NCHUNK, (n1 - n0 + P_CW - 1) / P_CW);
       for (int ch = 0; ch < nch; ++ch, ++cc) {
         const int cb = cc % P_CBUF;
         const int okc = pwait_warp(c_full + 8 * cb, (cc / P_CBUF) & 1, s_fail, lane);
@@ -727,13 +773,45 @@ int tc_gemm_sub(const TcPlan& p, int k, int ro, int co, int M, int N, int* err, 
     const int T = (M / tc::BM) * ((N + tc::BN - 1) / tc::BN);
     tc::k_gemm_tc_p<<<T < p.grid ? T : p.grid, tc::P_THREADS, tc::P_SMEM, st>>>(
         *(const CUtensorMap*)p.mA, *(const CUtensorMap*)p.mAlo, *(const CUtensorMap*)p.mB,
-        *(const CUtensorMap*)p.mBlo, *(const CUtensorMap*)p.mC, a);
+        *(const CUtensorMap*)p.mBlo, *(const CUtensorMap*)p.mC, *(const CUtensorMap*)p.mA,
+        *(const CUtensorMap*)p.mAlo, *(const CUtensorMap*)p.mBlo, a);
     return (int)cudaGetLastError();
   }
   dim3 grid(M / tc::BM, (N + tc::BN - 1) / tc::BN);
   tc::k_gemm_tc<<<grid, tc::THREADS, tc::SMEM_BYTES, st>>>(*(const CUtensorMap*)p.mA, *(const CUtensorMap*)p.mAlo,
                                                     *(const CUtensorMap*)p.mB, *(const CUtensorMap*)p.mBlo,
                                                     a);
+  return (int)cudaGetLastError();
+}
+
+int tc_update(const TcPlan& p, const TcPlan* q, int k, int org, bool strips, int* err, cudaStream_t st, int* ctr) {
+  const int o = org * LU_NB, M = p.Npad - o;
+  if (M <= 0 || (strips && M <= LU_NB)) return 0;
+  const int kk = k * LU_NB;
+  tc::TcArgs a{};
+  a.M = a.N = M;
+  a.ay0 = a.bly0 = o - kk - LU_NB;
+  a.bx0 = kk;
+  a.by0 = o;
+  a.alpha = -1.f;
+  a.beta = 1.f;
+  a.err = err;
+  a.cx0 = a.cy0 = o;
+  a.ctr = ctr;
+  a.strips = strips;
+  if (q) {
+    a.two = 1;
+    a.ay1 = a.bly1 = a.ay0 - LU_NB;
+    a.bx1 = kk + LU_NB;
+  }
+  const TcPlan& p1 = q ? *q : p;
+  const int mt = M / tc::BM;
+  const int T = strips ? mt - 1 + (M - LU_NB + tc::BN - 1) / tc::BN : mt * ((M + tc::BN - 1) / tc::BN);
+  count_launches(1);
+  tc::k_gemm_tc_p<<<T < p.grid ? T : p.grid, tc::P_THREADS, tc::P_SMEM, st>>>(
+      *(const CUtensorMap*)p.mA, *(const CUtensorMap*)p.mAlo, *(const CUtensorMap*)p.mB, *(const CUtensorMap*)p.mBlo,
+      *(const CUtensorMap*)p.mC, *(const CUtensorMap*)p1.mA, *(const CUtensorMap*)p1.mAlo,
+      *(const CUtensorMap*)p1.mBlo, a);
   return (int)cudaGetLastError();
 }
 

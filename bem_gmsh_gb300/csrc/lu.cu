@@ -1094,9 +1094,12 @@ constexpr int DIAG_SMEM_PRE = DIAG_SMEM + 1024 + DIAG_PRE_STAGES * DIAG_STAGE_BY
 // U_{k-1,k}, from that step's tensor-core operands (the maps of its TcPlan):
 // Lt / Ltlo rows 0..127, U_{k-1,k} from the matrix at (k index, n index) =
 // (bx0, by0), Ulo columns 0..127 (B maps with 128-column boxes).
+// two: step k-2's update as well (maps of its plan; the block is its second
+// block row and column).
 struct DiagPre {
   int on;
   int bx0, by0;
+  int two;
 };
 
 // acc[i][j] += sum_{q in [qs, qe)} P(r0 + i, q) Q(q, c0 + j) for column-major
@@ -1143,7 +1146,10 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
                                                  const __grid_constant__ CUtensorMap mA,
                                                  const __grid_constant__ CUtensorMap mAlo,
                                                  const __grid_constant__ CUtensorMap mB,
-                                                 const __grid_constant__ CUtensorMap mBlo, DiagPre pre) {
+                                                 const __grid_constant__ CUtensorMap mBlo,
+                                                 const __grid_constant__ CUtensorMap mA2,
+                                                 const __grid_constant__ CUtensorMap mAlo2,
+                                                 const __grid_constant__ CUtensorMap mBlo2, DiagPre pre) {
   extern __shared__ __align__(1024) float dsm[];
   float* S = dsm;                       // A -> L\U
   float* rowbuf = S + LU_NB * TLD;      // [warp 0-3][parity][2 rows][16]
@@ -1189,9 +1195,10 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
     // of theirs is read above this line
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int NCH = LU_NB / BK;
+    const int nchunk = pre.two ? 2 * NCH : NCH;
     const uint32_t full0 = bars, empty0 = bars + 8 * DIAG_PRE_STAGES, done = bars + 8 * 2 * DIAG_PRE_STAGES;
     if (warp == 0 && lane == 0) {
-      for (int c = 0; c < NCH; ++c) {
+      for (int c = 0; c < nchunk; ++c) {
         const int sidx = c % DIAG_PRE_STAGES;
         if (c >= DIAG_PRE_STAGES && !mbar_wait(empty0 + 8 * sidx, ((c / DIAG_PRE_STAGES) - 1) & 1)) {
           *s_pfail = 1;
@@ -1199,13 +1206,21 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
         }
         const uint32_t st = stg + sidx * DIAG_STAGE_BYTES;
         mbar_expect_tx(full0 + 8 * sidx, DIAG_STAGE_BYTES);
-        tma_load_2d(st, &mA, c * BK, 0, full0 + 8 * sidx);
-        tma_load_2d(st + A_BYTES, &mAlo, c * BK, 0, full0 + 8 * sidx);
-        tma_load_2d(st + 2 * A_BYTES, &mB, pre.bx0 + c * BK, pre.by0, full0 + 8 * sidx);
-        tma_load_2d(st + 2 * A_BYTES + DIAG_B_BYTES, &mBlo, c * BK, 0, full0 + 8 * sidx);
+        if (c < NCH) {
+          tma_load_2d(st, &mA, c * BK, 0, full0 + 8 * sidx);
+          tma_load_2d(st + A_BYTES, &mAlo, c * BK, 0, full0 + 8 * sidx);
+          tma_load_2d(st + 2 * A_BYTES, &mB, pre.bx0 + c * BK, pre.by0, full0 + 8 * sidx);
+          tma_load_2d(st + 2 * A_BYTES + DIAG_B_BYTES, &mBlo, c * BK, 0, full0 + 8 * sidx);
+        } else {
+          const int kc = (c - NCH) * BK;
+          tma_load_2d(st, &mA2, kc, LU_NB, full0 + 8 * sidx);
+          tma_load_2d(st + A_BYTES, &mAlo2, kc, LU_NB, full0 + 8 * sidx);
+          tma_load_2d(st + 2 * A_BYTES, &mB, pre.bx0 - LU_NB + kc, pre.by0, full0 + 8 * sidx);
+          tma_load_2d(st + 2 * A_BYTES + DIAG_B_BYTES, &mBlo2, kc, LU_NB, full0 + 8 * sidx);
+        }
       }
     } else if (warp == 1 && lane == 0) {
-      for (int c = 0; c < NCH; ++c) {
+      for (int c = 0; c < nchunk; ++c) {
         const int sidx = c % DIAG_PRE_STAGES;
         if (!mbar_wait(full0 + 8 * sidx, (c / DIAG_PRE_STAGES) & 1)) {
           *s_pfail = 1;
@@ -1772,17 +1787,22 @@ static float* sub_inverses(float* Dinv, int Npad, int k) {
 // that step's update on the tensor cores; early: the launch is ordered before
 // its predecessor in the stream ends (programmatic dependent launch)
 static void diag_block(float* A, int64_t ld, int Npad, float* Dinv, int* info, int k, cudaStream_t st,
-                       const TcPlan* P = nullptr, bool early = false) {
+                       const TcPlan* P = nullptr, bool early = false, const TcPlan* P2 = nullptr) {
   KScope kd(st, KC_LU_DIAG);
   static const CUtensorMap none{};
-  DiagPre pre{0, 0, 0};
-  const CUtensorMap* m[4] = {&none, &none, &none, &none};
+  DiagPre pre{0, 0, 0, 0};
+  const CUtensorMap* m[7] = {&none, &none, &none, &none, &none, &none, &none};
   if (P && k > 0) {
-    pre = DiagPre{1, (k - 1) * LU_NB, k * LU_NB};
+    pre = DiagPre{1, (k - 1) * LU_NB, k * LU_NB, P2 != nullptr};
     m[0] = (const CUtensorMap*)P->mA;
     m[1] = (const CUtensorMap*)P->mAlo;
     m[2] = (const CUtensorMap*)P->mB128;
     m[3] = (const CUtensorMap*)P->mBlo128;
+  }
+  if (pre.two) {
+    m[4] = (const CUtensorMap*)P2->mA;
+    m[5] = (const CUtensorMap*)P2->mAlo;
+    m[6] = (const CUtensorMap*)P2->mBlo128;
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(1);
@@ -1794,10 +1814,13 @@ static void diag_block(float* A, int64_t ld, int Npad, float* Dinv, int* info, i
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = early ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k_diag_lu, A, ld, k, sub_inverses(Dinv, Npad, 0), info, *m[0], *m[1], *m[2], *m[3], pre);
+  cudaLaunchKernelEx(&cfg, k_diag_lu, A, ld, k, sub_inverses(Dinv, Npad, 0), info, *m[0], *m[1], *m[2], *m[3], *m[4],
+                     *m[5], *m[6], pre);
   count_launches(1);
 }
 
+// the two panels of diagonal block k: U12 = L^{-1} A12, L21 = A21 U^{-1};
+// with a plan, also the step's tensor-core operands (Lt, Ltlo, Ulo)
 // Slices of 32 vectors while they are at most one per SM (2 x 2432 / 32 = 152),
 // the shortest chain; beyond that of 64, whose loaded block serves twice the
 // vectors.  LU of 2048 / 4096 / 8192 columns: 0.587 / 1.310 / 4.375 ms, with 64
@@ -1805,8 +1828,6 @@ static void diag_block(float* A, int64_t ld, int Npad, float* Dinv, int* info, i
 // (with the slice in shared memory and 16 block barriers 0.622 / 1.384 / 4.506).
 constexpr int PANEL_NARROW = 2432;
 
-// the two panels of diagonal block k: U12 = L^{-1} A12, L21 = A21 U^{-1};
-// with a plan, also the step's tensor-core operands (Lt, Ltlo, Ulo)
 static void panels(float* A, int64_t ld, int Npad, float* Dinv, int k, cudaStream_t st,
                    const TcPlan* P = nullptr) {
   const size_t kk = (size_t)k * LU_NB;
@@ -1868,7 +1889,7 @@ int lu_factor(float* A, int64_t ld, int Npad, float* Dinv, int* info, int x3, cu
   return (int)cudaGetLastError();
 }
 
-constexpr int LU_EARLY = 3072;  // see below
+constexpr int LU_EARLY = 3072, LU_PAIR = 3328;  // see below
 
 // Lookahead-1 schedule on three streams.  `la` (the critical path) factors
 // diagonal block k+1 after applying step k's update to the block itself
@@ -1878,7 +1899,20 @@ constexpr int LU_EARLY = 3072;  // see below
 // come from the panel kernel), and at the end forms the full inverses
 // of all diagonal blocks in one launch.  evP[k]: panels of step k ready;
 // evT[k]: bulk update of step k done; evR[k]: thin update of step k done.
-// tc[2]: plans with separate lo/transposed buffers for even and odd steps.
+// tc: LU_PLANS plans with operand buffers of their own, step k uses
+// tc[k % LU_PLANS].
+//
+// While more than LU_PAIR columns remain, two steps share one bulk update with
+// k = 256: an update of 128 reads and writes the trailing matrix for 128
+// multiply-adds per element, 95 us at 8064 columns of which the traffic takes
+// 77; two steps in one pass take 151.  After the first step of a pair only
+// block column and row k + 1 get its update, after the second block column and
+// row k + 1 get both (thin updates on the tensor cores, one tile per SM: 10 and
+// 15 us, where the FP32 kernel took 20 for one step), and the bulk takes the
+// rest; the diagonal block after a pair takes both steps' updates itself.
+// n = 4096 / 6144 / 8192: 1.314 / 2.563 / 4.387 ms without, 1.300 / 2.383 /
+// 3.942 with (limit 4352: 1.319 / 2.420 / 3.960; 5376: 1.317 / 2.488 / 4.051).
+// Only with the persistent kernel: batch workers run one CTA per tile.
 //
 // Once at most LU_EARLY columns remain, the bulk update (14 us at 2048) is
 // shorter than the diagonal block (26 us) it runs beside, so `la` waits for
@@ -1901,28 +1935,44 @@ int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, 
   cudaEventRecord(evP[0], la);
   for (int k = 0; k + 1 < K; ++k) {
     const int rem = Npad - (k + 1) * LU_NB;
-    const TcPlan& P = tc[k & 1];
-    const bool early = rem <= LU_EARLY, next_early = rem - LU_NB <= LU_EARLY;
+    const TcPlan &P = tc[k % LU_PLANS], &Pn = tc[(k + 1) % LU_PLANS], &Pp = tc[(k + LU_PLANS - 1) % LU_PLANS];
+    // first: steps k and k + 1 share a bulk update; second: this one and the
+    // step before do
+    const bool first = P.variant == 2 && k % 2 == 0 && rem - LU_NB > LU_PAIR;
+    const bool second = P.variant == 2 && k % 2 == 1 && rem > LU_PAIR;
+    const bool early = rem <= LU_EARLY || second, next_early = rem - LU_NB <= LU_EARLY;
+    // the last bulk update before this step: step k - 1's, or that of the
+    // pair before this one, which a second step's predecessor has waited for
     if (k >= 1 && !early) cudaStreamWaitEvent(la, evT[k - 1], 0);
     // thin update of step k without the diagonal block: needs panels k
-    // (evP[k]) and the bulk update of step k-1
+    // (evP[k]) and that bulk update
     cudaStreamWaitEvent(tl, evP[k], 0);
-    if (k >= 1) cudaStreamWaitEvent(tl, evT[k - 1], 0);
-    thin_part(A, ld, k, rem, LU_NB, rem - LU_NB, true, tl);
+    if (k >= 1 && !second) cudaStreamWaitEvent(tl, evT[k - 1], 0);
+    if (first || second) {
+      KScope kt(tl, KC_LU_THIN);
+      const int e = second ? tc_update(Pp, &P, k - 1, k + 1, true, err, tl)
+                           : tc_update(P, nullptr, k, k + 1, true, err, tl);
+      if (e) return e;
+    } else {
+      thin_part(A, ld, k, rem, LU_NB, rem - LU_NB, true, tl);
+    }
     cudaEventRecord(evR[k], tl);
     KScope crit(la, KC_LU_CRIT);
-    diag_block(A, ld, Npad, Dinv, info, k + 1, la, &P, early);
-    cudaStreamWaitEvent(st, evP[k], 0);
-    if (rem > LU_NB) {
-      KScope trail(st, KC_LU_TRAIL);
-      // operands Lt, Ltlo, Ulo of step k were written by its panels
-      int e = tc_gemm_sub(P, k, LU_NB, LU_NB, rem - LU_NB, rem - LU_NB, err, st, ctr);
-      if (e) return e;
+    diag_block(A, ld, Npad, Dinv, info, k + 1, la, &P, early, second ? &Pp : nullptr);
+    if (!first) {
+      cudaStreamWaitEvent(st, evP[k], 0);
+      if (rem > LU_NB) {
+        KScope trail(st, KC_LU_TRAIL);
+        // operands Lt, Ltlo, Ulo of step k were written by its panels
+        const int e = second ? tc_update(Pp, &P, k - 1, k + 2, false, err, st, ctr)
+                             : tc_gemm_sub(P, k, LU_NB, LU_NB, rem - LU_NB, rem - LU_NB, err, st, ctr);
+        if (e) return e;
+      }
+      cudaEventRecord(evT[k], st);
     }
-    cudaEventRecord(evT[k], st);
     cudaStreamWaitEvent(la, evR[k], 0);
     if (next_early) cudaStreamWaitEvent(la, evT[k], 0);
-    panels(A, ld, Npad, Dinv, k + 1, la, &tc[(k + 1) & 1]);
+    panels(A, ld, Npad, Dinv, k + 1, la, &Pn);
     cudaEventRecord(evP[k + 1], la);
   }
   cudaStreamWaitEvent(st, evP[K - 1], 0);
@@ -2073,7 +2123,8 @@ void diag_selftest(float* A1, float* A2, int64_t ld, float* D1, float* D2, float
   lu_attrs();
   {
     static const CUtensorMap none{};
-    k_diag_lu<<<1, 512, DIAG_SMEM, st>>>(A1, ld, 0, SI, info, none, none, none, none, DiagPre{0, 0, 0});
+    k_diag_lu<<<1, 512, DIAG_SMEM, st>>>(A1, ld, 0, SI, info, none, none, none, none, none, none, none,
+                                         DiagPre{0, 0, 0, 0});
   }
   k_panels<32><<<dim3(LU_NB / 32, 2), 128, panel_smem(32), st>>>(A1, ld, SI, D1, D1 + LU_NB * LU_NB, LU_NB, 1, 0, 0, 0,
                                                                 nullptr, nullptr, nullptr);

@@ -153,10 +153,10 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   SolvePin pin;
   if (!solve_pin(c, pin)) return BEM_ERR_NOMEM;
   Timer tf(c, 1), tr(c, 2);
-  bem::TcPlan tcp[2];
+  bem::TcPlan tcp[bem::LU_PLANS];
   const bool use_tc = c->opt_tcgen05 && x3 && c->lookahead_ready(K);
   if (use_tc) {
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < bem::LU_PLANS; ++h) {
       float* Lt = (float*)c->get(bem_ctx::SLOT_TC0 + 3 * h, sizeof(float) * (size_t)Npad * LU_NB);
       float* Ltlo = (float*)c->get(bem_ctx::SLOT_TC1 + 3 * h, sizeof(float) * (size_t)Npad * LU_NB);
       float* Ulo = (float*)c->get(bem_ctx::SLOT_TC2 + 3 * h, sizeof(float) * (size_t)Npad * LU_NB);
@@ -164,7 +164,8 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
       bem::tc_plan(tcp[h], A32, Npad, Npad, Lt, Ltlo, Ulo, c->opt_tcgen05, c->opt_tc_reserve);
     }
   }
-  const bool lookahead = use_tc && tcp[0].ok && tcp[1].ok;
+  bool lookahead = use_tc;
+  for (const bem::TcPlan& p : tcp) lookahead = lookahead && p.ok;
   // the whole factorization as one launch sequence (equilibration, LU, block
   // inverses, sweep couplings)
   // info[16], info[17]: tile counter of the persistent bulk updates
@@ -187,10 +188,10 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   // the replay removes the host launch gaps between dependent kernels of
   // the critical chain.  Its kernel arguments (tensor maps included) are
   // fixed at capture, hence the key.
-  const std::vector<const void*> key = {A64, (const void*)(intptr_t)lda, (const void*)(intptr_t)N, A32, cs, Dinv,
-                                        Mc, info, tcp[0].Lt, tcp[0].Ltlo, tcp[0].Ulo, tcp[1].Lt, tcp[1].Ltlo,
-                                        tcp[1].Ulo, st, (const void*)(intptr_t)lookahead,
-                                        (const void*)(intptr_t)tcp[0].variant, (const void*)(intptr_t)tcp[0].grid};
+  std::vector<const void*> key = {A64, (const void*)(intptr_t)lda, (const void*)(intptr_t)N, A32, cs, Dinv,
+                                  Mc, info, st, (const void*)(intptr_t)lookahead,
+                                  (const void*)(intptr_t)tcp[0].variant, (const void*)(intptr_t)tcp[0].grid};
+  for (const bem::TcPlan& p : tcp) key.insert(key.end(), {p.Lt, p.Ltlo, p.Ulo});
   const bool graphs = c->opt_graphs && lookahead && !c->prof.on;
   if (graphs && c->lu_graph_key != key) {
     if (c->lu_graph) cudaGraphExecDestroy(c->lu_graph);
@@ -779,22 +780,22 @@ extern "C" int bem_selftest(bem_ctx* c, int which, int n, double* out) {
   float* A2 = (float*)c->get(bem_ctx::SLOT_TEST1, sizeof(float) * (size_t)n * n);
   float* Dinv = (float*)c->get(bem_ctx::SLOT_LU2, sizeof(float) * bem::lu_dinv_floats(K));
   int* info = (int*)c->get(bem_ctx::SLOT_LU7, 256);
-  float* Lt = (float*)c->get(bem_ctx::SLOT_TC0, sizeof(float) * (size_t)n * LU_NB);
-  float* Ltlo = (float*)c->get(bem_ctx::SLOT_TC1, sizeof(float) * (size_t)n * LU_NB);
-  float* Ulo = (float*)c->get(bem_ctx::SLOT_TC2, sizeof(float) * (size_t)n * LU_NB);
-  if (!A1 || !A2 || !Dinv || !info || !Lt || !Ltlo || !Ulo) return BEM_ERR_NOMEM;
+  if (!A1 || !A2 || !Dinv || !info) return BEM_ERR_NOMEM;
   k_fill_test<<<1024, 256, 0, st>>>(A1, n, n, 12345u);
   cudaMemcpyAsync(A2, A1, sizeof(float) * (size_t)n * n, cudaMemcpyDeviceToDevice, st);
   cudaMemsetAsync(info, 0, 16, st);
-  bem::TcPlan tcp[2];
-  float* Lt2 = (float*)c->get(bem_ctx::SLOT_TC3, sizeof(float) * (size_t)n * LU_NB);
-  float* Ltlo2 = (float*)c->get(bem_ctx::SLOT_TC4, sizeof(float) * (size_t)n * LU_NB);
-  float* Ulo2 = (float*)c->get(bem_ctx::SLOT_TC5, sizeof(float) * (size_t)n * LU_NB);
-  if (!Lt2 || !Ltlo2 || !Ulo2 || !c->lookahead_ready(K)) return BEM_ERR_NOMEM;
-  if (!bem::tc_plan(tcp[0], A1, n, n, Lt, Ltlo, Ulo, c->opt_tcgen05, c->opt_tc_reserve) ||
-      !bem::tc_plan(tcp[1], A1, n, n, Lt2, Ltlo2, Ulo2, c->opt_tcgen05, c->opt_tc_reserve)) {
-    c->last_error = "tensor map encoding failed";
-    return BEM_ERR_UNSUPPORTED;
+  bem::TcPlan tcp[bem::LU_PLANS];
+  if (!c->lookahead_ready(K)) return BEM_ERR_NOMEM;
+  for (int h = 0; h < bem::LU_PLANS; ++h) {
+    float* o[3];
+    for (int i = 0; i < 3; ++i) {
+      o[i] = (float*)c->get(bem_ctx::SLOT_TC0 + 3 * h + i, sizeof(float) * (size_t)n * LU_NB);
+      if (!o[i]) return BEM_ERR_NOMEM;
+    }
+    if (!bem::tc_plan(tcp[h], A1, n, n, o[0], o[1], o[2], c->opt_tcgen05, c->opt_tc_reserve)) {
+      c->last_error = "tensor map encoding failed";
+      return BEM_ERR_UNSUPPORTED;
+    }
   }
   Timer t1, t2;
   cudaMemsetAsync(info + 16, 0, 8, st);
