@@ -248,7 +248,7 @@ __device__ __forceinline__ bool surely_far(const Box32& b, float px, float py, f
 // rad(R) = -(2 R^2 log R - R^2) / (8 pi k) (`_dibem_rad_id2d`, :173-177),
 // w_j = Jacobian_j * elem_weight_k.  With rad(R) / R^2 = (1 - log R^2) / (8 pi k)
 // and phi_int(R) / R^2 by phi_int_over_r2 a pair is 27 FP64 operations for an
-// odd spline (it was 90; 4098 x 4098 pairs 2.48 -> 0.84 ms, FP64 issue bound).
+// odd spline (it was 90; 4098 x 4098 pairs 2.48 -> 1.02 ms, FP64 issue bound).
 // Grid: x over 128-point row blocks, y over 32-element chunks staged in
 // shared memory; partial sums are added atomically.
 constexpr int IF_EC = 32;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(128) dibem_ifid_kernel(GeomDev g, IfidRule rw,
 // none and leave), then the elements' rule points are built in shared memory
 // and 16 lanes take a pair's rule (a thread per point went through its
 // elements alone: 13 of a warp's 32 lanes had work at best; 1.39 ms at 4098
-// nodes, now 0.06).
+// nodes, now 0.14).
 constexpr int NR_EC = 16, NR_PT = 128;
 __global__ void __launch_bounds__(NR_PT) dibem_near_kernel(const __grid_constant__ GeomDev g,
                                                           const __grid_constant__ Rules R, int rbf, double kcond,

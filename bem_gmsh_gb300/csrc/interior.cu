@@ -20,7 +20,7 @@
 // a = (rho + 1/rho) / 2, and the Gauss error is about rho^(-2 npg); rho is
 // the one that makes it 2^-60.  (npg >= 8 only: with fewer points the ellipse
 // is so large that little is gained.)  The other pairs take the map, by warps
-// (near_coop.cuh).  1000 points and 341 quadratic elements: the call 15.7 -> 0.43 ms.
+// (near_coop.cuh).  1000 points and 341 quadratic elements: the call 15.7 -> 0.39 ms.
 #include <cmath>
 #include <cstring>
 

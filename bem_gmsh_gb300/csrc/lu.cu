@@ -818,9 +818,9 @@ __global__ void __launch_bounds__(256) k_trsv(const float* __restrict__ A, int64
 // per warp; its eight partial sums meet in shared memory and one atomic per
 // row adds them to y.  The column split keeps at least 8 columns per warp and
 // spreads a small matrix over all SMs (the loop over 512 columns that every
-// thread ran took 90 us at N = 1023 whatever the GPU had idle: now 5 us);
+// thread ran took 90 us at N = 1023 whatever the GPU had idle: now 7.4);
 // at N = 8193 the bound is FP64 issue, 2 multiply-adds per clock and SM
-// (110 us; measured 136 before, 118 now).
+// (110 us; 138 measured from cold caches, before and now).
 constexpr int GV_WARPS = 8;
 __global__ void __launch_bounds__(32 * GV_WARPS) k_gemv64(const double* __restrict__ A, int64_t lda, int N,
                                                           const double* __restrict__ x, double* __restrict__ y,
@@ -864,7 +864,7 @@ __global__ void __launch_bounds__(32 * GV_WARPS) k_gemv64(const double* __restri
 // and the coefficients go straight to the host's page-locked words.  Four
 // warps per CTA, one per scheduler: a warp's FP64 add takes 64 cycles of its
 // scheduler whatever it adds, so more warps only lengthen the reductions
-// (with 16 of them a step took 15 us at N = 1023; now 8).
+// (with 16 of them a step took 15 us at N = 1023; now 10, and 21 at 8193).
 // ---------------------------------------------------------------------------
 constexpr int GS_CTAS = 16, GS_THREADS = 128, GS_MAXV = 32;
 
