@@ -486,23 +486,31 @@ def main():
     hbm, bf16, src = peaks()
     nb = (N + 127) // 128 * 128
     rems = [nb - (k + 1) * 128 for k in range(nb // 128)]
+    # bulk updates (extent, k): while more than 3328 columns remain, two steps
+    # share one pass over the trailing matrix
+    bulk = []
+    for k, r in enumerate(rems):
+        if k % 2 == 0 and r - 128 > 3328:
+            continue
+        if r > 128:
+            bulk.append((r - 128, 256 if k % 2 == 1 and r > 3328 else 128))
     iters_last = max(1, iters[-1] if iters else 1)
     algo = {
         # bytes: the FP64 system matrix A written once
         "far": ("hbm", 8.0 * N * N, "GB/s", "FP64 A written, 8 B/entry"),
         # bytes: 8 B/pair of listed near pairs is negligible; FP64 issue bound
         "near": ("hbm", 8.0 * 24 * N, "GB/s", "near/singular entries, FP64 issue bound"),
-        # bytes: FP64 A read twice (column scales, conversion) + FP32 copy written
-        "lu_prep": ("hbm", 16.0 * N * N + 4.0 * nb * nb, "GB/s", "A64 read x2 + A32 written"),
+        # bytes: FP64 A read once (the column stays in registers) + FP32 copy written
+        "lu_prep": ("hbm", 8.0 * N * N + 4.0 * nb * nb, "GB/s", "A64 read + A32 written"),
         # flops: diagonal block (4/3 128^3) + both panels (4 128^2 rem) + the
         # look-ahead column and row block updates (4 128^2 rem) per step
         "lu_crit": ("tensor", sum(4.0 / 3.0 * 128 ** 3 + 8.0 * 128 * 128 * r for r in rems), "TFLOP/s",
                     "latency-bound chain: one diagonal block per step on one SM"),
-        # bytes: the bulk trailing update reads and writes its FP32 block once
-        # per step, 8 rem'^2 B (3xTF32 intensity 96 flop/B is below the TF32
-        # machine balance, so HBM bounds it); operands come from L2
-        "lu_trail": ("hbm", sum(8.0 * max(r - 128, 0) ** 2 for r in rems), "GB/s",
-                     "tcgen05 3xTF32 trailing updates (k_gemm_tc_p): C read + write per step"),
+        # bytes: a bulk trailing update reads and writes its FP32 block once,
+        # 8 m^2 B (3xTF32 intensity 96 flop/B for one step, 192 for two, below
+        # and above the TF32 machine balance); operands come from L2
+        "lu_trail": ("hbm", sum(8.0 * m * m for m, _ in bulk), "GB/s",
+                     "tcgen05 3xTF32 trailing updates (k_gemm_tc_p): C read + write per update"),
         # bytes: FP32 L and U read once per preconditioner application
         "trsv": ("hbm", 4.0 * nb * nb * iters_last, "GB/s", "FP32 LU read per sweep pair"),
         # bytes: one FP64 A read per product (one per iteration + the final
@@ -522,10 +530,10 @@ def main():
     # of the bulk trailing update; its class is lu_trail
     dom = "lu_trail" if "lu_trail" in classes else max(classes, key=lambda k: classes[k]["ms_per_step"])
     roof = dict(classes[dom])
-    flops_trail = sum(2.0 * max(r - 128, 0) ** 2 * 128 for r in rems)
+    flops_trail = sum(2.0 * m * m * k for m, k in bulk)
     cap = GEMM_TRAFFIC_CAPTURE
     ratio = (cap["read_bytes"] + cap["write_bytes"]) / cap["algorithmic_bytes"]
-    nbulk = max(1, sum(1 for r in rems if r > 128))
+    nbulk = max(1, len(bulk))
     roof.update({"kernel": "k_gemm_tc_p (persistent bulk trailing update)", "kernel_class": dom,
                  "traffic": ratio * algo["lu_trail"][1] / nbulk,
                  "traffic_note": "bytes per average bulk launch: the measured DRAM read+write / algorithmic "
