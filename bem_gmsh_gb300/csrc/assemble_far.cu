@@ -173,7 +173,21 @@ struct PackArgs {
   double *rowsum, *b;
   int* counters;
 };
-__global__ void __launch_bounds__(256) pack_kernel(const __grid_constant__ PackArgs a) {
+// Bound by FP64 latency: a warp's FP64 instruction takes 64 cycles of its
+// scheduler, so the CTAs are small (at most one warp per scheduler up to 9700
+// points) and the logarithm table has CTAs of its own after the points' (in
+// CTAs of 256 with the table in the last one: 9.9 / 9.5 / 9.8 us at 160 / 2049 /
+// 8193 points, now 6.9 / 7.5 / 9.2).
+constexpr int PACK_T = 64;
+__global__ void __launch_bounds__(PACK_T) pack_kernel(const __grid_constant__ PackArgs a, int nb) {
+  if ((int)blockIdx.x >= nb) {
+    const int t = ((int)blockIdx.x - nb) * PACK_T + threadIdx.x;
+    if (t < df::kLogTable) {
+      const df::LogEntry e = df::log_entry(t);
+      a.logtab[t] = make_float4(e.rc_h, e.rc_l, e.lc_h, e.lc_l);
+    }
+    return;
+  }
   const GeomDev& g = a.g;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < 2) a.counters[i] = 0;
@@ -190,22 +204,19 @@ __global__ void __launch_bounds__(256) pack_kernel(const __grid_constant__ PackA
     else pack_node_dfk(g, a.R, a.ph, a.bv, i, (NodeDFK*)a.nodes);
   }
   if (i < g.ne) pack_elem(g, a.near_factor, i, a.elems);
-  if (a.prec == 3 && blockIdx.x == gridDim.x - 1 && threadIdx.x < df::kLogTable) {
-    const df::LogEntry e = df::log_entry(threadIdx.x);
-    a.logtab[threadIdx.x] = make_float4(e.rc_h, e.rc_l, e.lc_h, e.lc_l);
-  }
 }
 
 // Possibly-near (point, element) pairs into the pair list: one thread per
-// point, the CTA's 64 elements staged in shared memory (256 of them made a
-// chain of 20 us on any mesh).  Each warp first
+// point, the CTA's 32 elements staged in shared memory (256 of them made a
+// chain of 20 us on any mesh, 64 of 9.9 / 9.5 / 21 us at 160 / 2049 / 8193
+// points, now 6.8 / 7.1 / 18.3).  Each warp first
 // tests an element against the bounding box of its 32 points with the same
 // operations: IEEE subtraction is monotonic, so a box distance above the
 // limit means every point of the warp is far by the per-point test, and the
 // 32 point tests are skipped.  The hits of all the warp's elements take one
 // place in the list: an atomic with its return per element made a serial
 // chain of memory latencies (14 to 23 us, whatever the mesh).
-constexpr int CL_EC = 64;
+constexpr int CL_EC = 32;  // the hit masks of a warp's elements: one per lane
 __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, const float4* __restrict__ rows,
                                                             const ElemRec* __restrict__ elems, int nn,
                                                             int* pair_count, int2* pairs, int pair_cap) {
@@ -226,8 +237,7 @@ __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, cons
     by0 = fminf(by0, __shfl_xor_sync(0xffffffffu, by0, o));
     by1 = fmaxf(by1, __shfl_xor_sync(0xffffffffu, by1, o));
   }
-  // hit masks of element el: lane el % 32, word el / 32
-  unsigned m0 = 0, m1 = 0;
+  unsigned hits = 0;  // lane el: the points element el may be near to
   for (int el = 0; el < nel; ++el) {
     const ElemRec E = s_e[el];
     const float dx = fmaxf(fmaxf(__fsub_rn(E.lox, bx1), __fsub_rn(bx0, E.hix)), 0.f);
@@ -236,9 +246,9 @@ __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, cons
     // (a point on the element itself belongs to the on-element kernel)
     const bool need = valid && (i < (e0 + el) * nn || i >= (e0 + el + 1) * nn) && !box_far(r.x, r.y, r.z, r.w, E);
     const unsigned m = __ballot_sync(0xffffffffu, need);
-    if (lane == (el & 31)) (el < 32 ? m0 : m1) = m;
+    if (lane == el) hits = m;
   }
-  const int cnt = __popc(m0) + __popc(m1);
+  const int cnt = __popc(hits);
   int inc = cnt;
   for (int o = 1; o < 32; o <<= 1) {
     const int v = __shfl_up_sync(0xffffffffu, inc, o);
@@ -250,14 +260,10 @@ __global__ void __launch_bounds__(256) near_classify_kernel(int nt, int ne, cons
   if (lane == 0) base = atomicAdd(pair_count, total);
   base = __shfl_sync(0xffffffffu, base, 0) + inc - cnt;
   for (unsigned busy = __ballot_sync(0xffffffffu, cnt != 0); busy; busy &= busy - 1) {
-    const int src = __ffs(busy) - 1;
-    const unsigned a0 = __shfl_sync(0xffffffffu, m0, src), a1 = __shfl_sync(0xffffffffu, m1, src);
-    const int first = __shfl_sync(0xffffffffu, base, src);
-    const unsigned below = (1u << lane) - 1;
-    int slot = first + __popc(a0 & below);
-    if ((a0 >> lane & 1) && slot < pair_cap) pairs[slot] = make_int2(i, e0 + src);
-    slot = first + __popc(a0) + __popc(a1 & below);
-    if ((a1 >> lane & 1) && slot < pair_cap) pairs[slot] = make_int2(i, e0 + 32 + src);
+    const int el = __ffs(busy) - 1;
+    const unsigned m = __shfl_sync(0xffffffffu, hits, el);
+    const int slot = __shfl_sync(0xffffffffu, base, el) + __popc(m & ((1u << lane) - 1));
+    if ((m >> lane & 1) && slot < pair_cap) pairs[slot] = make_int2(i, e0 + el);
   }
 }
 
@@ -853,7 +859,8 @@ int launch_assembly(const AsmRequest& q, cudaStream_t st) {
   pa.rowsum = q.rowsum;
   pa.b = q.fused ? q.b : nullptr;
   pa.counters = q.counters;
-  pack_kernel<<<(g.nt + 255) / 256, 256, 0, st>>>(pa);
+  const int nb = (g.nt + PACK_T - 1) / PACK_T;
+  pack_kernel<<<nb + (q.prec == 3 ? (df::kLogTable + PACK_T - 1) / PACK_T : 0), PACK_T, 0, st>>>(pa, nb);
   const int key = q.ph.kind * 100 + q.prec * 10 + q.fused;
   switch (key) {
     case 0: launch_variant<1, 0, false>(q, st); break;
