@@ -1068,15 +1068,15 @@ void lu_prepare(const double* A64, int64_t lda, int N, int Npad, double* cs, flo
 //      next panel's factorization (which it slows from 2450 to 3000 cycles).
 // 26.6 us a step of the look-ahead LU (with block barriers after every phase
 // and B through the inverse of L_pp 28 to 30), 4.5 of them set-up and the
-// block's own update: A_kk -= L_{k,k-1} U_{k-1,k} (the thin update leaves the
-// block out) with the previous step's tensor-core operands, TMA loads and
-// tcgen05 MMAs into TMEM (3xTF32) while the block loads, then one TMEM read
-// per thread (the same update on mma.sync took 12 us; as a separate one-tile
-// launch it cost a launch on the chain).  67 KB of shared memory (195 KB with
-// the update's four operand stages) and the whole register file (512 threads x 128): the kernel runs alone on an SM
-// (capped at 64 registers to share an SM with a bulk-update tile it measured
-// 40 % slower).  A and ld must allow 16-byte accesses (ld % 4 == 0, 16-byte
-// aligned A).
+// block's own update by the previous step, or by both steps of a pair: A_kk -=
+// L_{k,k-1} U_{k-1,k} (the thin update leaves the block out) with those steps'
+// tensor-core operands, TMA loads and tcgen05 MMAs into TMEM (3xTF32) while the
+// block loads, then one TMEM read per thread (the same update on mma.sync took
+// 12 us; as a separate one-tile launch it cost a launch on the chain).  67 KB of
+// shared memory (195 KB with the update's four operand stages) and the whole
+// register file (512 threads x 128): the kernel runs alone on an SM (capped at
+// 64 registers to share an SM with a bulk-update tile it measured 40 % slower).
+// A and ld must allow 16-byte accesses (ld % 4 == 0, 16-byte aligned A).
 // ---------------------------------------------------------------------------
 constexpr int DB = LU_SB;       // panel width
 constexpr int TLD = LU_NB + 4;  // shared leading dimension
@@ -1407,10 +1407,6 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
       }
     }
   };
-  // The phases are pipelined: after the block row of U of panel p, warps
-  // 0-3 update only panel p+1's columns and factor them while warps 4-15
-  // store panel p, invert its 16 x 16 blocks (warps 4 and 5) and apply the
-  // rest of its trailing update.
   // 16 x 16 sub-block inverses, lane c < 16 solving for column c: unit-lower
   // by column-oriented forward substitution, upper by back substitution;
   // inverse(i, c) = out[c * 16 + i]
@@ -1439,6 +1435,10 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
         *(float4*)&out[i4] = make_float4(x[i4], x[i4 + 1], x[i4 + 2], x[i4 + 3]);
     }
   };
+  // The phases are pipelined: after the block row of U of panel p and the
+  // update of panel p+1's columns, warps 0-3 factor panel p+1 while warps 4-15
+  // store panel p, invert its 16 x 16 blocks (warps 4 and 5) and apply the
+  // rest of its trailing update.
   for (int p = -1; p < LU_NB / DB; ++p) {
     const int jb = p * DB;
     if (p >= 0) {
@@ -1680,7 +1680,8 @@ __global__ void __launch_bounds__(4 * W) k_panels(const float* __restrict__ Dk, 
 }
 
 // ---------------------------------------------------------------------------
-// Thin look-ahead updates of one LU step in FP32 on the CUDA cores: block
+// Thin look-ahead updates of one LU step in FP32 on the CUDA cores (steps that
+// are not part of a pair, see lu_factor_lookahead): block
 // column k+1 (C: rem x 128) and block row k+1 (C: 128 x rem-128) get
 // C -= L21 U12 with K = 128.  64 x 64 tiles, operands staged by cp.async,
 // 4 x 4 register tiles; a 1-D grid lists the tiles.  The column part covers
