@@ -45,21 +45,23 @@ int lu_solve_vec(const float* A, int64_t ld, int N, int Npad, const float* Dinv,
                  const double* cs, double* z, double* w, float* rf, unsigned long long* tags, int epoch, int* err,
                  cudaStream_t st, int wait_limit = 1 << 20, int wepoch_shift = 0, int pmax = LU_TRSV_PMAX);
 
+// The steps of the refinement return 0 or the CUDA error of their launch.
 // y += alpha A x
-void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, double alpha, cudaStream_t st);
+int gemv64(const double* A, int64_t lda, int N, const double* x, double* y, double alpha, cudaStream_t st);
 // Two passes of classical Gram-Schmidt of w against V[:, 0:m] (m <= 30) and
 // the normalization vn = w / |w|.  host (page-locked, 64 doubles): the
 // coefficients of the passes at [0] and [32], |w|^2 at [62]; hinfo: the two
-// ints at info.
-void gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
-                    int* hinfo, cudaStream_t st);
+// ints at info.  refuse (failure injection, normally 0): 1 no cluster above
+// the portable size is launched, 2 none at all.
+int gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
+                   int* hinfo, cudaStream_t st, int refuse = 0);
 // v = r / |r| (zeros for r = 0), x = 0 when given; *host = |r|^2; hcnt: the
-// two ints at cnt, when given
-void normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
-                 cudaStream_t st, const int* cnt = nullptr, int* hcnt = nullptr);
+// two ints at cnt, when given; refuse as above
+int normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
+                cudaStream_t st, const int* cnt = nullptr, int* hcnt = nullptr, int refuse = 0);
 // x += Z[:, 0:m] y (y on the host, m <= 32), w = b
-void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
-              cudaStream_t st);
+int add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
+             cudaStream_t st);
 
 // C (M x N) = beta C + alpha A (M x 128) B (128 x N); M, N multiples of 128.
 void gemm_tile128(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,

@@ -2061,7 +2061,7 @@ int lu_solve_vec(const float* A, int64_t ld, int N, int Npad, const float* Dinv,
   return (int)cudaLaunchCooperativeKernel((void*)k_trsv, dim3(K * P), dim3(256), args, dsm, st);
 }
 
-void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, double alpha, cudaStream_t st) {
+int gemv64(const double* A, int64_t lda, int N, const double* x, double* y, double alpha, cudaStream_t st) {
   KScope ks(st, KC_GEMV);
   count_launches(1);
   const int rb = (N + 31) / 32;
@@ -2070,47 +2070,61 @@ void gemv64(const double* A, int64_t lda, int N, const double* x, double* y, dou
   nc = nc < 1 ? 1 : (nc > most ? most : nc);
   const int cols = ((N + nc - 1) / nc + GV_WARPS - 1) / GV_WARPS * GV_WARPS;
   k_gemv64<<<dim3(rb, (N + cols - 1) / cols), 32 * GV_WARPS, 0, st>>>(A, lda, N, x, y, alpha, cols);
+  return (int)cudaGetLastError();
 }
 
-// one cluster: 16 CTAs (beyond the portable size) from N = 4096 on, where a
-// slice's FP64 arithmetic outweighs the wider barrier; else 8
+// One cluster: 16 CTAs (beyond the portable size) from N = 4096 on, where a
+// slice's FP64 arithmetic outweighs the wider barrier; else 8.  A GPU (or a
+// partition of one) that has no room for 16 refuses that launch: 8 then.
+// refuse (failure injection): 1 as such a GPU, 2 every cluster.
 template <class... P, class... X>
-static void gs_launch(void (*kern)(P...), int N, cudaStream_t st, X... args) {
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(k_gram_schmidt, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cudaFuncSetAttribute(k_normalize, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  });
-  const unsigned nc = N >= 4096 ? GS_CTAS : 8;
+static int gs_launch(void (*kern)(P...), int N, int refuse, cudaStream_t st, X... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = nc;
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(nc);
   cfg.blockDim = dim3(GS_THREADS);
   cfg.stream = st;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+  auto launch = [&](unsigned nc) {
+    if (refuse >= (nc > 8 ? 1 : 2)) return cudaErrorInvalidClusterSize;
+    at.val.clusterDim.x = nc;
+    cfg.gridDim = dim3(nc);
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+  };
+  count_launches(1);
+  if (N >= 4096) {
+    static std::once_flag once;
+    static cudaError_t wide;
+    std::call_once(once, [] {
+      wide = cudaFuncSetAttribute(k_gram_schmidt, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (wide == cudaSuccess)
+        wide = cudaFuncSetAttribute(k_normalize, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    });
+    if (wide == cudaSuccess && launch(GS_CTAS) == cudaSuccess) return 0;
+    cudaGetLastError();
+  }
+  const cudaError_t e = launch(8);
+  if (e != cudaSuccess) cudaGetLastError();
+  return (int)e;
 }
 
-void gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
-                    int* hinfo, cudaStream_t st) {
-  count_launches(1);
-  gs_launch(k_gram_schmidt, N, st, V, ldv, N, m, w, vn, host, info, hinfo);
+int gram_schmidt64(const double* V, int64_t ldv, int N, int m, double* w, double* vn, double* host, const int* info,
+                   int* hinfo, cudaStream_t st, int refuse) {
+  return gs_launch(k_gram_schmidt, N, refuse, st, V, ldv, N, m, w, vn, host, info, hinfo);
 }
-void normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
-                 cudaStream_t st, const int* cnt, int* hcnt) {
-  count_launches(1);
-  gs_launch(k_normalize, N, st, r, N, v, x, host, info, hinfo, cnt, hcnt);
+int normalize64(const double* r, int N, double* v, double* x, double* host, const int* info, int* hinfo,
+                cudaStream_t st, const int* cnt, int* hcnt, int refuse) {
+  return gs_launch(k_normalize, N, refuse, st, r, N, v, x, host, info, hinfo, cnt, hcnt);
 }
-void add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
-              cudaStream_t st) {
+int add_zy64(const double* Z, int64_t ldz, int N, int m, const double* y, double* x, const double* b, double* w,
+             cudaStream_t st) {
   count_launches(1);
   SmallVec yv{};
   for (int j = 0; j < m; ++j) yv.v[j] = y[j];
   k_add_zy<<<(N + 127) / 128, 128, 0, st>>>(Z, ldz, N, m, yv, x, b, w);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace bem

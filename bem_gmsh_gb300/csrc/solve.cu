@@ -111,6 +111,19 @@ bool solve_pin(bem_ctx* c, SolvePin& p) {
   return true;
 }
 
+// Before a step of the refinement is queued, the words its last kernel writes
+// hold what no kernel writes: a kernel that did not run cannot leave the
+// former step's, or the former call's, results in place of its own.
+constexpr int UNWRITTEN = -0x5a5a5a5a;
+void unwrite(const SolvePin& p, double* word, int at) {
+  *word = NAN;
+  p.info[at] = p.info[at + 1] = UNWRITTEN;
+}
+int unwritten(bem_ctx* c) {
+  c->last_error = "a kernel of the refinement did not run";
+  return BEM_ERR_CUDA;
+}
+
 }  // namespace
 
 void bem_release_solver(bem_ctx* c) {
@@ -181,7 +194,7 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
       r = bem::lu_factor(A32, Npad, Npad, Dinv, info, x3, st, nullptr, werr);
     if (r) return r;
     bem::lu_couplings(A32, Npad, Npad, Dinv, Mc, st);
-    return 0;
+    return (int)cudaGetLastError();
   };
   // A CUDA graph of that sequence (three streams, ~8 launches per LU step)
   // replaces its launches from the second call with the same buffers on:
@@ -239,21 +252,29 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   // first iteration is queued behind the factorization before anything of
   // either is known.  x = 0 at the start, so the first residual is b.
   std::vector<double> H((m + 1) * m), cg(m), sg(m), gvec(m + 1), y(m);
-  bem::normalize64(b, N, V, x, pin.dot, info, pin.info, st, asm_count, pin.info + 4);
+  // (their launches' first error in prc)
+  const int refuse = (c->opt_inject & 8) ? 2 : (c->opt_inject & 4) ? 1 : 0;
   int iters = 0, prc = 0;
+  auto run = [&](int e) {
+    if (e && !prc) prc = e;
+  };
+  unwrite(pin, pin.dot, 0);
+  run(bem::normalize64(b, N, V, x, pin.dot, info, pin.info, st, asm_count, pin.info + 4, refuse));
   bool converged = false, first = true;
   double bnorm = 0.0, beta = 0.0, prev_beta = INFINITY, relres = 1.0;
   while (!converged) {
     int j = 0;
     for (; j < m && iters < max_iter; ++j) {
       double* zj = Z + (size_t)j * N;
-      int e2 = bem::lu_solve_vec(A32, Npad, N, Npad, Dinv, Mc, V + (size_t)j * N, cs, zj, w, rf, tags, ++epoch, werr,
-                                 st, c->opt_wait_limit, (c->opt_inject & 2) ? 1 : 0, c->opt_sweep_ctas);
-      if (e2) prc = e2;
-      bem::gemv64(A64, lda, N, zj, w, 1.0, st);
-      bem::gram_schmidt64(V, N, N, j + 1, w, V + (size_t)(j + 1) * N, pin.hh, info, pin.info + 2, st);
+      run(bem::lu_solve_vec(A32, Npad, N, Npad, Dinv, Mc, V + (size_t)j * N, cs, zj, w, rf, tags, ++epoch, werr, st,
+                            c->opt_wait_limit, (c->opt_inject & 2) ? 1 : 0, c->opt_sweep_ctas));
+      run(bem::gemv64(A64, lda, N, zj, w, 1.0, st));
+      unwrite(pin, pin.hh + 62, 2);
+      run(bem::gram_schmidt64(V, N, N, j + 1, w, V + (size_t)(j + 1) * N, pin.hh, info, pin.info + 2, st, refuse));
       cudaError_t e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return c->cuda_fail(e, first ? "factor" : "refinement");
+      if (prc) return c->cuda_fail((cudaError_t)prc, "refinement launch");
+      if (pin.info[2] == UNWRITTEN || (first && pin.info[0] == UNWRITTEN)) return unwritten(c);
       if (first) {
         first = false;
         if (asm_count) {
@@ -286,7 +307,6 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
           return BEM_OK;
         }
       }
-      if (prc) return c->cuda_fail((cudaError_t)prc, "triangular solve launch");
       if (pin.info[3]) {
         c->last_error = "triangular-solve wait timed out";
         return BEM_ERR_INTERNAL;
@@ -323,13 +343,16 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
       for (int p = q + 1; p < j; ++p) s -= H[q + (size_t)p * (m + 1)] * y[p];
       y[q] = s / H[q + (size_t)q * (m + 1)];
     }
-    bem::add_zy64(Z, N, N, j, y.data(), x, b, w, st);
-    bem::gemv64(A64, lda, N, x, w, -1.0, st);
-    bem::normalize64(w, N, V, nullptr, pin.dot, info, pin.info + 2, st);
+    run(bem::add_zy64(Z, N, N, j, y.data(), x, b, w, st));
+    run(bem::gemv64(A64, lda, N, x, w, -1.0, st));
+    unwrite(pin, pin.dot, 2);
+    run(bem::normalize64(w, N, V, nullptr, pin.dot, info, pin.info + 2, st, nullptr, nullptr, refuse));
     if (hx) cudaMemcpyAsync(hx, x, sizeof(double) * N, cudaMemcpyDeviceToHost, st);
     tr.stop(st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return c->cuda_fail(e, "refinement");
+    if (prc) return c->cuda_fail((cudaError_t)prc, "refinement launch");
+    if (pin.info[2] == UNWRITTEN) return unwritten(c);
     beta = std::sqrt(*pin.dot);
     relres = beta / bnorm;
     converged = relres <= tol;
@@ -620,7 +643,7 @@ extern "C" int bem_ctx_set_option(bem_ctx* c, int option, int value) {
     return BEM_OK;
   }
   if (option == BEM_OPT_INJECT) {
-    if (value < 0 || value > 3) return BEM_ERR_INVALID;
+    if (value < 0 || value > 15) return BEM_ERR_INVALID;
     c->opt_inject = value;
     return BEM_OK;
   }

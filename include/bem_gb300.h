@@ -70,7 +70,11 @@ extern "C" {
                                    bit 0: every workspace allocation fails (BEM_ERR_NOMEM); bit 1: the
                                    triangular sweeps publish their results under another epoch than
                                    the one their readers wait for, so those bounded waits run out
-                                   (BEM_ERR_INTERNAL, the context stays usable) */
+                                   (BEM_ERR_INTERNAL, the context stays usable); bit 2: the
+                                   refinement's thread-block clusters above the portable size (N >= 4096)
+                                   are refused at launch, as on a GPU partition without room for them
+                                   (smaller ones take their place); bit 3: all of its clusters are
+                                   refused (BEM_ERR_CUDA) */
 #define BEM_OPT_NEARFIELD 8     /* near-singular map of the element integrals, the reference's `nearfield`
                                    knob (src/Core/Integration.jl:41-93, set per problem with set_cache!):
                                    0 (default) tanp3c, 1 plain Gauss rule, 2 euclid (sinh about the
