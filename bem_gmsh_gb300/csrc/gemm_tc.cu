@@ -62,9 +62,8 @@ struct TcArgs {
   int cx0, cy0;   // C map (persistent kernel): row and column of C(0, 0)
   int* ctr;       // persistent kernel: {next tile, CTAs done} (zero at launch),
                   // or null for the static order t = blockIdx.x + i gridDim.x
-  // persistent kernel: a second product of 128 in k added to the same tile
-  // (ay1, bx1, bly1 as ay0, bx0, bly0, with the second set of maps)
-  int two;
+  // persistent kernel of two products: the second one's ay0, bx0, bly0 (with
+  // the second set of maps)
   int ay1, bx1, bly1;
   // persistent kernel: only the first block column (from its second block row
   // on) and the first block row (from its second block column on) of C
@@ -268,13 +267,24 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_gemm_tc(const __grid_co
 // the look-ahead's diagonal and panel kernels) loops over 128 x 256 tiles in
 // column-major tile order (the B panel of a tile column stays in L2):
 //   warp 0, one lane : TMA producer of the operand chunks (P_STAGES ring).
-//   warp 1, one lane : MMA issuer into one of two 256-column TMEM
-//                      accumulators, so that tile t+1's MMAs run while the
-//                      epilogue drains tile t.
-//   warp 2, one lane : TMA producer of C in 128 x 64 chunks (two buffers).
-//   warps 4..7       : epilogue (TMEM lane quadrant = warp % 4): C chunk from
+//   warp 1, one lane : MMA issuer into the two 256-column TMEM accumulators
+//                      in turn, so that the next product's MMAs run while the
+//                      epilogue drains the last one.
+//   warp 2, one lane : TMA producer of C in 128 x 32 chunks (five buffers).
+//   warps 4..        : epilogue (TMEM lane quadrant = warp % 4): C chunk from
 //                      shared memory, r = beta C + alpha acc written back in
 //                      place, a TMA store of the chunk.
+// TWO: two products of 128 in k (two steps of the LU) update a tile in one
+// pass over C.  Each has an accumulator of its own and their sum is rounded to
+// nearest: tensor cores truncate their running sum at every instruction, and
+// one sum over both doubles the error of an update whose terms have one sign
+// (|L U - A| of an 8064-column collocation matrix 2.5e-6 against 1.1e-6 for
+// single steps, random matrices 3.2e-7 against 2.4e-7).  The epilogue, eight
+// warps with 16 columns of each chunk, takes the first product into registers
+// (128 a thread) as soon as it is there, which frees its accumulator for the
+// next tile while the second is drained: LU of 8192 columns 4.11 ms; with both
+// left in TMEM until the tile is drained 4.36 (one sum for both, and the thin
+// updates in 3xTF32 as well: 3.94).
 // C thus moves in 32 KB asynchronous copies instead of per-thread loads, and
 // neither producer waits on the other.  Every wait is bounded and also stops
 // when another role has failed (s_fail), so a failure ends the kernel within
@@ -301,7 +311,11 @@ constexpr int P_CBUF = BEM_TCP_CBUF;           // C chunk buffers
 constexpr int P_CBYTES = BM * P_CW * 4;
 constexpr int P_NCHUNK = BN / P_CW;            // C chunks per tile
 static_assert(P_CW % 32 == 0 && BN % P_CW == 0 && P_CBUF >= 2 && P_CBUF <= 8, "C chunking");
-constexpr int P_THREADS = 256;
+// epilogue warps and threads of the two forms (see k_gemm_tc_p)
+template <bool TWO>
+constexpr int P_EPI = TWO ? 8 : 4;
+template <bool TWO>
+constexpr int P_THREADS = 128 + 32 * P_EPI<TWO>;
 constexpr int P_SMEM = P_STAGES * STAGE_BYTES + P_CBUF * P_CBYTES + 1024 + 512;
 static_assert(P_SMEM <= 227 * 1024, "persistent kernel shared memory");
 constexpr uint32_t P_TMEM_COLS = 512;
@@ -369,7 +383,8 @@ __device__ __forceinline__ int take_tile(uint32_t tile_full, uint32_t tile_empty
   return t;
 }
 
-__global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constant__ CUtensorMap mA,
+template <bool TWO>
+__global__ void __launch_bounds__(P_THREADS<TWO>, 1) k_gemm_tc_p(const __grid_constant__ CUtensorMap mA,
                                                           const __grid_constant__ CUtensorMap mAlo,
                                                           const __grid_constant__ CUtensorMap mB,
                                                           const __grid_constant__ CUtensorMap mBlo,
@@ -402,6 +417,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Tiles til(a);
   const int T = til.count;
+  constexpr int EPI = P_EPI<TWO>, COLS = P_CW * 4 / EPI;  // epilogue warps; a warp's columns of a C chunk
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < P_STAGES; ++i) {
@@ -410,7 +426,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(acc_full + 8 * i, 1);
-      mbar_init(acc_empty + 8 * i, 4);  // one arrival per epilogue warp
+      mbar_init(acc_empty + 8 * i, EPI);  // one arrival per epilogue warp
     }
     for (int i = 0; i < P_CBUF; ++i) {
       mbar_init(c_full + 8 * i, 1);
@@ -435,8 +451,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *s_tmem;
-  constexpr int NCH = LU_NB / BK;
-  const int nchunk = a.two ? 2 * NCH : NCH;
+  constexpr int NCH = LU_NB / BK, PROD = TWO ? 2 : 1;
 
   if (warp == 0 && lane == 0) {
     // operand producer; it also claims the tiles (from the global counter
@@ -453,7 +468,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
       if (t < 0) break;
       int m0, n0, n1;
       til.at(t, m0, n0, n1);
-      for (int c = 0; c < nchunk && !*s_fail; ++c, ++opc) {
+      for (int c = 0; c < PROD * NCH && !*s_fail; ++c, ++opc) {
         const int s = opc % P_STAGES;
         if (opc >= P_STAGES && !pwait(op_empty + 8 * s, ((opc / P_STAGES) - 1) & 1, s_fail)) break;
         const uint32_t st = tiles + s * STAGE_BYTES;
@@ -492,76 +507,96 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
       if (*s_fail) break;
     }
   } else if (warp == 1 && lane == 0) {
-    // MMA issuer
+    // MMA issuer: product u = PROD it + p of this CTA goes to accumulator u & 1
     int opc = 0;
-    for (int it = 0;; ++it) {
+    bool ok = true;
+    for (int it = 0; ok; ++it) {
       if (take_tile(tile_full, tile_empty, s_tile, it, s_fail) < 0) break;
-      const int b = it & 1;
-      if (it >= 2 && !pwait(acc_empty + 8 * b, ((it >> 1) - 1) & 1, s_fail)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t acc = tmem + (uint32_t)(b * BN);
-      bool ok = true;
-      for (int c = 0; c < nchunk; ++c, ++opc) {
-        const int s = opc % P_STAGES;
-        if (!pwait(op_full + 8 * s, (opc / P_STAGES) & 1, s_fail)) { ok = false; break; }
-        s_cnt[2] = opc + 1;
+      for (int p = 0; p < PROD && ok; ++p) {
+        const int u = PROD * it + p, b = u & 1;
+        if (u >= 2 && !pwait(acc_empty + 8 * b, ((u >> 1) - 1) & 1, s_fail)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = tiles + s * STAGE_BYTES;
-        const uint64_t dah = sdesc(st), dal = sdesc(st + A_BYTES);
-        const uint64_t dbh = sdesc(st + 2 * A_BYTES), dbl = sdesc(st + 2 * A_BYTES + B_BYTES);
+        const uint32_t acc = tmem + (uint32_t)(b * BN);
+        for (int c = 0; c < NCH; ++c, ++opc) {
+          const int s = opc % P_STAGES;
+          if (!pwait(op_full + 8 * s, (opc / P_STAGES) & 1, s_fail)) { ok = false; break; }
+          s_cnt[2] = opc + 1;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t st = tiles + s * STAGE_BYTES;
+          const uint64_t dah = sdesc(st), dal = sdesc(st + A_BYTES);
+          const uint64_t dbh = sdesc(st + 2 * A_BYTES), dbl = sdesc(st + 2 * A_BYTES + B_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < BK / 8; ++ks) {
-          const uint64_t off = (uint64_t)((ks * 32) >> 4);
-          const uint32_t acc0 = (c > 0 || ks > 0) ? 1u : 0u;
-          mma_tf32(acc, dal + off, dbh + off, acc0);
-          mma_tf32(acc, dah + off, dbl + off, 1u);
-          mma_tf32(acc, dah + off, dbh + off, 1u);
+          for (int ks = 0; ks < BK / 8; ++ks) {
+            const uint64_t off = (uint64_t)((ks * 32) >> 4);
+            const uint32_t acc0 = (c > 0 || ks > 0) ? 1u : 0u;
+            mma_tf32(acc, dal + off, dbh + off, acc0);
+            mma_tf32(acc, dah + off, dbl + off, 1u);
+            mma_tf32(acc, dah + off, dbh + off, 1u);
+          }
+          mma_commit(op_empty + 8 * s);
         }
-        mma_commit(op_empty + 8 * s);
+        if (ok) mma_commit(acc_full + 8 * b);
       }
-      if (!ok) break;
-      mma_commit(acc_full + 8 * b);
     }
   } else if (warp >= 4) {
     // epilogue: warp w owns TMEM lanes 32 (w % 4) .. + 31 (the tile's rows).
-    // All four warps run the same sequence of waits and named barriers over
+    // All its warps run the same sequence of waits and named barriers over
     // every tile; lane 0 waits and the warp follows its answer, so a failure
     // only skips work and no warp is left at a barrier.
-    const int quad = warp & 3;
+    const int quad = warp & 3, c0 = TWO ? ((warp - 4) >> 2) * COLS : 0;
     const int rloc = quad * 32 + lane;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
     int cc = 0;
     for (int it = 0;; ++it) {
-      // thread 128 takes the tile for the four warps
+      // thread 128 takes the tile for all
       if (threadIdx.x == 128) *s_etile = take_tile(tile_full, tile_empty, s_tile, it, s_fail);
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI) : "memory");
       const int t = *s_etile;
       if (t < 0) break;
       int m0, n0, n1;
       til.at(t, m0, n0, n1);
-      const int b = it & 1;
-      const int okt = pwait_warp(acc_full + 8 * b, (it >> 1) & 1, s_fail, lane);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * BN);
       const int nch = min(P_NCHUNK, (n1 - n0 + P_CW - 1) / P_CW);
-      for (int ch = 0; ch < nch; ++ch, ++cc) {
+      uint32_t held[TWO ? P_NCHUNK : 1][COLS];
+      int okt = 1;
+      if constexpr (TWO) {
+        // the first product into registers, its accumulator back to the MMAs
+        okt = pwait_warp(acc_full, it & 1, s_fail, lane);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (okt) {
+#pragma unroll
+          for (int ch = 0; ch < P_NCHUNK; ++ch) tmem_ld<COLS>(lane_addr + ch * P_CW, held[ch]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int ch = 0; ch < P_NCHUNK; ++ch) tmem_loaded<COLS>(held[ch]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
+      }
+      const int b = TWO ? 1 : it & 1;
+      if (!pwait_warp(acc_full + 8 * b, TWO ? it & 1 : (it >> 1) & 1, s_fail, lane)) okt = 0;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int ch = 0; ch < P_NCHUNK; ++ch) {
+        if (ch >= nch) break;
         const int cb = cc % P_CBUF;
         const int okc = pwait_warp(c_full + 8 * cb, (cc / P_CBUF) & 1, s_fail, lane);
         if (okc && threadIdx.x == 128) s_cnt[3] = cc + 1;
         if (okt && okc) {
-          float* cs = (float*)(dsm + (cbuf0 - base_u) + cb * P_CBYTES);
+          float* cs = (float*)(dsm + (cbuf0 - base_u) + cb * P_CBYTES) + c0 * BM + rloc;
+          uint32_t v[COLS];
+          tmem_ld<COLS>(lane_addr + b * BN + ch * P_CW, v);
+          tmem_ld_wait();
+          tmem_loaded<COLS>(v);
 #pragma unroll
-          for (int q = 0; q < P_CW / 32; ++q) {
-            uint32_t v[32];
-            tmem_ld32(lane_addr + ch * P_CW + q * 32, v);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              float* cp = cs + (q * 32 + j) * BM + rloc;
-              *cp = a.beta * *cp + a.alpha * __uint_as_float(v[j]);
-            }
+          for (int j = 0; j < COLS; ++j) {
+            float x = __uint_as_float(v[j]);
+            if constexpr (TWO) x += __uint_as_float(held[ch][j]);
+            cs[j * BM] = a.beta * cs[j * BM] + a.alpha * x;
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI) : "memory");
         if (threadIdx.x == 128) {
           // the buffer of the previous chunk is released once its store has
           // read it; this chunk's store stays in flight meanwhile
@@ -574,6 +609,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_gemm_tc_p(const __grid_constan
           }
           if (cc > 0) mbar_arrive(c_empty + 8 * ((cc - 1) % P_CBUF));
         }
+        ++cc;
       }
       // the accumulator may be overwritten once every epilogue warp read it
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -730,7 +766,9 @@ bool tc_plan(TcPlan& p, float* A, int64_t ld, int Npad, float* Lt, float* Ltlo, 
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     p.grid = nsm - (reserve < 0 ? 0 : reserve);
     if (p.grid >= 1 &&
-        cudaFuncSetAttribute(tc::k_gemm_tc_p, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::P_SMEM) ==
+        cudaFuncSetAttribute(tc::k_gemm_tc_p<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::P_SMEM) ==
+            cudaSuccess &&
+        cudaFuncSetAttribute(tc::k_gemm_tc_p<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::P_SMEM) ==
             cudaSuccess)
       p.variant = 2;
   }
@@ -771,7 +809,7 @@ int tc_gemm_sub(const TcPlan& p, int k, int ro, int co, int M, int N, int* err, 
     a.cy0 = cy0;
     a.ctr = ctr;
     const int T = (M / tc::BM) * ((N + tc::BN - 1) / tc::BN);
-    tc::k_gemm_tc_p<<<T < p.grid ? T : p.grid, tc::P_THREADS, tc::P_SMEM, st>>>(
+    tc::k_gemm_tc_p<false><<<T < p.grid ? T : p.grid, tc::P_THREADS<false>, tc::P_SMEM, st>>>(
         *(const CUtensorMap*)p.mA, *(const CUtensorMap*)p.mAlo, *(const CUtensorMap*)p.mB,
         *(const CUtensorMap*)p.mBlo, *(const CUtensorMap*)p.mC, *(const CUtensorMap*)p.mA,
         *(const CUtensorMap*)p.mAlo, *(const CUtensorMap*)p.mBlo, a);
@@ -800,7 +838,6 @@ int tc_update(const TcPlan& p, const TcPlan* q, int k, int org, bool strips, int
   a.ctr = ctr;
   a.strips = strips;
   if (q) {
-    a.two = 1;
     a.ay1 = a.bly1 = a.ay0 - LU_NB;
     a.bx1 = kk + LU_NB;
   }
@@ -808,7 +845,8 @@ int tc_update(const TcPlan& p, const TcPlan* q, int k, int org, bool strips, int
   const int mt = M / tc::BM;
   const int T = strips ? mt - 1 + (M - LU_NB + tc::BN - 1) / tc::BN : mt * ((M + tc::BN - 1) / tc::BN);
   count_launches(1);
-  tc::k_gemm_tc_p<<<T < p.grid ? T : p.grid, tc::P_THREADS, tc::P_SMEM, st>>>(
+  (q ? tc::k_gemm_tc_p<true> : tc::k_gemm_tc_p<false>)<<<T < p.grid ? T : p.grid, q ? tc::P_THREADS<true> : tc::P_THREADS<false>,
+                                                         tc::P_SMEM, st>>>(
       *(const CUtensorMap*)p.mA, *(const CUtensorMap*)p.mAlo, *(const CUtensorMap*)p.mB, *(const CUtensorMap*)p.mBlo,
       *(const CUtensorMap*)p.mC, *(const CUtensorMap*)p1.mA, *(const CUtensorMap*)p1.mAlo,
       *(const CUtensorMap*)p1.mBlo, a);

@@ -1095,7 +1095,7 @@ constexpr int DIAG_SMEM_PRE = DIAG_SMEM + 1024 + DIAG_PRE_STAGES * DIAG_STAGE_BY
 // Lt / Ltlo rows 0..127, U_{k-1,k} from the matrix at (k index, n index) =
 // (bx0, by0), Ulo columns 0..127 (B maps with 128-column boxes).
 // two: step k-2's update as well (maps of its plan; the block is its second
-// block row and column).
+// block row and column), in an accumulator of its own.
 struct DiagPre {
   int on;
   int bx0, by0;
@@ -1183,7 +1183,7 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
     }
     if (warp == 1) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)),
-                   "r"(LU_NB)
+                   "r"(2 * LU_NB)
                    : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -1230,13 +1230,14 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
         const uint32_t st = stg + sidx * DIAG_STAGE_BYTES;
         const uint64_t dah = sdesc(st), dal = sdesc(st + A_BYTES);
         const uint64_t dbh = sdesc(st + 2 * A_BYTES), dbl = sdesc(st + 2 * A_BYTES + DIAG_B_BYTES);
+        const uint32_t acc = tmem + (uint32_t)(c >= NCH ? LU_NB : 0);
 #pragma unroll
         for (int ks = 0; ks < BK / 8; ++ks) {
           const uint64_t o = (uint64_t)((ks * 32) >> 4);
-          const uint32_t acc0 = (c > 0 || ks > 0) ? 1u : 0u;
-          mma_tf32(tmem, dal + o, dbh + o, acc0, IDESC_N128);
-          mma_tf32(tmem, dah + o, dbl + o, 1u, IDESC_N128);
-          mma_tf32(tmem, dah + o, dbh + o, 1u, IDESC_N128);
+          const uint32_t acc0 = (c % NCH > 0 || ks > 0) ? 1u : 0u;
+          mma_tf32(acc, dal + o, dbh + o, acc0, IDESC_N128);
+          mma_tf32(acc, dah + o, dbl + o, 1u, IDESC_N128);
+          mma_tf32(acc, dah + o, dbh + o, 1u, IDESC_N128);
         }
         mma_commit(empty0 + 8 * sidx);
       }
@@ -1272,6 +1273,12 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
       const int q = warp & 3, cb = 32 * (warp >> 2), r = 32 * q + lane;
       uint32_t v[32];
       tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)cb, v);
+      if (pre.two) {
+        uint32_t v1[32];
+        tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(LU_NB + cb), v1);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(v1[j]));
+      }
 #pragma unroll
       for (int j = 0; j < 32; ++j) S[(cb + j) * TLD + r] -= __uint_as_float(v[j]);
     } else if (t == 0) {
@@ -1283,7 +1290,7 @@ __global__ void __launch_bounds__(512, 1) k_diag_lu(float* __restrict__ A, int64
     __syncthreads();
     if (warp == 1) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(LU_NB) : "memory");
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * LU_NB) : "memory");
     }
   }
   int bad = 0;
@@ -1680,8 +1687,7 @@ __global__ void __launch_bounds__(4 * W) k_panels(const float* __restrict__ Dk, 
 }
 
 // ---------------------------------------------------------------------------
-// Thin look-ahead updates of one LU step in FP32 on the CUDA cores (steps that
-// are not part of a pair, see lu_factor_lookahead): block
+// Thin look-ahead updates of one LU step in FP32 on the CUDA cores: block
 // column k+1 (C: rem x 128) and block row k+1 (C: 128 x rem-128) get
 // C -= L21 U12 with K = 128.  64 x 64 tiles, operands staged by cp.async,
 // 4 x 4 register tiles; a 1-D grid lists the tiles.  The column part covers
@@ -1906,13 +1912,17 @@ constexpr int LU_EARLY = 3072, LU_PAIR = 3328;  // see below
 // While more than LU_PAIR columns remain, two steps share one bulk update with
 // k = 256: an update of 128 reads and writes the trailing matrix for 128
 // multiply-adds per element, 95 us at 8064 columns of which the traffic takes
-// 77; two steps in one pass take 151.  After the first step of a pair only
-// block column and row k + 1 get its update, after the second block column and
-// row k + 1 get both (thin updates on the tensor cores, one tile per SM: 10 and
-// 15 us, where the FP32 kernel took 20 for one step), and the bulk takes the
-// rest; the diagonal block after a pair takes both steps' updates itself.
-// n = 4096 / 6144 / 8192: 1.314 / 2.563 / 4.387 ms without, 1.300 / 2.383 /
-// 3.942 with (limit 4352: 1.319 / 2.420 / 3.960; 5376: 1.317 / 2.488 / 4.051).
+// 77.  After the first step of a pair block column and row k + 1 get its update
+// (thin update), and block column and row k + 2 too, on the tensor cores and
+// off the critical path; after the second, block column and row k + 1 get that
+// step's thin update and the bulk takes the rest; the diagonal block after a
+// pair takes both steps' updates itself.  Every entry so gets the operations
+// of single steps (its last update in FP32, the others in 3xTF32, 128 products
+// a sum) and one rounding of the matrix less: |L U - A| / |A| at 8064 columns,
+// random and collocation matrices, 2.38e-7 and 1.09e-6 without pairs, 2.23e-7
+// and 1.08e-6 with.  n = 4096 / 6144 / 8192: 1.333 / 2.566 / 4.393 ms without,
+// 1.323 / 2.473 / 4.108 with (limit 4352: 1.332 / 2.485 / 4.114; 5376: 1.332 /
+// 2.512 / 4.149).
 // Only with the persistent kernel: batch workers run one CTA per tile.
 //
 // Once at most LU_EARLY columns remain, the bulk update (14 us at 2048) is
@@ -1949,15 +1959,13 @@ int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, 
     // (evP[k]) and that bulk update
     cudaStreamWaitEvent(tl, evP[k], 0);
     if (k >= 1 && !second) cudaStreamWaitEvent(tl, evT[k - 1], 0);
-    if (first || second) {
-      KScope kt(tl, KC_LU_THIN);
-      const int e = second ? tc_update(Pp, &P, k - 1, k + 1, true, err, tl)
-                           : tc_update(P, nullptr, k, k + 1, true, err, tl);
-      if (e) return e;
-    } else {
-      thin_part(A, ld, k, rem, LU_NB, rem - LU_NB, true, tl);
-    }
+    thin_part(A, ld, k, rem, LU_NB, rem - LU_NB, true, tl);
     cudaEventRecord(evR[k], tl);
+    if (first) {
+      KScope kt(tl, KC_LU_THIN);
+      const int e = tc_update(P, nullptr, k, k + 2, true, err, tl);
+      if (e) return e;
+    }
     KScope crit(la, KC_LU_CRIT);
     diag_block(A, ld, Npad, Dinv, info, k + 1, la, &P, early, second ? &Pp : nullptr);
     if (!first) {

@@ -1,0 +1,41 @@
+// The look-ahead LU of a column-major FP64 matrix, for tests/test_gpu_lu_factors.py:
+// A32 receives L\U, cs the column scales; n a multiple of 128.
+#include "../../bem_gmsh_gb300/csrc/bem_lu.h"
+
+#include <vector>
+
+extern "C" int h_factor(const double* A64, int n, float* A32, double* cs, int variant) {
+  using namespace bem;
+  const int K = n / LU_NB;
+  int lo = 0, hi = 0, rc = 1;
+  cudaDeviceGetStreamPriorityRange(&lo, &hi);
+  cudaStream_t st[3];
+  for (int i = 0; i < 3; ++i) cudaStreamCreateWithPriority(&st[i], cudaStreamNonBlocking, i ? hi : lo);
+  std::vector<cudaEvent_t> ev(3 * K + 1);
+  for (auto& e : ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+  float* Dinv = nullptr;
+  int *info = nullptr, h[2] = {1, 1};
+  const size_t op = (size_t)n * LU_NB;
+  float* ops = nullptr;
+  TcPlan tc[LU_PLANS];
+  bool ok = cudaMalloc(&Dinv, sizeof(float) * lu_dinv_floats(K)) == cudaSuccess &&
+            cudaMalloc(&info, 256) == cudaSuccess && cudaMemset(info, 0, 256) == cudaSuccess &&
+            cudaMalloc(&ops, sizeof(float) * op * 3 * LU_PLANS) == cudaSuccess;
+  for (int i = 0; ok && i < LU_PLANS; ++i)
+    ok = tc_plan(tc[i], A32, n, n, ops + op * 3 * i, ops + op * (3 * i + 1), ops + op * (3 * i + 2), variant) &&
+         tc[i].variant == variant;
+  if (ok) {
+    cudaDeviceSynchronize();
+    lu_prepare(A64, n, n, n, cs, A32, n, st[0]);
+    rc = lu_factor_lookahead(A32, n, n, Dinv, info, st[0], st[1], ev[3 * K], ev.data(), ev.data() + K, st[2],
+                             ev.data() + 2 * K, tc, info + 1, info + 16);
+    if (cudaDeviceSynchronize() != cudaSuccess) rc = 2;
+    cudaMemcpy(h, info, sizeof(h), cudaMemcpyDeviceToHost);
+  }
+  cudaFree(Dinv);
+  cudaFree(info);
+  cudaFree(ops);
+  for (auto& e : ev) cudaEventDestroy(e);
+  for (auto& s : st) cudaStreamDestroy(s);
+  return rc ? rc : (h[0] || h[1] ? 3 : 0);
+}
