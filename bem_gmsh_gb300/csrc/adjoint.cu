@@ -576,7 +576,8 @@ extern "C" int bem_adjoint_laplace2d(bem_ctx* c, const bem_geom2d* g, double k, 
   bem_solve_stats st{};
   for (int attempt = 0;; ++attempt) {
     // (the solve checks the assembly's pair count; too short a list: again)
-    rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b, attempt == 0);
+    rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b,
+                                 attempt == 0 && bem_pairs_fit(near_factor));
     if (rc) return rc;
     rc = bem_solve_mixed_dev(c, N, A, ld, b, tol, max_iter, 1, u, &st);
     if (rc != BEM_RETRY) break;

@@ -423,8 +423,6 @@ int bem_stage_geom(bem_ctx* c, const bem_geom2d* g, int npg, int mem, GeomDev& g
   return BEM_OK;
 }
 
-// Runs one assembly (device pointers already set in q), retrying once with
-// a larger pair list if the first estimate overflowed.
 int bem_assembly_result(bem_ctx* c, const int* counts) {
   if (counts[1] != 0) {
     c->last_error = "bulk-copy wait timed out in the far-field kernel";
@@ -434,6 +432,8 @@ int bem_assembly_result(bem_ctx* c, const int* counts) {
   return counts[0] <= c->asm_cap ? BEM_OK : BEM_RETRY;
 }
 
+// Runs one assembly (device pointers already set in q), again with a larger
+// pair list if the first estimate overflowed (with `later`, the caller does).
 int bem_run_assembly(bem_ctx* c, AsmRequest& q, bool later) {
   const int nt = q.g.nt;
   const int dof = q.ph.kind == 0 ? 1 : 2;

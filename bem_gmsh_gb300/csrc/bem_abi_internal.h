@@ -128,6 +128,12 @@ int bem_stage_geom(bem_ctx* c, const bem_geom2d* g, int npg, int mem, bem::GeomD
 // the far kernel's status (asm_count, two device ints) are checked by the
 // solve that follows, with bem_assembly_result.
 int bem_run_assembly(bem_ctx* c, bem::AsmRequest& q, bool later = false);
+// Whether `later` is worth it: a smooth boundary has about 2 (near_factor + 1)
+// elements near a point and the pair list starts with room for 16, so up to 3
+// it overflows on unusual meshes only (boundaries many times closer than their
+// elements are long).  An overflow found by the solve costs a factorization
+// (1000 points with every pair near: 13.5 ms against 9.1), the wait saved 10 us.
+inline bool bem_pairs_fit(double near_factor) { return near_factor <= 3.0; }
 // BEM_OK; BEM_RETRY when the pair list was too short (the next assembly of
 // the context has a longer one); BEM_ERR_INTERNAL
 constexpr int BEM_RETRY = 1000;

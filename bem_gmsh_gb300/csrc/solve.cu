@@ -559,7 +559,7 @@ extern "C" int bem_solve2d(bem_ctx* c, const bem_geom2d* g, int kind, double prm
   // the mixed solve checks the assembly's pair count with its own first
   // results; one that had too short a list is run again
   rc = bem_assemble_system_dev(c, g, ph, BC, BV, npg, near_factor, mem, prec, A, ld, nullptr, b,
-                               mode == BEM_SOLVE_MIXED);
+                               mode == BEM_SOLVE_MIXED && bem_pairs_fit(near_factor));
   ta.stop(c->stream);
   if (rc) return rc;
   double* hx = nullptr;
