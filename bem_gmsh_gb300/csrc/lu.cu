@@ -924,9 +924,11 @@ __device__ __forceinline__ void gs_reduce(GsShared& s, int m, int buf, bool firs
 
 // w -= V (V^T w) twice (classical Gram-Schmidt with reorthogonalization),
 // vn = w / |w|.  The second pass's sums include |w|^2 before that pass, and
-// |w|^2 after it is that minus the squared coefficients (they are rounding
-// next to it).  host: [0..31] and [32..61] the two passes' coefficients, [62]
-// |w|^2; hinfo: the two LU status words.
+// |w|^2 after it is that minus the squared coefficients, which are rounding
+// next to it (2^-26 of it at most, far below the sum's own rounding); when they
+// are not, the first pass left rounding only and the vector is formed and
+// summed instead.  host: [0..31] and [32..61] the two passes' coefficients,
+// [62] |w|^2; hinfo: the two LU status words.
 __global__ void __launch_bounds__(GS_THREADS)
     k_gram_schmidt(const double* __restrict__ V, int64_t ldv, int N, int m, double* w, double* __restrict__ vn,
                    double* __restrict__ host, const int* __restrict__ info, int* __restrict__ hinfo) {
@@ -954,13 +956,24 @@ __global__ void __launch_bounds__(GS_THREADS)
     gs_reduce(s, cnt, pass, pass == 0);
     if (blockIdx.x == 0 && t < m) host[32 * pass + t] = s.h[t];
   }
-  double n2 = s.h[m];
-  for (int q = 0; q < m; ++q) n2 = fma(-s.h[q], s.h[q], n2);
-  const double sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+  double h2 = 0.0, n2 = s.h[m];
+  for (int q = 0; q < m; ++q) h2 = fma(s.h[q], s.h[q], h2);
+  const bool sum = h2 > 0x1p-26 * n2;  // the same in every CTA
+  n2 -= h2;
+  double sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0, acc = 0.0;
   for (int i = i0 + t; i < i1; i += GS_THREADS) {
     double a = w[i];
     for (int q = 0; q < m; ++q) a = fma(-V[i + (size_t)q * ldv], s.h[q], a);
-    vn[i] = a * sc;
+    vn[i] = sum ? a : a * sc;
+    if (sum) acc = fma(a, a, acc);
+  }
+  if (sum) {
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) s.warp[warp][0] = acc;
+    gs_reduce(s, 1, 0, false);  // (every CTA has read the first pass's sums)
+    n2 = s.h[0];
+    sc = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+    for (int i = i0 + t; i < i1; i += GS_THREADS) vn[i] *= sc;
   }
   if (blockIdx.x == 0 && t == 0) {
     host[62] = n2;

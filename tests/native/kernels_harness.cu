@@ -1,9 +1,22 @@
-// The look-ahead LU of a column-major FP64 matrix, for tests/test_gpu_lu_factors.py:
-// A32 receives L\U, cs the column scales; n a multiple of 128.
+// Kernels that no entry point runs alone, for the tests (conftest.py, kernels).
 #include "../../bem_gmsh_gb300/csrc/bem_lu.h"
 
 #include <vector>
 
+// One Gram-Schmidt step, all pointers on the device but host (page-locked, 64
+// doubles): bem::gram_schmidt64.
+extern "C" int h_gram_schmidt(const double* V, int N, int m, double* w, double* vn, double* host) {
+  int *info = nullptr, *hinfo = nullptr;
+  int rc = cudaMalloc(&info, 16) || cudaMemset(info, 0, 16) || cudaMallocHost(&hinfo, 16);
+  if (!rc) rc = bem::gram_schmidt64(V, N, N, m, w, vn, host, info, hinfo, 0);
+  if (cudaDeviceSynchronize() != cudaSuccess) rc = -1;
+  cudaFree(info);
+  cudaFreeHost(hinfo);
+  return rc;
+}
+
+// The look-ahead LU of a column-major FP64 matrix: A32 receives L\U, cs the
+// column scales; n a multiple of 128.
 extern "C" int h_factor(const double* A64, int n, float* A32, double* cs, int variant) {
   using namespace bem;
   const int K = n / LU_NB;

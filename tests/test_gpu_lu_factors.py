@@ -1,27 +1,16 @@
 """The factors of the look-ahead LU against 64 bits: |L U - A| with steps in
 pairs (BEM_OPT_TCGEN05 = 2, above 3712 columns) and without (1)."""
 import ctypes
-import os
-import subprocess
-import tempfile
 
 import pytest
-
-from bem_gmsh_gb300 import _build
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-HERE = os.path.dirname(os.path.abspath(__file__))
-
 
 @pytest.fixture(scope="module")
-def factor():
-    so = os.path.join(tempfile.mkdtemp(prefix="lu_harness_"), "lu_harness.so")
-    subprocess.check_call([_build._nvcc(), *_build.ARCH, "-O2", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
-                           "-cudart", "static", os.path.join(HERE, "native", "lu_harness.cu"), "-o", so,
-                           _build.LIB, "-Xlinker", "-rpath=" + _build.BUILD])
-    f = ctypes.CDLL(so).h_factor
+def factor(kernels):
+    f = kernels.h_factor
     f.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]
 
     def error(A, variant):
