@@ -94,7 +94,8 @@ __device__ __forceinline__ void interior_finish(double gt, double hs, double* ou
   }
 }
 
-// near-field maps other than tanp3c: every pair by one thread
+// near-field maps other than tanp3c, and no memory for the far rule: every
+// pair by one thread
 __global__ void __launch_bounds__(IT) interior_general_kernel(const __grid_constant__ InteriorArgs a) {
   const V2 pf{a.xp[blockIdx.x], a.yp[blockIdx.x]};
   double gt = 0.0, hs = 0.0;
@@ -320,13 +321,16 @@ extern "C" int bem_interior_laplace2d(bem_ctx* c, const bem_geom2d* g, double k,
   ia.xp = dx;
   ia.yp = dy;
   ia.out = dout;
-  if (R.nearfield != 0 || (int64_t)gd.ne * npg > (int64_t)1 << 30) {
+  // 48 bytes per element and rule node for the far rule; without them (no
+  // memory left, or more than 2^30 nodes) every pair takes the map
+  const size_t ne = (size_t)gd.ne, nr = ne * (size_t)npg;
+  double* rec = nullptr;
+  if (R.nearfield == 0 && nr <= (size_t)1 << 30)
+    rec = (double*)c->get(bem_ctx::SLOT_OUT2, sizeof(double) * (3 * ne + 6 * nr));
+  if (!rec) {
     interior_general_kernel<<<(unsigned)m, IT, 0, c->stream>>>(ia);
     count_launches(1);
   } else {
-    const size_t ne = (size_t)gd.ne, nr = ne * (size_t)npg;
-    double* rec = (double*)c->get(bem_ctx::SLOT_OUT2, sizeof(double) * (3 * ne + 6 * nr));
-    if (!rec) return BEM_ERR_NOMEM;
     const double rho = std::exp2(60.0 / (2.0 * npg));
     ia.a = npg >= 8 ? 0.5 * (rho + 1.0 / rho) : 0.0;
     ia.ex = rec;
