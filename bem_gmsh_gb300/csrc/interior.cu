@@ -10,17 +10,21 @@
 // reproducible.
 //
 // Most elements are far from a point, in units of their own size, and there
-// the npg-point Gauss rule and the near-field map's rule both give the
-// integral to rounding; the map costs 27 000 FP64 operations a pair, the
-// Gauss nodes, whose positions, weights and boundary data can be prepared per
-// element, 24 each.  Which pairs those are is decided by a bound, not by a
-// distance alone: with the element's geometry x(t) = x(0) + sum c_d t^d, if
+// the npg-point Gauss rule gives the integral to rounding, as the near-field
+// map's rule with many points does; the map costs 27 000 FP64 operations a
+// pair, the Gauss nodes, whose positions, weights and boundary data can be
+// prepared per element, 24 each.  Which pairs those are is decided by a bound,
+// not by a distance alone: with the element's geometry x(t) = x(0) + sum c_d t^d, if
 //   |p - x(0)| > sum_{d >= 1} |c_d| a^d   and   |c_1| > sum_{d >= 2} d |c_d| a^(d-1)
 // then log r, 1/r^2 and |x'| are analytic in the Bernstein ellipse of semi-axis
-// a = (rho + 1/rho) / 2, and the Gauss error is about rho^(-2 npg); rho is
-// the one that makes it 2^-60.  (npg >= 8 only: with fewer points the ellipse
-// is so large that little is gained.)  The other pairs take the map, by warps
-// (near_coop.cuh).  1000 points and 341 quadratic elements: the call 15.7 -> 0.39 ms.
+// a = (rho + 1/rho) / 2, where the field basis of degree p grows to about
+// rho^p, and the Gauss error is about rho^(p - 2 npg); rho is the one that
+// makes it 2^-60.  Against 64-point rules, at the edge of the bound, straight
+// and curved elements of degree 1 to 5, 8 to 32 points: within 1e-14 of the
+// largest integral, which is the sums' rounding (the map with 8 points: 3e-11).
+// (npg >= 8 only: with fewer points the ellipse is so large that little is
+// gained.)  The other pairs take the map, by warps (near_coop.cuh).  1000
+// points and 341 quadratic elements: the call 15.7 -> 0.39 ms.
 #include <cmath>
 #include <cstring>
 
@@ -331,7 +335,7 @@ extern "C" int bem_interior_laplace2d(bem_ctx* c, const bem_geom2d* g, double k,
     interior_general_kernel<<<(unsigned)m, IT, 0, c->stream>>>(ia);
     count_launches(1);
   } else {
-    const double rho = std::exp2(60.0 / (2.0 * npg));
+    const double rho = std::exp2(60.0 / (2.0 * npg - (gd.nn - 1)));
     ia.a = npg >= 8 ? 0.5 * (rho + 1.0 / rho) : 0.0;
     ia.ex = rec;
     ia.ey = rec + ne;
