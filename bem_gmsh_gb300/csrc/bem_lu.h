@@ -107,9 +107,15 @@ int tc_gemm_sub(const TcPlan& p, int k, int ro, int co, int M, int N, int* err, 
 // variant 2.
 int tc_update(const TcPlan& p, const TcPlan* q, int k, int org, bool strips, int* err, cudaStream_t st,
               int* ctr = nullptr);
+// Steps share bulk updates in pairs while more than LU_PAIR columns remain
+// (lu_factor_lookahead in lu.cu says why), with plans of variant 2.
+constexpr int LU_PAIR = 3328;
 // ctr: two zeroed device ints for the bulk updates' tile counter (or null);
-// tc: LU_PLANS plans with buffers of their own, step k uses tc[k % LU_PLANS]
+// tc: LU_PLANS plans, step k uses tc[k % LU_PLANS].  A pair's operands are in
+// use until its bulk update ends, two steps after: four plans with buffers of
+// their own then, else (lu_own_plans) two, each given twice.
 constexpr int LU_PLANS = 4;
+inline int lu_own_plans(int Npad, int variant) { return variant == 2 && Npad - 2 * LU_NB > LU_PAIR ? 4 : 2; }
 int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, cudaStream_t st,
                         cudaStream_t la, cudaEvent_t fork, cudaEvent_t* evP, cudaEvent_t* evT,
                         cudaStream_t tl, cudaEvent_t* evR, const TcPlan* tc, int* err, int* ctr = nullptr);

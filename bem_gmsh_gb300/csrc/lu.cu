@@ -1909,7 +1909,7 @@ int lu_factor(float* A, int64_t ld, int Npad, float* Dinv, int* info, int x3, cu
   return (int)cudaGetLastError();
 }
 
-constexpr int LU_EARLY = 3072, LU_PAIR = 3328;  // see below
+constexpr int LU_EARLY = 3072;  // see below
 
 // Lookahead-1 schedule on three streams.  `la` (the critical path) factors
 // diagonal block k+1 after applying step k's update to the block itself
@@ -1919,8 +1919,7 @@ constexpr int LU_EARLY = 3072, LU_PAIR = 3328;  // see below
 // come from the panel kernel), and at the end forms the full inverses
 // of all diagonal blocks in one launch.  evP[k]: panels of step k ready;
 // evT[k]: bulk update of step k done; evR[k]: thin update of step k done.
-// tc: LU_PLANS plans with operand buffers of their own, step k uses
-// tc[k % LU_PLANS].
+// tc: LU_PLANS plans, step k uses tc[k % LU_PLANS].
 //
 // While more than LU_PAIR columns remain, two steps share one bulk update with
 // k = 256: an update of 128 reads and writes the trailing matrix for 128

@@ -170,6 +170,10 @@ int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const
   const bool use_tc = c->opt_tcgen05 && x3 && c->lookahead_ready(K);
   if (use_tc) {
     for (int h = 0; h < bem::LU_PLANS; ++h) {
+      if (h >= 2 && h >= bem::lu_own_plans(Npad, tcp[0].variant)) {
+        tcp[h] = tcp[h - 2];
+        continue;
+      }
       float* Lt = (float*)c->get(bem_ctx::SLOT_TC0 + 3 * h, sizeof(float) * (size_t)Npad * LU_NB);
       float* Ltlo = (float*)c->get(bem_ctx::SLOT_TC1 + 3 * h, sizeof(float) * (size_t)Npad * LU_NB);
       float* Ulo = (float*)c->get(bem_ctx::SLOT_TC2 + 3 * h, sizeof(float) * (size_t)Npad * LU_NB);
