@@ -2062,7 +2062,7 @@ int lu_solve_vec(const float* A, int64_t ld, int N, int Npad, const float* Dinv,
     lu_solve_vec_steps(A, ld, Npad, Dinv, rf, rf + Npad, st);
     k_from_f32_scale<<<(N + 255) / 256, 256, 0, st>>>(rf, cs, N, z);
     cudaMemsetAsync(w, 0, sizeof(double) * N, st);
-    count_launches(2);
+    count_launches(4 * K);
     return (int)cudaGetLastError();
   }
   // CTAs per block row: as many as stay resident, at most pmax
