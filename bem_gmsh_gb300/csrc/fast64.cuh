@@ -22,7 +22,8 @@
 // pipes.  Arguments that are not positive, normal and finite take the
 // platform's functions.
 //
-// On the host (tests) the approximations are replaced by 1/x and 1/sqrt(x).
+// On the host (tests) the approximations are replaced by 1/x and 1/sqrt(x)
+// without their low 32 bits, which the hardware's do not have either.
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -226,7 +227,7 @@ BEM_HD double rcp_approx(double x) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   return y;
 #else
-  return 1.0 / x;
+  return from_bits(bits(1.0 / x) & ~0xffffffffull);
 #endif
 }
 BEM_HD double rsqrt_approx(double x) {
@@ -235,7 +236,7 @@ BEM_HD double rsqrt_approx(double x) {
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   return y;
 #else
-  return 1.0 / std::sqrt(x);
+  return from_bits(bits(1.0 / std::sqrt(x)) & ~0xffffffffull);
 #endif
 }
 

@@ -1,4 +1,5 @@
 // Kernels that no entry point runs alone, for the tests (conftest.py, kernels).
+#include "../../bem_gmsh_gb300/csrc/bem_crmath.cuh"
 #include "../../bem_gmsh_gb300/csrc/bem_lu.h"
 
 #include <vector>
@@ -51,4 +52,26 @@ extern "C" int h_factor(const double* A64, int n, float* A32, double* cs, int va
   for (auto& e : ev) cudaEventDestroy(e);
   for (auto& s : st) cudaStreamDestroy(s);
   return rc ? rc : (h[0] || h[1] ? 3 : 0);
+}
+
+// The FP64 functions of fast64.cuh and the tangent of bem_crmath.cuh on the
+// device, x, y, o device arrays of n: 0 log, 1 x / y, 2 1 / x, 3 sqrt, 4 tan,
+// 5 tan in full.
+__global__ void k_function(int which, const double* x, const double* y, int n, double* o) {
+  using namespace bem;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  switch (which) {
+    case 0: o[i] = f64::log(x[i]); break;
+    case 1: o[i] = f64::div(x[i], y[i]); break;
+    case 2: o[i] = f64::rcp(x[i]); break;
+    case 3: o[i] = f64::sqrt(x[i]); break;
+    case 4: o[i] = crm::cr_tan(x[i]); break;
+    default: o[i] = crm::cr_tan_full(x[i]); break;
+  }
+}
+extern "C" int h_function(int which, const double* x, const double* y, int n, double* o) {
+  k_function<<<(n + 255) / 256, 256>>>(which, x, y, n, o);
+  const int rc = (int)cudaGetLastError();
+  return cudaDeviceSynchronize() != cudaSuccess ? -1 : rc;
 }
