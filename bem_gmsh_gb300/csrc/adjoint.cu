@@ -33,6 +33,7 @@
 #include "bem_abi_internal.h"
 #include "bem_lu.h"
 #include "near_coop.cuh"
+#include "warp_sum.cuh"
 
 int bem_solve_mixed_dev(bem_ctx* c, int N, const double* A64, int64_t lda, const double* b, double tol,
                         int max_iter, int x3, double* x, bem_solve_stats* stats, double* hx = nullptr);
@@ -99,22 +100,6 @@ __device__ __forceinline__ void far_pair_grad(const AdjArgs& a, int i, int j, do
 // r d to the normal, and to the Jacobian (d (r.n) - lambda_i q_j log R2 / 2 k)
 // / J: 40 FP64 operations and a box test in FP32.
 constexpr int AF_ROWS = 64;
-__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
-#pragma unroll
-  for (int k = 4, o = 16; k >= 1; k >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int q = 0; q < k; ++q) {
-      const double send = up ? v[q] : v[q + k], keep = up ? v[q + k] : v[q];
-      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  double s = v[0];
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  return s;
-}
-
 __global__ void __launch_bounds__(128) adj_far_kernel(const __grid_constant__ AdjArgs a) {
   __shared__ float4 s_row[AF_ROWS];
   __shared__ double s_x[AF_ROWS], s_y[AF_ROWS], s_l[AF_ROWS], s_T[AF_ROWS];

@@ -14,11 +14,13 @@
 //   near_classify_kernel  the same box test over all (point, element) pairs,
 //                   ahead of the far kernel, lists the possibly-near pairs, so
 //                   that the near kernel runs beside the far kernel.
-//   near_kernel     one thread per listed pair: the exact FP64 near test
+//   near_kernel     a warp per up to 16 listed pairs: the exact FP64 near test
 //                   (`_near_element`, :736-754), then the tanp3c near-singular
-//                   integral, or FP64 far lumping if the pair is far after all.
-//   singular_kernel one thread per boundary collocation node: interpolated
-//                   Guiggiani on its own element (:397-457).
+//                   integral, or FP64 far lumping if the pair is far after all
+//                   (near_general_kernel: one thread per pair, other maps).
+//   singular_kernel four lanes per boundary collocation node: interpolated
+//                   Guiggiani on its own element (:397-457), as fixed weights
+//                   of its samples (singular_telles_kernel: one thread a node).
 //   finalize_kernel the row-sum diagonal H_ii = -sum_{j!=i} H_ij (:384-390,
 //                   :777-787), accumulated on the fly in FP64.
 // Output is either (H, G) column-major, or the boundary-condition swap of
@@ -769,8 +771,7 @@ static void launch_variant(const AsmRequest& q, cudaStream_t st) {
     fa.c1h = c1.h;
     fa.c1l = c1.l;
   }
-  fa.px = g.px; fa.py = g.py; fa.nx = g.nx; fa.ny = g.ny; fa.jac = g.jac;
-  for (int k = 0; k < BEM_MAXNN; ++k) fa.ew[k] = q.R.ew[k];
+  fa.px = g.px; fa.py = g.py;
   fa.H = q.H; fa.G = q.G; fa.A32 = q.A32;
   fa.bc = q.bc; fa.bv = q.bv; fa.b = q.b;
   fa.rowsum = q.rowsum;

@@ -8,8 +8,10 @@
 // domain), takes domains largest-first from a shared counter and runs the
 // full assembly + solve pipeline of bem_solve2d on it.  The blocked LU of one
 // domain is latency-bound on its diagonal chain, so running several domains
-// at once fills the SMs that one domain leaves idle.  Results are identical
-// to single-domain calls (same kernels, same order of operations per domain).
+// at once fills the SMs that one domain leaves idle.  The factors
+// of a large domain differ from a single call's by FP32 rounding: the workers'
+// trailing updates take one step each, a single call's two above 3584 columns
+// (lu_factor_lookahead).  Everything else is the single call's.
 #include <algorithm>
 #include <atomic>
 #include <numeric>

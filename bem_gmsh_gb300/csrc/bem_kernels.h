@@ -85,8 +85,7 @@ struct FarArgs {
   float c1h, c1l;           // double-float Kelvin: c = 1 - 2 nu as hi + lo
   const float4* logtab;     // double-float log table (129 entries)
   const ElemRec* elems;
-  const double *px, *py, *nx, *ny, *jac;
-  double ew[BEM_MAXNN];
+  const double *px, *py;
   void* H;      // H (or A when fused)
   void* G;      // G (unused when fused)
   float* A32;   // FP32 copy of A (mixed precision)

