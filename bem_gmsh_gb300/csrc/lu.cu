@@ -1889,28 +1889,30 @@ constexpr int LU_EARLY = 3072;  // see below
 
 // Lookahead-1 schedule on three streams.  `la` (the critical path) factors
 // diagonal block k+1 after applying step k's update to the block itself
-// (inside the diagonal kernel), then its panels; `tl` meanwhile applies the rest of step k's thin update (block
-// column k+1 below the diagonal block and block row k+1 right of it, FP32);
-// `st` runs the bulk of step k's trailing update (its tensor-core operands
-// come from the panel kernel), and at the end forms the full inverses
-// of all diagonal blocks in one launch.  evP[k]: panels of step k ready;
-// evT[k]: bulk update of step k done; evR[k]: thin update of step k done.
+// (inside the diagonal kernel), then its panels; `tl` meanwhile applies the
+// rest of step k's thin update (block column k+1 below the diagonal block and
+// block row k+1 right of it, FP32); `st` runs the bulk of step k's trailing
+// update (its tensor-core operands come from the panel kernel), and at the end
+// forms the full inverses of all diagonal blocks in one launch.  evP[k]: panels
+// of step k ready; evT[k]: update of step k on `st` done; evR[k]: thin update
+// of step k done.
 // tc: LU_PLANS plans, step k uses tc[k % LU_PLANS].
 //
 // While more than LU_PAIR columns remain, two steps share one bulk update with
 // k = 256: an update of 128 reads and writes the trailing matrix for 128
 // multiply-adds per element, 95 us at 8064 columns of which the traffic takes
-// 77.  After the first step of a pair block column and row k + 1 get its update
-// (thin update), and block column and row k + 2 too, on the tensor cores and
-// off the critical path; after the second, block column and row k + 1 get that
-// step's thin update and the bulk takes the rest; the diagonal block after a
-// pair takes both steps' updates itself.  Every entry so gets the operations
+// 77; two steps in one pass take 146.  After the first step of a pair block
+// column and row k + 1 get its thin update, and block column and row k + 2 its
+// update on the tensor cores; after the second, block column and row k + 1 get
+// that step's thin update and the bulk takes the rest; the diagonal block after
+// a pair takes both steps' updates itself.  Every entry so gets the operations
 // of single steps (its last update in FP32, the others in 3xTF32, 128 products
 // a sum) and one rounding of the matrix less: |L U - A| / |A| at 8064 columns,
 // random and collocation matrices, 2.38e-7 and 1.09e-6 without pairs, 2.23e-7
-// and 1.08e-6 with.  n = 4096 / 6144 / 8192: 1.333 / 2.566 / 4.393 ms without,
-// 1.323 / 2.473 / 4.108 with (limit 4352: 1.332 / 2.485 / 4.114; 5376: 1.332 /
-// 2.512 / 4.149).
+// and 1.08e-6 with.  The factorization of a solve at n = 4096 / 6144 / 8192,
+// replayed from its graph: 1.29 / 2.58 / 4.50 ms without, 1.28 / 2.45 / 4.19
+// with (limit 4352: 1.29 / 2.48 / 4.20; 5376: 1.29 / 2.53 / 4.26); launched
+// directly 1.37 / 2.65 / 4.68 and 1.38 / 2.68 / 4.48.
 // Only with the persistent kernel: batch workers run one CTA per tile.
 //
 // Once at most LU_EARLY columns remain, the bulk update (14 us at 2048) is
@@ -1920,7 +1922,9 @@ constexpr int LU_EARLY = 3072;  // see below
 // panels' programmatic dependent: its set-up (4.8k cycles: TMEM, barriers,
 // the first instruction lines) and launch overlap the panels.  n = 1024 /
 // 2048 / 4096: 0.344 / 0.691 / 1.437 ms without, 0.309 / 0.622 / 1.386 with
-// (limit 2048: 1.396, 4096: 1.41; at 8192 the bulk update bounds both).
+// (limit 2048: 1.396, 4096: 1.41; at 8192 the bulk update bounds both).  The
+// steps of a pair do the same: the diagonal block has its SM before the thin
+// update's CTAs take them all (else 10 to 16 us a pair).
 int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, cudaStream_t st,
                         cudaStream_t la, cudaEvent_t fork, cudaEvent_t* evP, cudaEvent_t* evT,
                         cudaStream_t tl, cudaEvent_t* evR, const TcPlan* tc, int* err, int* ctr) {
@@ -1937,38 +1941,39 @@ int lu_factor_lookahead(float* A, int64_t ld, int Npad, float* Dinv, int* info, 
     const TcPlan &P = tc[k % LU_PLANS], &Pn = tc[(k + 1) % LU_PLANS], &Pp = tc[(k + LU_PLANS - 1) % LU_PLANS];
     // first: steps k and k + 1 share a bulk update; second: this one and the
     // step before do
-    const bool first = P.variant == 2 && k % 2 == 0 && rem - LU_NB > LU_PAIR;
-    const bool second = P.variant == 2 && k % 2 == 1 && rem > LU_PAIR;
-    const bool early = rem <= LU_EARLY || second, next_early = rem - LU_NB <= LU_EARLY;
+    auto first_of_pair = [&](int q, int r) { return P.variant == 2 && q % 2 == 0 && r - LU_NB > LU_PAIR; };
+    const bool first = first_of_pair(k, rem), second = k > 0 && first_of_pair(k - 1, rem + LU_NB);
+    const bool early = rem <= LU_EARLY || first || second;
+    const bool next_early = rem - LU_NB <= LU_EARLY || first_of_pair(k + 1, rem - LU_NB);
     // the last bulk update before this step: step k - 1's, or that of the
     // pair before this one, which a second step's predecessor has waited for
     if (k >= 1 && !early) cudaStreamWaitEvent(la, evT[k - 1], 0);
+    {
+      KScope crit(la, KC_LU_CRIT);
+      diag_block(A, ld, Npad, Dinv, info, k + 1, la, &P, early, second ? &Pp : nullptr);
+    }
     // thin update of step k without the diagonal block: needs panels k
-    // (evP[k]) and that bulk update
+    // (evP[k]) and that bulk update (a second step: the block column and row
+    // that its predecessor updated ahead)
     cudaStreamWaitEvent(tl, evP[k], 0);
-    if (k >= 1 && !second) cudaStreamWaitEvent(tl, evT[k - 1], 0);
+    if (k >= 1) cudaStreamWaitEvent(tl, evT[k - 1], 0);
     thin_part(A, ld, k, rem, LU_NB, rem - LU_NB, true, tl);
     cudaEventRecord(evR[k], tl);
-    if (first) {
-      KScope kt(tl, KC_LU_THIN);
-      const int e = tc_update(P, nullptr, k, k + 2, true, err, tl);
+    cudaStreamWaitEvent(st, evP[k], 0);
+    // (the bulk of a pair would hold every SM before the thin update starts)
+    if (second) cudaStreamWaitEvent(st, evR[k], 0);
+    if (rem > LU_NB) {
+      KScope trail(st, first ? KC_LU_THIN : KC_LU_TRAIL);
+      // operands Lt, Ltlo, Ulo of step k were written by its panels
+      const int e = first    ? tc_update(P, nullptr, k, k + 2, true, err, st)
+                    : second ? tc_update(Pp, &P, k - 1, k + 2, false, err, st, ctr)
+                             : tc_gemm_sub(P, k, LU_NB, LU_NB, rem - LU_NB, rem - LU_NB, err, st, ctr);
       if (e) return e;
     }
+    cudaEventRecord(evT[k], st);
     KScope crit(la, KC_LU_CRIT);
-    diag_block(A, ld, Npad, Dinv, info, k + 1, la, &P, early, second ? &Pp : nullptr);
-    if (!first) {
-      cudaStreamWaitEvent(st, evP[k], 0);
-      if (rem > LU_NB) {
-        KScope trail(st, KC_LU_TRAIL);
-        // operands Lt, Ltlo, Ulo of step k were written by its panels
-        const int e = second ? tc_update(Pp, &P, k - 1, k + 2, false, err, st, ctr)
-                             : tc_gemm_sub(P, k, LU_NB, LU_NB, rem - LU_NB, rem - LU_NB, err, st, ctr);
-        if (e) return e;
-      }
-      cudaEventRecord(evT[k], st);
-    }
     cudaStreamWaitEvent(la, evR[k], 0);
-    if (next_early) cudaStreamWaitEvent(la, evT[k], 0);
+    if (next_early && !first) cudaStreamWaitEvent(la, evT[k], 0);
     panels(A, ld, Npad, Dinv, k + 1, la, &Pn);
     cudaEventRecord(evP[k + 1], la);
   }
