@@ -75,7 +75,7 @@ __device__ __forceinline__ void pack_node_d(const GeomDev& g, const Rules& R, co
                                             NodeD* nodes) {
   const double w = g.jac[j] * R.ew[j % g.nn];
   const coop::Consts k = ph.kind == 0 ? coop::make_consts<1>(ph) : coop::Consts{1.0, 0.0, 1.0, 0.0};
-  nodes[j] = NodeD{g.nx[j] * (k.cT * w), g.ny[j] * (k.cT * w), k.cU * w, 0.0};
+  nodes[j] = NodeD{g.nx[j], g.ny[j], k.cU * w, k.cT * w};
 }
 
 // double-float node record (Laplace): G = log(R2) cG, H = (r.n) / R2 cH with
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
               gv[b][s * DOF + ar] = far[s] ? U[ar * DOF + b] : 0.f;
             }
         } else {
-          // 22 FP64 operations for a Laplace pair (fast64.cuh, constants
+          // 23 FP64 operations for a Laplace pair (fast64.cuh, constants
           // folded into the record; it was 59: the compiler's logarithm and
           // quotient), 46 for a Kelvin one.  FP64 issue bounds the kernel:
           // 4100 x 4100 entries of H and G 1.62 -> 0.77 ms.
@@ -614,12 +614,15 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
             const double rx = s_x[el * nn + k] - sx[s], ry = s_y[el * nn + k] - sy[s];
             if constexpr (NC == 1) {
               const double R2 = fma(rx, rx, ry * ry);
-              U[0] = nd.c * f64::log(R2);
-              Tk[0] = f64::div(fma(rx, nd.nx, ry * nd.ny), R2);
+              U[0] = nd.cu * f64::log(R2);
+              Tk[0] = nd.ct * f64::div(fma(rx, nd.nx, ry * nd.ny), R2);
             } else {
               coop::kernel_values<NC>(kc, rx, ry, nd.nx, nd.ny, U, Tk);
 #pragma unroll
-              for (int c = 0; c < NC; ++c) U[c] *= nd.c;
+              for (int c = 0; c < NC; ++c) {
+                U[c] *= nd.cu;
+                Tk[c] *= nd.ct;
+              }
             }
           } else {
 #pragma unroll

@@ -15,9 +15,11 @@ struct __align__(16) NodeRec {
 };
 
 // 32-byte node record of the FP64 far field, in the place of a NodeRec.
-// Laplace: {n cT w, cU w, -}; Kelvin: {n w, w, -} (constants of coop::Consts).
+// Laplace: {n, cU w, cT w}; Kelvin: {n, w, w} (constants of coop::Consts).  The
+// normal is not scaled: r . n cancels, and a rounding of its terms shows (6 %
+// of the error of an entry of H).
 struct __align__(16) NodeD {
-  double nx, ny, c, pad;
+  double nx, ny, cu, ct;
 };
 
 // 64-byte node record of the double-float far field (Laplace): coordinates
