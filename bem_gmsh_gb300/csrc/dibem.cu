@@ -182,7 +182,7 @@ __device__ __forceinline__ T dibem_phi_int(int kind, T R, T kcond, T epsa) {
   }
 }
 
-// phi_int(R) / R^2 in FP64, up to the factor phi_int_scale: the powers of R
+// phi_int(R) / R^2 in FP64, times phi_int_divisor: the powers of R
 // cancel before they are formed, so a pair needs no quotient (an FP64 quotient
 // is five and a half multiply-adds of GB300's small FP64 pipe)
 __device__ __forceinline__ double phi_int_over_r2(int kind, double R2, double lgR2, double epsa) {
@@ -198,16 +198,17 @@ __device__ __forceinline__ double phi_int_over_r2(int kind, double R2, double lg
     default: return (R2 * R2 * R2) * R;
   }
 }
-__device__ __forceinline__ double phi_int_scale(int kind, double kcond) {
+// (sums are divided by it once: a factor 1 / 3 would round every sum one way)
+__device__ __forceinline__ double phi_int_divisor(int kind, double kcond) {
   switch (kind) {
-    case 1: return 1.0 / 3.0;
-    case 2: return 1.0 / 16.0;
-    case 3: return 1.0 / 5.0;
-    case 4: return 1.0 / 36.0;
-    case 5: return 1.0 / 7.0;
-    case 6: return 1.0 / 64.0;
-    case 7: return 1.0 / 9.0;
-    default: return 1.0 / (8.0 * kPi * kcond);
+    case 1: return 3.0;
+    case 2: return 16.0;
+    case 3: return 5.0;
+    case 4: return 36.0;
+    case 5: return 7.0;
+    case 6: return 64.0;
+    case 7: return 9.0;
+    default: return 8.0 * kPi * kcond;
   }
 }
 
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(128) dibem_ifid_kernel(GeomDev g, IfidRule rw,
     }
   }
   if constexpr (sizeof(T) == 8) {
-    aF *= phi_int_scale(rbf, kcond);
+    aF /= phi_int_divisor(rbf, kcond);
     aD *= radc;
   }
   atomicAdd(IF + i, aF);
@@ -400,7 +401,7 @@ __global__ void __launch_bounds__(NR_PT) dibem_near_kernel(const __grid_constant
     qy[v][3] = bad ? 0.0 : -(flip * dx);
   }
   __syncthreads();
-  const double cF = phi_int_scale(rbf, kcond), cD = 1.0 / (8.0 * kPi * kcond);
+  const double dF = phi_int_divisor(rbf, kcond), cD = 1.0 / (8.0 * kPi * kcond);
   const int lg = t & 15;
   for (int p0 = 0; p0 < count; p0 += NR_PT / 16) {
     const int p = p0 + (t >> 4);
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(NR_PT) dibem_near_kernel(const __grid_constant
       aD += __shfl_xor_sync(0xffffffffu, aD, o);
     }
     if (p < count && lg == 0) {
-      atomicAdd(IF + ip, aF * cF);
+      atomicAdd(IF + ip, aF / dF);
       atomicAdd(ID + ip, aD * cD);
     }
   }

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from bem_gmsh_gb300 import star_domain
-from bem_gmsh_gb300.api import H_G_gpu
+from bem_gmsh_gb300.api import H_G_gpu, dibem_ifid
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +31,16 @@ def test_orthogonal_normal_gives_zero():
     dad.jacobian[0] = 1.0 / 3.0
     H, G = H_G_gpu(dad, T=np.float64, npg=8, store=False)
     assert np.all(H[2:, 0] == 0.0) and np.all(G[2:, 0] != 0.0)
+
+
+@pytest.mark.parametrize("rbf, divisor", [("PHS1", 3), ("PHS3", 5), ("PHS5", 7)])
+def test_radial_integrals_are_divided(rbf, divisor):
+    """phi_int(R) / R^2 (r . n) for R = 5 i / 64 and r . n = 4 i / 64: whole
+    numbers over a power of two, divided once."""
+    dad = points((4 / 64, 3 / 64))
+    dad.normal[0] = (1.0, 0.0)
+    IF, _ = dibem_ifid(dad, rbf=rbf)
+    i = np.arange(2, 80)
+    # R, R^3, R^5 times r . n: at most 31 bits, exact
+    want = (5 * i / 64.0) ** {3: 1, 5: 3, 7: 5}[divisor] * (4 * i / 64.0)
+    assert np.array_equal(IF[2:], want / divisor)
