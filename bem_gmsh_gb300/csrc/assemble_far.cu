@@ -74,8 +74,12 @@ __device__ __forceinline__ void pack_node(const GeomDev& g, const Rules& R, cons
 __device__ __forceinline__ void pack_node_d(const GeomDev& g, const Rules& R, const Physics& ph, int j,
                                             NodeD* nodes) {
   const double w = g.jac[j] * R.ew[j % g.nn];
-  const coop::Consts k = ph.kind == 0 ? coop::make_consts<1>(ph) : coop::Consts{1.0, 0.0, 1.0, 0.0};
-  nodes[j] = NodeD{g.nx[j], g.ny[j], k.cU * w, k.cT * w};
+  if (ph.kind == 0) {
+    const coop::Consts k = coop::make_consts<1>(ph);
+    nodes[j] = NodeD{g.nx[j], g.ny[j], k.cU * w, k.cT * w};
+  } else {
+    nodes[j] = NodeD{g.nx[j] * w, g.ny[j] * w, w, 0.0};
+  }
 }
 
 // double-float node record (Laplace): G = log(R2) cG, H = (r.n) / R2 cH with
@@ -619,10 +623,7 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
             } else {
               coop::kernel_values<NC>(kc, rx, ry, nd.nx, nd.ny, U, Tk);
 #pragma unroll
-              for (int c = 0; c < NC; ++c) {
-                U[c] *= nd.cu;
-                Tk[c] *= nd.ct;
-              }
+              for (int c = 0; c < NC; ++c) U[c] *= nd.cu;
             }
           } else {
 #pragma unroll

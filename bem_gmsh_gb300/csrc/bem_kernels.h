@@ -15,9 +15,10 @@ struct __align__(16) NodeRec {
 };
 
 // 32-byte node record of the FP64 far field, in the place of a NodeRec.
-// Laplace: {n, cU w, cT w}; Kelvin: {n, w, w} (constants of coop::Consts).  The
-// normal is not scaled: r . n cancels, and a rounding of its terms shows (6 %
-// of the error of an entry of H).
+// Laplace: {n, cU w, cT w}; Kelvin: {n w, w, -} (constants of coop::Consts).  The
+// Laplace normal is not scaled: r . n cancels, and a rounding of its terms shows
+// (6 % of the error of an entry of H; Kelvin's other terms hide it, and four
+// products more are 8 % of its time).
 struct __align__(16) NodeD {
   double nx, ny, cu, ct;
 };
