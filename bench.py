@@ -132,13 +132,12 @@ def cpu_reference(dad_factory, steps, warmup, npg):
     return ts, x, stages
 
 
-# DRAM traffic of one bulk trailing update (k_gemm_tc_p, the persistent
-# kernel) at the C2 trailing size, from one ncu capture of the update timed
-# alone (bem_selftest which = 3, n = 8192, trailing block 8064^2):
-# dram__bytes_read 276934400 B + dram__bytes_write 200425984 B for
-# 8 * 8064^2 = 520224768 algorithmic bytes.
-GEMM_TRAFFIC_CAPTURE = {"launch": "bulk update alone, trailing block 8064^2", "read_bytes": 276934400,
-                        "write_bytes": 200425984, "algorithmic_bytes": 8 * 8064 ** 2}
+# DRAM traffic of one bulk trailing update of two steps (k_gemm_tc_p<true>),
+# from one ncu capture (bem_selftest which = 1, n = 8192, the first pair's
+# trailing block 7808^2): dram__bytes_read 283838208 B + dram__bytes_write
+# 191046912 B for 8 * 7808^2 = 487718912 algorithmic bytes.
+GEMM_TRAFFIC_CAPTURE = {"launch": "bulk update of two steps, trailing block 7808^2", "read_bytes": 283838208,
+                        "write_bytes": 191046912, "algorithmic_bytes": 8 * 7808 ** 2}
 
 
 def extra_configs(ctx):
