@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(256) far_kernel(FarArgs a) {
           // 23 FP64 operations for a Laplace pair (fast64.cuh, constants
           // folded into the record; it was 59: the compiler's logarithm and
           // quotient), 46 for a Kelvin one.  FP64 issue bounds the kernel:
-          // 4100 x 4100 entries of H and G 1.62 -> 0.77 ms.
+          // 4100 x 4100 entries of H and G 1.62 -> 0.81 ms.
           double U[NC], Tk[NC];
           if (far[s]) {
             const NodeD& nd = s_ndd[el * nn + k];

@@ -24,7 +24,7 @@
 // largest integral, which is the sums' rounding (the map with 8 points: 3e-11).
 // (npg >= 8 only: with fewer points the ellipse is so large that little is
 // gained.)  The other pairs take the map, by warps (near_coop.cuh).  1000
-// points and 341 quadratic elements: the call 15.7 -> 0.39 ms.
+// points and 341 quadratic elements: the call 15.7 -> 0.40 ms.
 #include <cmath>
 #include <cstring>
 
