@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(128) dibem_ifid_kernel(GeomDev g, IfidRule rw,
     }
   }
   if constexpr (sizeof(T) == 8) {
-    aF /= phi_int_divisor(rbf, kcond);
+    aF = f64::div(aF, phi_int_divisor(rbf, kcond));
     aD *= radc;
   }
   atomicAdd(IF + i, aF);
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(NR_PT) dibem_near_kernel(const __grid_constant
       aD += __shfl_xor_sync(0xffffffffu, aD, o);
     }
     if (p < count && lg == 0) {
-      atomicAdd(IF + ip, aF / dF);
+      atomicAdd(IF + ip, f64::div(aF, dF));
       atomicAdd(ID + ip, aD * cD);
     }
   }
