@@ -57,7 +57,7 @@ struct AdjArgs {
   const int* ncand;
   int ccap;
   int2* pairs;     // near pairs (i, e)
-  int* count;      // [0] near pair count, [1] overflow flag
+  int* count;      // [0] near pair count, [1] overflow flag, [2] tasks claimed
   int cap;
   double* S;       // values of the near integrals, neval per pair
 };
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(128) adj_near_kernel(const __grid_constant__ A
   const Rules& R = a.R;
   const int nev = near_values(NN);
   const int64_t count = (int64_t)min(a.count[0], a.cap) * nev;
-  const int nwarps = gridDim.x * 4, gw = warp * gridDim.x + blockIdx.x;
+  if (blockIdx.x >= NEAR_CTAS && count <= NEAR_MANY * PAIRS) return;
   for (int q = threadIdx.x; q < R.npg; q += blockDim.x) {
     s_q[q] = R.qsi[q];
     s_w[q] = R.w[q];
@@ -292,7 +292,15 @@ __global__ void __launch_bounds__(128) adj_near_kernel(const __grid_constant__ A
   ph.k = a.k;
   const Consts kc = make_consts<1>(ph);
   Slot* slots = s_slots[warp];
-  for (int64_t base = (int64_t)gw * PAIRS; base < count; base += (int64_t)nwarps * PAIRS) {
+  // one task per warp of the first CTAs, the others claimed, as the pairs of
+  // an assembly (near_kernel): other gradients of a batch may hold any SMs
+  auto claim = [&] {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(a.count + 2, 1);
+    return (int64_t)(4 * NEAR_CTAS + __shfl_sync(FULL, t, 0)) * PAIRS;
+  };
+  for (int64_t base = blockIdx.x < NEAR_CTAS ? (int64_t)(warp * NEAR_CTAS + (int)blockIdx.x) * PAIRS : claim();
+       base < count; base = claim()) {
     const int np = (int)min((int64_t)PAIRS, count - base);
     if (lane < np) {
       const int64_t t = base + lane;
@@ -586,7 +594,7 @@ extern "C" int bem_adjoint_laplace2d(bem_ctx* c, const bem_geom2d* g, double k, 
   char* np = (char*)c->get(bem_ctx::SLOT_ADJ2, (sizeof(double) * nev + sizeof(int2)) * (size_t)cap);
   int* cnt = (int*)c->get(bem_ctx::SLOT_COUNTERS, 64) + 4;
   if (!np || !cnt) return BEM_ERR_NOMEM;
-  cudaMemsetAsync(cnt, 0, 2 * sizeof(int), c->stream);
+  cudaMemsetAsync(cnt, 0, 3 * sizeof(int), c->stream);
   cudaMemsetAsync(gX, 0, sizeof(double) * 5 * (size_t)N, c->stream);
   AdjArgs aa{};
   aa.g = gd;
@@ -614,11 +622,11 @@ extern "C" int bem_adjoint_laplace2d(bem_ctx* c, const bem_geom2d* g, double k, 
     adj_near_general_kernel<<<4096, 64, 0, c->stream>>>(aa);
   } else {
     switch (gd.nn) {
-      case 2: adj_near_kernel<2><<<304, 128, 0, c->stream>>>(aa); break;
-      case 3: adj_near_kernel<3><<<304, 128, 0, c->stream>>>(aa); break;
-      case 4: adj_near_kernel<4><<<304, 128, 0, c->stream>>>(aa); break;
-      case 5: adj_near_kernel<5><<<304, 128, 0, c->stream>>>(aa); break;
-      case 6: adj_near_kernel<6><<<304, 128, 0, c->stream>>>(aa); break;
+      case 2: adj_near_kernel<2><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
+      case 3: adj_near_kernel<3><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
+      case 4: adj_near_kernel<4><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
+      case 5: adj_near_kernel<5><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
+      case 6: adj_near_kernel<6><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
     }
   }
   adj_near_slope_kernel<<<std::min((16 * n + 127) / 128, 152 * 16), 128, 0, c->stream>>>(aa);

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(PACK_T) pack_kernel(const __grid_constant__ Pa
   }
   const GeomDev& g = a.g;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 2) a.counters[i] = 0;
+  if (i < 3) a.counters[i] = 0;
   if (i < g.nt) {
     pack_row(g, i, a.rows);
     for (int c = 0; c < a.dof * a.dof; ++c) a.rowsum[(size_t)i * a.dof * a.dof + c] = 0.0;
@@ -785,7 +785,7 @@ static void launch_variant(const AsmRequest& q, cudaStream_t st) {
   NearArgs na{};
   na.g = g; na.R = q.R; na.ph = q.ph; na.near_factor = q.near_factor;
   na.ld = q.ld; na.ldg = q.ldg; na.pair_cap = q.pair_cap;
-  na.pair_count = q.counters; na.pairs = q.pairs;
+  na.pair_count = q.counters; na.claim = q.counters + 2; na.pairs = q.pairs;
   na.H = q.H; na.G = q.G; na.A32 = q.A32;
   na.bc = q.bc; na.bv = q.bv; na.b = q.b; na.rowsum = q.rowsum; na.gdiag = q.gdiag;
   na.mode = PREC == 0 ? 0 : (!FUSED ? 1 : (MIXED ? 3 : 2));  // PREC 3: fused FP64 (2)

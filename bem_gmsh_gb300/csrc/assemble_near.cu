@@ -106,9 +106,17 @@ __global__ void __launch_bounds__(128) near_general_kernel(const __grid_constant
 }
 
 // The listed pairs by warps (near_coop.cuh).  FP64 issue bounds it: a warp
-// with 16 pairs issues about 3000 FP64 instructions.  The grid is two CTAs
-// of four warps per SM; a warp takes as many pairs as spread the list over
-// the GPU's 608 schedulers, one at least and 16 at most.
+// with 16 pairs issues about 3000 FP64 instructions.  A task is as many pairs
+// as spread the list over the GPU's 608 schedulers, one at least and 16 at
+// most.  The kernel runs beside the far and on-element kernels, whose CTAs may
+// hold any SMs when it starts: with two CTAs of four warps per SM and a fixed
+// share each, they now and then stood four to an SM on half of the SMs (333 000
+// pairs 5.5 or 10.5 ms).  So the warps of the first 304 CTAs have one task each
+// (claimed tasks would gather on the SMs that start first: 1000 nodes 0.29 ms
+// instead of 0.12), and they claim the others from a counter.  From four rounds
+// of tasks on 304 CTAs more claim too, which find an SM where the first ones
+// have left some free; before that they would only crowd some SMs (8193 nodes,
+// 1366 tasks: H and G in FP32 0.63 ms instead of 0.59).
 template <int NC, int NN>
 __global__ void __launch_bounds__(128) near_kernel(const __grid_constant__ NearArgs a) {
   using namespace coop;
@@ -116,9 +124,13 @@ __global__ void __launch_bounds__(128) near_kernel(const __grid_constant__ NearA
   __shared__ double s_q[BEM_MAXNPG], s_w[BEM_MAXNPG];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int count = min(*a.pair_count, a.pair_cap);
-  const int nwarps = gridDim.x * 4, gw = warp * gridDim.x + blockIdx.x;
-  const int spread = min(nwarps, 608);
-  const int per = max(1, min(PAIRS, (count + spread - 1) / spread));
+  const int per = max(1, min(PAIRS, (count + 607) / 608));
+  if (blockIdx.x >= NEAR_CTAS && count <= NEAR_MANY * PAIRS) return;
+  auto claim = [&] {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(a.claim, 1);
+    return (4 * NEAR_CTAS + __shfl_sync(FULL, t, 0)) * per;
+  };
   const GeomDev& g = a.g;
   const Rules& R = a.R;
   for (int q = threadIdx.x; q < R.npg; q += blockDim.x) {
@@ -130,7 +142,8 @@ __global__ void __launch_bounds__(128) near_kernel(const __grid_constant__ NearA
   const int ng = R.ngeo > 0 ? R.ngeo : NN;
   const int G = per == 1 ? 32 : (per == 2 ? 16 : 8);
   Slot* slots = s_slots[warp];
-  for (int base = gw * per; base < count; base += nwarps * per) {
+  for (int base = blockIdx.x < NEAR_CTAS ? (warp * NEAR_CTAS + (int)blockIdx.x) * per : claim(); base < count;
+       base = claim()) {
     const int np = min(per, count - base);
     if (lane < np) {
       const int2 pr = a.pairs[base + lane];
@@ -471,7 +484,7 @@ static void launch_near_nc(const NearArgs& na, cudaStream_t st) {
     near_general_kernel<NC><<<nblk, 128, 0, st>>>(na);
     return;
   }
-  const int nblk = 304;
+  const int nblk = 2 * NEAR_CTAS;  // as many as stay resident
   switch (na.R.nn) {
     case 2: near_kernel<NC, 2><<<nblk, 128, 0, st>>>(na); break;
     case 3: near_kernel<NC, 3><<<nblk, 128, 0, st>>>(na); break;

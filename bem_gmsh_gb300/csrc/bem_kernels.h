@@ -101,6 +101,11 @@ struct FarArgs {
   int* status;
 };
 
+// CTAs of the near kernels with a task of their own, two per SM
+constexpr int NEAR_CTAS = 304;
+// tasks above which as many CTAs more claim some: four for each of those warps
+constexpr int NEAR_MANY = 4 * 4 * NEAR_CTAS;
+
 struct NearArgs {
   GeomDev g;
   Rules R;
@@ -109,6 +114,7 @@ struct NearArgs {
   int64_t ld, ldg;
   int pair_cap;
   const int* pair_count;
+  int* claim;   // next task of the near kernel, zero at its start
   const int2* pairs;
   void* H;
   void* G;
@@ -164,7 +170,7 @@ struct AsmRequest {
   ElemRec* elems;
   double* rowsum;
   double* gdiag;
-  int* counters;  // [0] pair count, [1] status
+  int* counters;  // [0] pair count, [1] status, [2] tasks claimed
   int2* pairs;
   int pair_cap;
   // optional side stream for the on-element kernel (runs beside the far and
