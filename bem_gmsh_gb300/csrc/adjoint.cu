@@ -622,11 +622,11 @@ extern "C" int bem_adjoint_laplace2d(bem_ctx* c, const bem_geom2d* g, double k, 
     adj_near_general_kernel<<<4096, 64, 0, c->stream>>>(aa);
   } else {
     switch (gd.nn) {
-      case 2: adj_near_kernel<2><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
-      case 3: adj_near_kernel<3><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
-      case 4: adj_near_kernel<4><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
-      case 5: adj_near_kernel<5><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
-      case 6: adj_near_kernel<6><<<2 * NEAR_CTAS, 128, 0, c->stream>>>(aa); break;
+      case 2: adj_near_kernel<2><<<near_ctas(near_factor), 128, 0, c->stream>>>(aa); break;
+      case 3: adj_near_kernel<3><<<near_ctas(near_factor), 128, 0, c->stream>>>(aa); break;
+      case 4: adj_near_kernel<4><<<near_ctas(near_factor), 128, 0, c->stream>>>(aa); break;
+      case 5: adj_near_kernel<5><<<near_ctas(near_factor), 128, 0, c->stream>>>(aa); break;
+      case 6: adj_near_kernel<6><<<near_ctas(near_factor), 128, 0, c->stream>>>(aa); break;
     }
   }
   adj_near_slope_kernel<<<std::min((16 * n + 127) / 128, 152 * 16), 128, 0, c->stream>>>(aa);

@@ -116,7 +116,10 @@ __global__ void __launch_bounds__(128) near_general_kernel(const __grid_constant
 // instead of 0.12), and they claim the others from a counter.  From four rounds
 // of tasks on 304 CTAs more claim too, which find an SM where the first ones
 // have left some free; before that they would only crowd some SMs (8193 nodes,
-// 1366 tasks: H and G in FP32 0.63 ms instead of 0.59).
+// 1366 tasks: H and G in FP32 0.63 ms instead of 0.59).  Even CTAs that leave at
+// once change where the first ones stand (cubic and quartic elements, 1000 to
+// 2600 nodes: 10 to 20 % of the call), so they are launched above a near factor
+// of 3 only.
 template <int NC, int NN>
 __global__ void __launch_bounds__(128) near_kernel(const __grid_constant__ NearArgs a) {
   using namespace coop;
@@ -484,7 +487,7 @@ static void launch_near_nc(const NearArgs& na, cudaStream_t st) {
     near_general_kernel<NC><<<nblk, 128, 0, st>>>(na);
     return;
   }
-  const int nblk = 2 * NEAR_CTAS;  // as many as stay resident
+  const int nblk = near_ctas(na.near_factor);
   switch (na.R.nn) {
     case 2: near_kernel<NC, 2><<<nblk, 128, 0, st>>>(na); break;
     case 3: near_kernel<NC, 3><<<nblk, 128, 0, st>>>(na); break;

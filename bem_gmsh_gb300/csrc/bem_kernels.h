@@ -105,6 +105,7 @@ struct FarArgs {
 constexpr int NEAR_CTAS = 304;
 // tasks above which as many CTAs more claim some: four for each of those warps
 constexpr int NEAR_MANY = 4 * 4 * NEAR_CTAS;
+inline int near_ctas(double near_factor) { return near_factor > 3.0 ? 2 * NEAR_CTAS : NEAR_CTAS; }
 
 struct NearArgs {
   GeomDev g;
